@@ -323,3 +323,17 @@ def test_longest_chain_pair_properties():
     assert sum(c != '-' for c in qrow) <= 37860 and sum(c != '-' for c in trow) <= 37860
     matched = sum(a != '-' and b != '-' for a, b in zip(qrow, trow))
     assert matched > 0.8 * 37860
+
+
+@pytest.mark.parametrize("far", [3.0e7, 2.0e18, 1.5e19, float("inf")])
+def test_far_residues(oracle, far):
+    """Structures with one residue far away, up to where squared distances
+    reach the end of the FP32 range and beyond: the score terms there are
+    those of an IEEE division, bit for bit."""
+    from gtalign_alpha_b200 import synth
+    wl = synth.config0(seed=41, n_refs=6, qlen=90, lmin=40, lmax=130)
+    q, r = synth.pack(wl.queries), synth.pack(wl.refs)
+    r.x[r.offs[1] + 5] = far
+    r.y[r.offs[3] + 11] = -far
+    res, ora = run_both(oracle, q, r, OPTSETS["speed13"])
+    assert_same(res, ora, q.n, r.n)
