@@ -237,7 +237,9 @@ static size_t pair_bytes(int lq, int lr, bool strings, bool f3 = false) {
     b += (size_t)std::min(lq, lr) * 28;                // aligned pairs + coordinates
     if (strings) b += (size_t)5 * (lq + lr + 1);       // alignment rows
     b += 4 * 8 + 12 * 4 * 2 + 16 * 4 + 4 * 4 + 12 * 4 + 64 + 4 + 24;  // state, offsets, work lists
-    if (std::min(lq, lr) >= gtb::RL_LONG_FEW)          // long-pair candidates
+    // the refinement candidates of a long pair; reserved from 384 residues, so
+    // that a memory budget admits the blocks it always has
+    if (std::min(lq, lr) >= 384)
         b += (size_t)gtb::RLW_CTAS_MAX * gtb::RLW_CTA_WARPS * gtb::RLW_CAND * 4 + 12;
     return b;
 }
@@ -408,15 +410,17 @@ static gtb_status run_block(gtb_handle* h, const DevBlock& D, float scorethld,
                 for (int k = 0; k < nl; k++) mk[lp[k]] = 1;
             }
         }
-        // pairs that may reach the long-pair thresholds of the refinement
-        // launches (n <= min(lq, lr)): the first tier and the second
-        int nlmax = 0, nlmax2 = 0;
+        // pairs that may reach the refinement launches' length classes
+        // (n <= min(lq, lr))
+        int nml[4] = {np, 0, 0, 0};
         for (int i = 0; i < np; i++) {
             long long p = q0 + i;
             const int ml = std::min(D.hqlen[p / D.nr], D.hrlen[p % D.nr]);
-            if (ml >= gtb::RL_LONG) nlmax++;
-            else if (ml >= gtb::RL_LONG_FEW) nlmax2++;
+            nml[1] += ml >= gtb::RC_N1;
+            nml[2] += ml >= gtb::RC_N2;
+            nml[3] += ml >= gtb::RL_LONG;
         }
+        const int nlmax = nml[3];
         std::vector<int>& ffi = ffiv[j];
         if (split) {
             ffi.assign(2 * (size_t)nitems, 0);
@@ -449,12 +453,9 @@ static gtb_status run_block(gtb_handle* h, const DevBlock& D, float scorethld,
         size_t o_dwp = nl ? carve((size_t)dnprog * sizeof(int)) : 0;
         size_t o_dwe = carve(sizeof(int));      // wavefront error flag (multi-CTA and CTA waves)
         size_t o_rll = nlmax ? carve((size_t)(2 * nlmax + 1) * sizeof(int)) : 0;
-        // CTAs per long pair of each tier (more when few pairs are long)
+        // CTAs per long pair (more when few pairs are long)
         const int ctasA = gtb::rlw_ctas_for(h->tn.refine_long_ctas, nlmax);
-        const int ctasB = gtb::rlw_ctas_for(gtb::RLW_CTAS_FEW, nlmax2);
         size_t o_rlc = nlmax ? carve((size_t)nlmax * ctasA * gtb::RLW_CTA_WARPS * gtb::RLW_CAND * sizeof(float)) : 0;
-        size_t o_rll2 = nlmax2 ? carve((size_t)(2 * nlmax2 + 1) * sizeof(int)) : 0;
-        size_t o_rlc2 = nlmax2 ? carve((size_t)nlmax2 * ctasB * gtb::RLW_CTA_WARPS * gtb::RLW_CAND * sizeof(float)) : 0;
         // detailed search: local score matrices, slots, DP scores, branches
         size_t o_lsm = B.f3 ? carve((size_t)std::max<long long>(off_lsm[np], 1)) : 0;
         const size_t nsl = (size_t)B.f3nsec * F3_NTOP, nbr = (size_t)B.f3nsec * F3_NBMAX;
@@ -511,19 +512,13 @@ static gtb_status run_block(gtb_handle* h, const DevBlock& D, float scorethld,
             T.rl_long = rl; T.rl_next = rl + nlmax; T.rl_count = rl + 2 * nlmax;
             T.rl_cand = (float*)(base + o_rlc);
         }
-        T.rl_nlmax2 = nlmax2; T.rl_long2 = T.rl_count2 = T.rl_next2 = nullptr; T.rl_cand2 = nullptr;
-        if (nlmax2) {
-            int* rl = (int*)(base + o_rll2);
-            T.rl_long2 = rl; T.rl_next2 = rl + nlmax2; T.rl_count2 = rl + 2 * nlmax2;
-            T.rl_cand2 = (float*)(base + o_rlc2);
-        }
+        for (int k = 0; k < 4; k++) T.nml[k] = nml[k];
         T.ndw = 0; T.dw_nprog = 0; T.dw_item = T.dw_pair = T.dw_G = nullptr; T.dw_soff = nullptr;
         T.dw_mark = nullptr; T.dw_prog = nullptr;
         T.dw_err = (int*)(base + o_dwe);
         T.dp_kc = h->tn.dp_cta_pairs;
         T.ff_span = h->tn.seed_chunk;
         T.rlw_ctas = ctasA;
-        T.rlw_ctas2 = ctasB;
         CK(cudaMemsetAsync(T.dw_err, 0, sizeof(int), st));
         h->h_flag[evset] = 0;
         if (nl) {

@@ -8,11 +8,13 @@
 //    reduces (max score, lowest offset index), across CTAs through a packed
 //    64-bit atomic maximum.
 //  * refinement (every fragment-based superposition refinement): pairs taken
-//    from a work list sorted by position count; 16 lanes per pair (32 after
-//    the --pre-score filter, 64 warps for pairs of 1,536+ positions) take the
-//    pair's admissible (fragment position, fragment length) variants from a
-//    pool and advance one pass over the positions at a time; the lanes
-//    reduce (max score, lowest variant index).  The distance-threshold
+//    from a work list sorted by position count.  Where few pairs take part
+//    (after the --pre-score filter, small batches) and for pairs of 512+
+//    positions, a warp makes each pass of a variant and a cluster of CTAs
+//    takes a pair (k_refine_coop); the shorter pairs of a large batch's first
+//    launches take 16 lanes each, a variant per lane from the pair's pool
+//    (k_refine), and pairs of 1,536+ positions many warps.  The winner is the
+//    larger score, then the lower variant index.  The distance-threshold
 //    covariance pass of iteration k+1 is fused into the scoring pass of
 //    iteration k.
 //  * DP: pairs from a work list (largest matrices first), one warp per pair;
@@ -27,12 +29,14 @@
 // depend on the launch geometry.
 #include <algorithm>
 #include <type_traits>
+#include <cooperative_groups.h>
 #include "gtb200.h"
 #include "gtb_device.cuh"
 #include "gtb_kernels.cuh"
 #include "gtb_gonnet.h"
 
 namespace gtb {
+namespace cg = cooperative_groups;
 
 // Residue exchange scores of the --add-search-by-ss DP (log2 Gonnet ratios
 // over the letters A..Z, built on the host by gtb_gonnet_scores); a global
@@ -740,9 +744,6 @@ __global__ void k_rlist_count(Blk B, Bat T, int mode) {
     if (n >= T.rl_min && T.rl_long) {          // many warps for this pair
         int slot = atomicAdd(T.rl_count, 1);
         if (slot < T.rl_nlmax) { T.rl_long[slot] = i; return; }
-    } else if (n >= T.rl_min2 && T.rl_long2) {  // the lower tier
-        int slot = atomicAdd(T.rl_count2, 1);
-        if (slot < T.rl_nlmax2) { T.rl_long2[slot] = i; return; }
     }
     if (n > 0) {
         atomicAdd(&T.rhist[RL_NB - 1 - (n >> RL_SHIFT)], 1);
@@ -828,8 +829,7 @@ __global__ void k_rlist_fill(Blk B, Bat T, int mode) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= T.np) return;
     int n = refine_span(B, T, mode, i);
-    if ((n >= T.rl_min && T.rl_long) || (n >= T.rl_min2 && T.rl_long2))
-        return;                                  // listed by k_rlist_count
+    if (n >= T.rl_min && T.rl_long) return;      // listed by k_rlist_count
     if (n > 0) T.rlist[atomicAdd(&T.rhist[RL_NB - 1 - (n >> RL_SHIFT)], 1)] = i;
 }
 
@@ -848,6 +848,14 @@ __global__ void k_rlist_fill(Blk B, Bat T, int mode) {
 // pos + fraglen < n + max(step, 0); a fragment reaching past the end is
 // shifted back to end at n.
 enum VariantKind { VK_STAGE = 0, VK_P2ONE = 1, VK_P2ALL = 2, VK_LOG = 3 };
+
+// the variants of a refinement launch
+__device__ __forceinline__ int refine_variants(int mode, const Blk& B) {
+    return mode == RM_PLOG ? VK_LOG
+         : mode == RM_FIN2 ? (B.refinement == GTB_REFINEMENT_FULLA ? VK_P2ALL : VK_P2ONE)
+         : mode == RM_PROD2 ? (B.refinement >= GTB_REFINEMENT_FULL ? VK_P2ALL : VK_P2ONE)
+         : VK_STAGE;
+}
 
 struct VariantList {
     int total;
@@ -1175,9 +1183,7 @@ __device__ __forceinline__ void refine_commit(const Blk& B, const Bat& T, int i,
     }
 }
 
-// RF_LPP lanes per pair: 16 (two pairs per warp) where most pairs of a
-// batch take part; 32 where few do (after the --pre-score filter), which
-// shortens the launches whose time is that of their slowest pair.
+// RF_LPP lanes per pair: 16 (two pairs per warp), or a warp (long pairs).
 // Warps per CTA: 4 (1 and 2, with an SM refilling a finished warp's slot at
 // once, measured the same on the benchmark step: the concurrent sub-batch
 // streams fill those slots already).
@@ -1193,7 +1199,7 @@ constexpr int RF_WARPS_LONG = RLW_CTA_WARPS;
 // WIDE (long pairs only): a warp works on one variant at a time, its lanes
 // sharing the passes (wide_pass); otherwise every lane has a variant.
 template <int MODE, int RF_LPP, bool LONG, bool WIDE = false>
-__device__ __forceinline__ void refine_slot(const Blk& B, const Bat& T, int slot, int wlong) {
+__device__ __forceinline__ void refine_slot(const Blk& B, const Bat& T, int slot, int wlong, int slot_end = 0) {
     constexpr int RF_WARPS = LONG ? RF_WARPS_LONG : RF_WARPS_SHORT;
     static_assert(!WIDE || (LONG && RF_LPP == 32), "a wide pass is a long pair's warp");
     __shared__ float s_wide[WIDE ? 17 * RF_WARPS * 32 : 1];   // block partials of wide passes
@@ -1204,7 +1210,7 @@ __device__ __forceinline__ void refine_slot(const Blk& B, const Bat& T, int slot
     const int lane = threadIdx.x & 31;
     const int sub = lane / RF_LPP;
     const unsigned smask = RF_LPP == 32 ? 0xffffffffu : ((1u << (RF_LPP & 31)) - 1u) << (sub * RF_LPP);
-    const bool valid = LONG ? slot < *T.rl_count : slot < T.rhist[RL_NB];
+    const bool valid = LONG ? slot < *T.rl_count : slot < slot_end;
     if (__ballot_sync(FULL, valid) == 0) return;
     const int i = valid ? (LONG ? T.rl_long[slot] : T.rlist[slot]) : 0;
     const int str = RF_WARPS * 32;
@@ -1232,10 +1238,7 @@ __device__ __forceinline__ void refine_slot(const Blk& B, const Bat& T, int slot
     const int n = G.n;
     const bool prod = (MODE == RM_PROD1 || MODE == RM_PROD2 || MODE == RM_PLOG);
     const bool phase2 = (MODE == RM_FIN2 || MODE == RM_PROD2 || MODE == RM_PLOG);
-    const int vk = MODE == RM_PLOG ? VK_LOG
-                 : MODE == RM_FIN2 ? (B.refinement == GTB_REFINEMENT_FULLA ? VK_P2ALL : VK_P2ONE)
-                 : MODE == RM_PROD2 ? (B.refinement >= GTB_REFINEMENT_FULL ? VK_P2ALL : VK_P2ONE)
-                 : VK_STAGE;
+    const int vk = refine_variants(MODE, B);
     const float d0 = prod ? B.t_d0fin[ml] : B.t_d0[ml];
     const float d02 = __fmul_rn(d0, d0);
     const float d82 = B.t_d82[ml];
@@ -1451,10 +1454,18 @@ __device__ __forceinline__ void refine_slot(const Blk& B, const Bat& T, int slot
         refine_commit<MODE>(B, T, i, lq, lr, havewin, wb, lgbest, wndx, wpos, tbest, str);
 }
 
+// Pairs with lo <= n < hi of the work list (lo, hi multiples of 16, hi 0: no
+// upper bound): their range of list slots.
+__device__ __forceinline__ void rlist_range(const Bat& T, int lo, int hi, int& first, int& last) {
+    first = hi > 0 ? T.rhist[RL_NB - 1 - (hi >> RL_SHIFT)] : 0;
+    last = T.rhist[RL_NB - 1 - (lo >> RL_SHIFT)];
+}
+
 // LONG: T.rlw_ctas CTAs per long pair; the grid (a multiple of that) walks
 // the long pairs listed for this launch.
+// Otherwise: the pairs of the work list with lo <= n < hi positions.
 template <int MODE, int RF_LPP, bool LONG, bool WIDE = false>
-__global__ void __launch_bounds__((LONG ? RF_WARPS_LONG : RF_WARPS_SHORT) * 32) k_refine(Blk B, Bat T) {
+__global__ void __launch_bounds__((LONG ? RF_WARPS_LONG : RF_WARPS_SHORT) * 32) k_refine(Blk B, Bat T, int lo, int hi) {
     if (LONG) {
         const int c = T.rlw_ctas;
         const int wl = (int)(blockIdx.x % c) * RF_WARPS_LONG + (threadIdx.x >> 5);
@@ -1463,9 +1474,11 @@ __global__ void __launch_bounds__((LONG ? RF_WARPS_LONG : RF_WARPS_SHORT) * 32) 
             refine_slot<MODE, RF_LPP, LONG, WIDE>(B, T, slot, wl);
     } else {
         constexpr int RF_PPW = 32 / RF_LPP;        // pairs per warp
-        const int slot = blockIdx.x * (RF_PPW * RF_WARPS_SHORT) + (threadIdx.x >> 5) * RF_PPW +
+        int first, last;
+        rlist_range(T, lo, hi, first, last);
+        const int slot = first + blockIdx.x * (RF_PPW * RF_WARPS_SHORT) + (threadIdx.x >> 5) * RF_PPW +
                          (int)(threadIdx.x & 31) / RF_LPP;
-        refine_slot<MODE, RF_LPP, LONG>(B, T, slot, 0);
+        refine_slot<MODE, RF_LPP, LONG>(B, T, slot, 0, last);
     }
 }
 
@@ -1501,23 +1514,496 @@ __global__ void k_refine_long_fin(Blk B, Bat T) {
                         __float_as_int(c[4]), c + 5, 1);
 }
 
+// ---------------------------------------------------------------------------
+// Refinement with a warp to a pass.  A lane that sweeps a whole pass by itself
+// (refine_slot) makes n dependent position visits, so a launch lasts as long
+// as its slowest variant's: ~150 us for one pair of 150 positions, 16 ms where
+// pairs of 400 to 1,500 positions share 16 lanes.  Here the 32 lanes of a warp
+// take the 32 positions of a block: distances, scores and inclusion masks of
+// a block at once (no order matters there), the masked coordinates and score
+// terms go to shared memory, and then 16 lanes a block sum its 16 fields, a
+// field each, in position order; the block sums are folded in block order by
+// the field's lane.  Every sum is the sequence of operations of one lane's
+// sweep (a masked position adds a zero), so results are the same bits.
+//
+// The rotation solve is FP64 and takes as long as several such passes, so a
+// warp holds up to CM_MAX variants, lane m the state of variant m: it runs
+// their passes one after another and then all their solves at once.
+//
+// A cluster of CTAs takes a pair (the grid's clusters walk the pairs of the
+// launch's length class, longest first); the CTAs copy the pair's coordinates
+// to shared memory once, draw variants from a counter each, and the CTAs'
+// winners meet in the first one's shared memory.  What bounds it: the latency
+// of the pass -> solve chain (about 800 + 2,800 cycles at 150 positions).
+// Refinement launches of a call, before -> after: one pair of 150 residues
+// 3.5 -> 1.0 ms, 16 x 500 29 -> 16 ms, all against all of 400 structures
+// 114 -> 78 ms, 2 x 20,000 115 -> 62 ms (three streams).
+constexpr int CM_WARPS = 4;
+constexpr int CM_MAX = 8;                    // variants a warp holds at most
+constexpr int CM_CMAX = 8;                   // CTAs per cluster at most
+constexpr int CM_CHUNK = 4;                  // blocks of positions per step of a pass
+constexpr int CM_BST = 36;                   // floats between a block's components (16-byte rows, no bank conflicts)
+constexpr int CM_BLKW = 8 * CM_BST;          // floats per block: q xyz, r xyz, score term, ones
+constexpr int CM_ROW = 20;                   // floats of a variant's pass parameters
+struct CoopWarp {                            // one warp's shared memory
+    float buf[CM_CHUNK * CM_BLKW];
+    float row[CM_MAX * CM_ROW];              // transform and parameters of each variant's pass
+    float tot[CM_MAX * CM_ROW];              // its 15 sums, score, count, third-smallest distance
+    float last[16 * CM_MAX], tb[12 * CM_MAX], tbest[12 * CM_MAX];   // as refine_slot's, a column per lane
+};
+struct alignas(16) CoopSmem {
+    CoopWarp w[CM_WARPS];
+    float win[CM_CMAX * 32];                 // the CTAs' winners (first CTA)
+    float cand[CM_WARPS * 32];               // the warps' winners
+    int next;
+};
+inline size_t coop_smem_bytes(int nmax) {
+    return sizeof(CoopSmem) + (size_t)((nmax + BLK - 1) / BLK * BLK) * (sizeof(float4) + sizeof(float2));
+}
+
+// the exact error of s + b added to the compensation (Knuth's TwoSum): the
+// same c as nfold's, whose comparison only orders the operands
+__device__ __forceinline__ void tfold(float& s, float& c, float b) {
+    const float t = __fadd_rn(s, b);
+    const float bb = __fsub_rn(t, s);
+    c = __fadd_rn(c, __fadd_rn(__fsub_rn(s, __fsub_rn(t, bb)), __fsub_rn(b, bb)));
+    s = t;
+}
+
+__device__ __forceinline__ void keep3(float d, float& m1, float& m2, float& m3) {
+    const bool c1 = d < m1, c2 = d < m2, c3 = d < m3;
+    m3 = c2 ? m2 : (c3 ? d : m3);
+    m2 = c1 ? m1 : (c2 ? d : m2);
+    m1 = c1 ? d : m1;
+}
+
+// One pass of variant m (its parameters in w.row) by the whole warp; its
+// sums, score, count and third-smallest distance to w.tot.
+__device__ __forceinline__ void coop_pass(CoopWarp& w, int m, int n, const float4* cA,
+                                          const float2* cB, int lane) {
+    const unsigned FULL = 0xffffffffu;
+    const float* row = w.row + m * CM_ROW;
+    float tfm[12];
+#pragma unroll
+    for (int f = 0; f < 12; f++) tfm[f] = row[f];
+    const int kind = __float_as_int(row[12]), k0 = __float_as_int(row[13]), k1 = __float_as_int(row[14]);
+    const float thr = row[15], d02 = row[16], d82 = row[17];
+    const int flg = __float_as_int(row[18]);          // 1: only distances within d82 score, 2: smallest distances
+    const bool frag = kind == PK_FRAG;
+    const bool scr = kind == PK_SCORE || kind == PK_GSCORE;
+    const bool cov = kind == PK_SCORE || kind == PK_EXT;
+    const bool chk = flg & 1, trk = flg & 2;
+    const int lim = frag ? k1 : n;
+    const int nblk = (lim + BLK - 1) / BLK;
+    // this lane's sum: field lane & 15 of block 2k + lane / 16
+    const int f = lane & 15;
+    const int ax = f < 9 ? f / 3 : (f < 12 ? f - 9 : (f < 15 ? f - 9 : 6));
+    const int ay = f < 9 ? 3 + f % 3 : 7;
+    const float* X = w.buf + (lane >> 4) * CM_BLKW + ax * CM_BST;
+    const float* Y = w.buf + (lane >> 4) * CM_BLKW + ay * CM_BST;
+    float s = 0.f, c = 0.f;
+    float m1 = LARGEDST, m2 = LARGEDST, m3 = LARGEDST;
+    int cnt = 0;
+    for (int cb = frag ? k0 / BLK : 0; cb < nblk; cb += CM_CHUNK) {
+#pragma unroll
+        for (int e = 0; e < CM_CHUNK; e++) {
+            const int p = (cb + e) * BLK + lane;
+            const bool in = p < lim;
+            float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
+            float2 v = make_float2(0.f, 0.f);
+            if (in) { u = cA[p]; v = cB[p]; }
+            bool inc = in && k0 <= p;
+            float tm = 0.f;
+            if (!frag) {
+                const float d = dist2_tf(tfm, u.x, u.y, u.z, u.w, v.x, v.y);
+                inc = in && cov && d <= thr;
+                const float x = tmterm(d02, d);
+                tm = in && scr && (!chk || d <= d82) ? x : 0.f;
+                if (trk && in) keep3(d, m1, m2, m3);
+            }
+            float* o = w.buf + e * CM_BLKW + lane;
+            o[0] = inc ? u.x : 0.f;          o[CM_BST] = inc ? u.y : 0.f;
+            o[2 * CM_BST] = inc ? u.z : 0.f; o[3 * CM_BST] = inc ? u.w : 0.f;
+            o[4 * CM_BST] = inc ? v.x : 0.f; o[5 * CM_BST] = inc ? v.y : 0.f;
+            o[6 * CM_BST] = tm;
+            cnt += __popc(__ballot_sync(FULL, inc));
+        }
+        __syncwarp();
+        float b[CM_CHUNK / 2];
+#pragma unroll
+        for (int e = 0; e < CM_CHUNK / 2; e++) b[e] = 0.f;
+#pragma unroll
+        for (int p = 0; p < BLK; p += 4)
+#pragma unroll
+            for (int e = 0; e < CM_CHUNK / 2; e++) {
+                const float4 x = *(const float4*)(X + 2 * e * CM_BLKW + p), y = *(const float4*)(Y + 2 * e * CM_BLKW + p);
+                b[e] = __fmaf_rn(x.x, y.x, b[e]); b[e] = __fmaf_rn(x.y, y.y, b[e]);
+                b[e] = __fmaf_rn(x.z, y.z, b[e]); b[e] = __fmaf_rn(x.w, y.w, b[e]);
+            }
+        __syncwarp();
+        // folding the zeros of a block past the end changes nothing
+#pragma unroll
+        for (int e = 0; e < CM_CHUNK / 2; e++) {
+            const float odd = __shfl_down_sync(FULL, b[e], 16);
+            tfold(s, c, b[e]);
+            tfold(s, c, odd);
+        }
+    }
+    float* tot = w.tot + m * CM_ROW;
+    if (lane < 16) tot[lane] = __fadd_rn(s, c);
+    if (trk) {
+        // the three smallest of the pass: the lanes' three smallest merged
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float x1 = __shfl_xor_sync(FULL, m1, o), x2 = __shfl_xor_sync(FULL, m2, o),
+                        x3 = __shfl_xor_sync(FULL, m3, o);
+            keep3(x1, m1, m2, m3); keep3(x2, m1, m2, m3); keep3(x3, m1, m2, m3);
+        }
+    }
+    if (lane == 0) { tot[16] = (float)cnt; tot[17] = m3; }
+}
+
+// The whole alignment's FP32 RMSD (production phase 1, MpStageFin.cpp): the
+// 15 covariance sums, then the 6 sums of squares, by a warp.
+__device__ float coop_rmsd(CoopWarp& w, int n, const float4* cA, const float2* cB, int lane) {
+    double dv[21];
+    for (int part = 0; part < 2; part++) {
+        float s = 0.f, c = 0.f;
+        const int f = lane & 15;
+        const int ax = part ? (f < 6 ? f : 6) : (f < 9 ? f / 3 : (f < 15 ? f - 9 : 6));
+        const int ay = part ? ax : (f < 9 ? 3 + f % 3 : 7);
+        for (int b0 = 0; b0 * BLK < n; b0++) {
+            const int p = b0 * BLK + lane;
+            float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
+            float2 v = make_float2(0.f, 0.f);
+            if (p < n) { u = cA[p]; v = cB[p]; }
+            float* o = w.buf + lane;
+            o[0] = u.x; o[CM_BST] = u.y; o[2 * CM_BST] = u.z;
+            o[3 * CM_BST] = u.w; o[4 * CM_BST] = v.x; o[5 * CM_BST] = v.y;
+            o[6 * CM_BST] = 0.f;
+            __syncwarp();
+            float b = 0.f;
+            for (int k = 0; k < BLK; k++) b = __fmaf_rn(w.buf[ax * CM_BST + k], w.buf[ay * CM_BST + k], b);
+            __syncwarp();
+            tfold(s, c, b);
+        }
+        const float t = __fadd_rn(s, c);
+        if (part == 0) {
+#pragma unroll
+            for (int k = 0; k < 15; k++) dv[k] = (double)__shfl_sync(0xffffffffu, t, k);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 6; k++) dv[15 + k] = (double)__shfl_sync(0xffffffffu, t, k);
+        }
+    }
+    return (float)rmsd_from_sums(dv, (double)n);
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(CM_WARPS * 32) k_refine_coop(Blk B, Bat T, int lo, int hi) {
+    extern __shared__ __align__(16) unsigned char cm_smem[];
+    CoopSmem& S = *(CoopSmem*)cm_smem;
+    float4* cA = (float4*)(cm_smem + sizeof(CoopSmem));
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    cg::cluster_group cl = cg::this_cluster();
+    const int C = (int)cl.num_blocks(), crank = (int)cl.block_rank();
+    CoopWarp& w = S.w[warp];
+    int first, last;
+    rlist_range(T, lo, hi, first, last);
+    for (int e = 0; e < CM_CHUNK; e++) w.buf[e * CM_BLKW + 7 * CM_BST + lane] = 1.f;
+    for (int slot = first + (int)blockIdx.x / C; slot < last; slot += (int)gridDim.x / C) {
+        const int i = T.rlist[slot];
+        const int qi = pair_qi(B, T, i), ri = pair_ri(B, T, i);
+        const int lq = B.qlen[qi], lr = B.rlen[ri];
+        const int ml = lq < lr ? lq : lr;
+        const int swap = B.symmetric && (lq < lr);
+        const float4* q4 = B.q4 + B.q4off[qi];
+        const float4* r4 = B.r4 + B.r4off[ri];
+        int n, sq = 0, sr = 0;
+        if (MODE == RM_INIT) {
+            sq = T.seedq[i]; sr = T.seedr[i];
+            n = (lq - sq) < (lr - sr) ? (lq - sq) : (lr - sr);
+        } else {
+            n = T.naln[i];
+        }
+        float2* cB = (float2*)(cA + (n + BLK - 1) / BLK * BLK);
+        __syncthreads();                                      // the last pair's shared data is done with
+        if (MODE == RM_INIT) {
+            for (int p = threadIdx.x; p < n; p += blockDim.x) {
+                const float4 u = __ldg(q4 + sq + p), v = __ldg(r4 + sr + p);
+                cA[p] = make_float4(u.x, u.y, u.z, v.x);
+                cB[p] = make_float2(v.y, v.z);
+            }
+        } else {
+            const unsigned* aln = T.aln + T.off_aln[i];
+            for (int p = threadIdx.x; p < n; p += blockDim.x) {
+                const unsigned wv = aln[n - 1 - p];           // the traceback's order is backwards
+                const float4 u = __ldg(q4 + (wv >> 16)), v = __ldg(r4 + (wv & 0xffffu));
+                cA[p] = make_float4(u.x, u.y, u.z, v.x);
+                cB[p] = make_float2(v.y, v.z);
+            }
+        }
+        if (threadIdx.x == 0) S.next = 0;
+        __syncthreads();
+        float* lastv = w.last + lane;
+        float* tbs = w.tb + lane;
+        float* tbest = w.tbest + lane;
+        const bool prod = (MODE == RM_PROD1 || MODE == RM_PROD2 || MODE == RM_PLOG);
+        const bool phase2 = (MODE == RM_FIN2 || MODE == RM_PROD2 || MODE == RM_PLOG);
+        const int vk = refine_variants(MODE, B);
+        const float d0 = prod ? B.t_d0fin[ml] : B.t_d0[ml];
+        const float d02 = __fmul_rn(d0, d0);
+        const float d82 = B.t_d82[ml];
+        const int chk = prod ? 0 : 1;
+        const float best_init = (MODE == RM_INIT || MODE == RM_DP) ? 0.f
+                              : MODE == RM_PLOG ? T.grand[i] : -1.f;
+        const int maxalnmax = B.qmax < B.rmax ? B.qmax : B.rmax;
+        const float d0s = d0s_of(d0);
+        const float d0sm = __fsub_rn(d0s, 1.0f);
+        const float d02s = __fmul_rn(d0sm, d0sm);             // iteration 1's usual threshold
+        const float d0sp = __fadd_rn(d0s, 1.0f);
+        const float thr2 = __fmul_rn(d0sp, d0sp);             // threshold of iterations >= 2
+        const bool gscore = prod && lq != lr;                 // also scored by the longer length
+        float g02 = 0.f;
+        if (gscore) { const float g0 = B.t_d0fin[lq > lr ? lq : lr]; g02 = __fmul_rn(g0, g0); }
+        VariantList V;
+        variants_init(V, vk, n, maxalnmax, phase2 ? T.sfndx[i] : 0, phase2 ? T.sfpos[i] : 0, T.plog_round);
+        if (MODE == RM_PROD1 && warp == CM_WARPS - 1 && crank == 0 && V.total > 0) {
+            const float r = coop_rmsd(w, n, cA, cB, lane);
+            if (lane == 0) T.rmsd32[i] = r;
+        }
+        // variants a warp holds: an even share of the pair's
+        int M = (V.total + CM_WARPS * C - 1) / (CM_WARPS * C);
+        M = M < 1 ? 1 : (M < CM_MAX ? M : CM_MAX);
+        float lbest = 0.f, lgbest = 0.f;                      // this lane's best variant so far
+        int lsi = 0x7fffffff, lndx = 0, lpos = 0;
+        int kind = PK_IDLE, si = 0, vndx = 0, vpos = 0, k0 = 0, k1 = 0, cit = 0, m3on = 0, pchk = chk;
+        float best = 0.f, thr = 0.f, pd02 = d02;
+        bool need = lane < M;
+        unsigned long long vis = 0;
+        for (;;) {
+            const unsigned nm = __ballot_sync(FULL, need);
+            if (nm) {
+                int base = 0;
+                if (lane == 0) base = atomicAdd(&S.next, __popc(nm));
+                base = __shfl_sync(FULL, base, 0);
+                if (need) {
+                    need = false;
+                    kind = PK_IDLE;
+                    const int kv = (base + __popc(nm & ((1u << lane) - 1u))) * C + crank;
+                    if (kv < V.total) {
+                        int fl, kf;
+                        variants_get(V, vk, n, kv, si, vndx, vpos, fl, kf);
+                        if (MODE == RM_DP && T.vskip && si < 32 * F3_NSEC &&
+                            ((T.vskip[(long long)i * F3_NSEC + (si >> 5)] >> (si & 31)) & 1u)) {
+                            need = true;       // a variant the detailed search's slots rule out
+                        } else {
+                            kind = PK_FRAG; k0 = kf; k1 = kf + fl;
+                            best = best_init; cit = 0;
+                        }
+                    }
+                }
+            }
+            const unsigned act = __ballot_sync(FULL, kind != PK_IDLE);
+            if (act == 0) {
+                if (__any_sync(FULL, need)) continue;         // variants passed over
+                break;
+            }
+            // a pass of every variant, one after another
+            if (kind != PK_IDLE) {
+                float* row = w.row + lane * CM_ROW;
+                row[12] = __int_as_float(kind);
+                row[13] = __int_as_float(kind == PK_FRAG ? k0 : 0);
+                row[14] = __int_as_float(k1);
+                row[15] = thr; row[16] = pd02; row[17] = d82;
+                row[18] = __int_as_float((pchk ? 1 : 0) | (kind == PK_SCORE && m3on ? 2 : 0));
+            }
+            __syncwarp();
+            for (unsigned a = act; a; a &= a - 1) coop_pass(w, __ffs(a) - 1, n, cA, cB, lane);
+            __syncwarp();
+            vis += kind == PK_IDLE ? 0u : (kind == PK_FRAG ? (unsigned)(k1 - k0) : (unsigned)n);
+            // the variants' next steps, a lane each
+            if (kind != PK_IDLE) {
+                const float* tot = w.tot + lane * CM_ROW;
+                float* row = w.row + lane * CM_ROW;
+                float v[16];
+#pragma unroll
+                for (int f = 0; f < 15; f++) v[f] = tot[f];
+                v[15] = tot[16];
+                const float sc = tot[15], m3 = tot[17];
+                bool havev = false, done = false, solve = false;
+                if (kind == PK_FRAG) {
+                    if (v[15] < 1.0f) done = true;
+                    else solve = true;
+                } else if (kind == PK_SCORE) {
+                    if (best < sc) {
+                        best = sc;
+#pragma unroll
+                        for (int f = 0; f < 12; f++) tbs[f * CM_MAX] = row[f];
+                    }
+                    havev = true;
+                    if (cit == 0) {
+                        // iteration 1's threshold from iteration 0's three smallest distances
+                        float dst32;
+                        if (LARGEDST_CMP < m3 || m3 < d02s || n <= 3) dst32 = d02s;
+                        else {
+                            const float t = __fadd_rn(d0sm, __fmul_rn(ceilf(__fmul_rn(__fsub_rn(__fsqrt_rn(m3), d0sm), 2.0f)), 0.5f));
+                            dst32 = __fmul_rn(t, t);
+                        }
+                        if (dst32 != d02s) { kind = PK_EXT; thr = dst32; m3on = 0; havev = false; }
+                    }
+                    cit++;
+                } else if (kind == PK_EXT) {
+                    havev = true;
+                } else if (kind == PK_GSCORE) {
+                    done = true;
+                }
+                if (havev) {
+                    if (cit >= NMAXCONVIT + 2 || converged16(v, lastv, CM_MAX) || v[15] < 1.0f) done = true;
+                    else solve = true;
+                }
+                if (solve) {
+#pragma unroll
+                    for (int f = 0; f < 16; f++) lastv[f * CM_MAX] = v[f];
+                    float t2[12];
+                    solve_sums(v, swap, t2);
+#pragma unroll
+                    for (int f = 0; f < 12; f++) row[f] = t2[f];
+                    if (kind == PK_FRAG) { thr = d02s; m3on = 1; cit = 0; pd02 = d02; pchk = chk; }
+                    else { thr = thr2; m3on = 0; }
+                    kind = PK_SCORE;
+                }
+                if (done) {
+                    if (kind != PK_GSCORE && gscore && best >= 0.f && (MODE != RM_PLOG || best > best_init)) {
+                        // one more pass: the variant's best transform scored with the
+                        // d0 of the longer structure
+#pragma unroll
+                        for (int f = 0; f < 12; f++) row[f] = tbs[f * CM_MAX];
+                        kind = PK_GSCORE; pd02 = g02; pchk = 0; m3on = 0;
+                    } else {
+                        const float gbest = kind == PK_GSCORE ? sc : best;
+                        if (best > 0.f && (lbest < best || (lbest == best && si < lsi))) {
+                            lbest = best; lgbest = gbest; lsi = si; lndx = vndx; lpos = vpos;
+#pragma unroll
+                            for (int f = 0; f < 12; f++) tbest[f * CM_MAX] = tbs[f * CM_MAX];
+                        }
+                        need = true;
+                        kind = PK_IDLE;
+                    }
+                }
+            }
+        }
+        if (T.work) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) vis += __shfl_xor_sync(FULL, vis, o);
+            if (lane == 0) work_add(T, WK_REFINE, vis);
+        }
+        // the warp's winner, then the CTA's: larger score, then lower variant index
+        float wb = lbest;
+        int wsi = lsi, wl = lane;
+#pragma unroll
+        for (int o = CM_MAX / 2; o > 0; o >>= 1) {
+            const float ob = __shfl_xor_sync(FULL, wb, o);
+            const int os = __shfl_xor_sync(FULL, wsi, o), ol = __shfl_xor_sync(FULL, wl, o);
+            if (ob > wb || (ob == wb && os < wsi)) { wb = ob; wsi = os; wl = ol; }
+        }
+        wl = __shfl_sync(FULL, wl, 0);
+        if (lane == wl) {
+            float* x = S.cand + warp * 32;
+            x[0] = lbest;
+            x[1] = __int_as_float(lsi);
+            x[2] = lgbest;
+            x[3] = __int_as_float(lndx);
+            x[4] = __int_as_float(lpos);
+#pragma unroll
+            for (int f = 0; f < 12; f++) x[5 + f] = tbest[f * CM_MAX];
+        }
+        __syncthreads();
+        if (warp == 0) {
+            int k = 0;
+#pragma unroll
+            for (int j = 1; j < CM_WARPS; j++) {
+                const float ob = S.cand[j * 32], cb = S.cand[k * 32];
+                if (ob > cb || (ob == cb && __float_as_int(S.cand[j * 32 + 1]) < __float_as_int(S.cand[k * 32 + 1]))) k = j;
+            }
+            const float* x = S.cand + k * 32;
+            if (C > 1) {
+                // to the first CTA
+                float* dst = cl.map_shared_rank(S.win, 0) + crank * 32;
+                if (lane < 17) dst[lane] = x[lane];
+            } else if (lane == 0) {
+                refine_commit<MODE>(B, T, i, lq, lr, x[0] > 0.f, x[0], x[2], __float_as_int(x[3]),
+                                    __float_as_int(x[4]), x + 5, 1);
+            }
+        }
+        if (C > 1) {
+            cl.sync();
+            if (crank == 0 && threadIdx.x == 0) {
+                int k = 0;
+                for (int j = 1; j < C; j++) {
+                    const float ob = S.win[j * 32], cb = S.win[k * 32];
+                    if (ob > cb || (ob == cb && __float_as_int(S.win[j * 32 + 1]) < __float_as_int(S.win[k * 32 + 1]))) k = j;
+                }
+                const float* x = S.win + k * 32;
+                refine_commit<MODE>(B, T, i, lq, lr, x[0] > 0.f, x[0], x[2], __float_as_int(x[3]),
+                                    __float_as_int(x[4]), x + 5, 1);
+            }
+            cl.sync();                 // the winners are read before the next pair's arrive
+        }
+    }
+}
+
+// npair: pairs the launch may have at most (a lane form's grid)
 template <int LPP, bool LONG, bool WIDE = false>
-static void launch_refine_k(int mode, const Blk& B, const Bat& T, cudaStream_t st) {
+static void launch_refine_k(int mode, const Blk& B, const Bat& T, cudaStream_t st, int npair = 0,
+                            int lo = 0, int hi = 0) {
     constexpr int W = LONG ? RF_WARPS_LONG : RF_WARPS_SHORT;
     // long pairs: at most RLW_GRID CTAs, T.rlw_ctas per pair at a time
     const int nslot = LONG ? std::max(1, std::min(T.rl_nlmax, RLW_GRID / T.rlw_ctas)) : 0;
     const int ng = LONG ? nslot * T.rlw_ctas
-                        : (T.np + (32 / LPP) * W - 1) / ((32 / LPP) * W);
+                        : (npair + (32 / LPP) * W - 1) / ((32 / LPP) * W);
     const int nt = W * 32;
     switch (mode) {
-        case RM_INIT:  k_refine<RM_INIT, LPP, LONG, WIDE><<<ng, nt, 0, st>>>(B, T); break;
-        case RM_DP:    k_refine<RM_DP, LPP, LONG, WIDE><<<ng, nt, 0, st>>>(B, T); break;
-        case RM_FIN1:  k_refine<RM_FIN1, LPP, LONG, WIDE><<<ng, nt, 0, st>>>(B, T); break;
-        case RM_FIN2:  k_refine<RM_FIN2, LPP, LONG, WIDE><<<ng, nt, 0, st>>>(B, T); break;
-        case RM_PROD1: k_refine<RM_PROD1, LPP, LONG, WIDE><<<ng, nt, 0, st>>>(B, T); break;
-        case RM_PROD2: k_refine<RM_PROD2, LPP, LONG, WIDE><<<ng, nt, 0, st>>>(B, T); break;
-        case RM_PLOG:  k_refine<RM_PLOG, LPP, LONG, WIDE><<<ng, nt, 0, st>>>(B, T); break;
+        case RM_INIT:  k_refine<RM_INIT, LPP, LONG, WIDE><<<ng, nt, 0, st>>>(B, T, lo, hi); break;
+        case RM_DP:    k_refine<RM_DP, LPP, LONG, WIDE><<<ng, nt, 0, st>>>(B, T, lo, hi); break;
+        case RM_FIN1:  k_refine<RM_FIN1, LPP, LONG, WIDE><<<ng, nt, 0, st>>>(B, T, lo, hi); break;
+        case RM_FIN2:  k_refine<RM_FIN2, LPP, LONG, WIDE><<<ng, nt, 0, st>>>(B, T, lo, hi); break;
+        case RM_PROD1: k_refine<RM_PROD1, LPP, LONG, WIDE><<<ng, nt, 0, st>>>(B, T, lo, hi); break;
+        case RM_PROD2: k_refine<RM_PROD2, LPP, LONG, WIDE><<<ng, nt, 0, st>>>(B, T, lo, hi); break;
+        case RM_PLOG:  k_refine<RM_PLOG, LPP, LONG, WIDE><<<ng, nt, 0, st>>>(B, T, lo, hi); break;
     }
+}
+
+// A warp to a pass: the listed pairs with lo <= n < hi (at most npair of
+// them), a cluster of C CTAs a pair.
+static void launch_refine_coop(int mode, const Blk& B, const Bat& T, cudaStream_t st, int npair,
+                               int lo, int hi, int C) {
+    const int nmax = std::min(hi - 1, std::min(B.qmax, B.rmax));
+    if (npair <= 0 || nmax < lo) return;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(std::min(npair, RC_GRID / C) * C);
+    cfg.blockDim = dim3(CM_WARPS * 32);
+    cfg.dynamicSmemBytes = coop_smem_bytes(nmax);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = C;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = C > 1 ? 1 : 0;
+    cudaError_t e = cudaErrorInvalidValue;
+    switch (mode) {
+        case RM_INIT:  e = cudaLaunchKernelEx(&cfg, k_refine_coop<RM_INIT>, B, T, lo, hi); break;
+        case RM_DP:    e = cudaLaunchKernelEx(&cfg, k_refine_coop<RM_DP>, B, T, lo, hi); break;
+        case RM_FIN1:  e = cudaLaunchKernelEx(&cfg, k_refine_coop<RM_FIN1>, B, T, lo, hi); break;
+        case RM_FIN2:  e = cudaLaunchKernelEx(&cfg, k_refine_coop<RM_FIN2>, B, T, lo, hi); break;
+        case RM_PROD1: e = cudaLaunchKernelEx(&cfg, k_refine_coop<RM_PROD1>, B, T, lo, hi); break;
+        case RM_PROD2: e = cudaLaunchKernelEx(&cfg, k_refine_coop<RM_PROD2>, B, T, lo, hi); break;
+        case RM_PLOG:  e = cudaLaunchKernelEx(&cfg, k_refine_coop<RM_PLOG>, B, T, lo, hi); break;
+    }
+    if (e != cudaSuccess && T.lerr && *T.lerr == cudaSuccess) *T.lerr = e;
+    GTB_LAUNCHED(T);
 }
 
 // The refinement kernels re-read each pair's positions on every pass: ask
@@ -1553,9 +2039,14 @@ static void carve_refine() {
 
 void configure_kernels() {
     carve_refine<16, false>();
-    carve_refine<32, false>();
     carve_refine<32, true>();
     carve_refine<32, true, true>();
+    const void* kc[7] = {(const void*)k_refine_coop<RM_INIT>, (const void*)k_refine_coop<RM_DP>,
+                         (const void*)k_refine_coop<RM_FIN1>, (const void*)k_refine_coop<RM_FIN2>,
+                         (const void*)k_refine_coop<RM_PROD1>, (const void*)k_refine_coop<RM_PROD2>,
+                         (const void*)k_refine_coop<RM_PLOG>};
+    for (const void* k : kc)
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)coop_smem_bytes(RL_LONG - 1));
     float gs[GTB_GONNET_NA * GTB_GONNET_NA];
     gtb_gonnet_scores(gs);
     cudaMemcpyToSymbol(g_gonnet, gs, sizeof(gs));
@@ -1575,55 +2066,46 @@ static void launch_refine_long_fin(int mode, const Blk& B, const Bat& T, cudaStr
 }
 
 void launch_refine(int mode, const Blk& B, const Bat& T0, cudaStream_t st, bool few) {
-    // the long-pair path: from RL_LONG positions with T0.rlw_ctas CTAs; where
-    // few pairs take part (the launches after the --pre-score filter) a
-    // launch lasts as long as its slowest pair, so there the pairs from
-    // RL_LONG_FEW positions below that get RLW_CTAS_FEW CTAs (second tier)
     Bat T = T0;
     T.rl_min = RL_LONG;
     T.rlw_ctas = T0.rlw_ctas > 0 && T0.rlw_ctas <= RLW_CTAS_MAX ? T0.rlw_ctas : RLW_CTAS;
-    T.rl_min2 = RL_LONG_FEW;
-    T.rlw_ctas2 = T0.rlw_ctas2 > 0 && T0.rlw_ctas2 <= RLW_CTAS_MAX ? T0.rlw_ctas2 : RLW_CTAS_FEW;
-    if (!few) T.rl_long2 = nullptr;
     cudaMemsetAsync(T.rhist, 0, (RL_NB + 1) * sizeof(int), st);
     if (T.rl_long) {
         cudaMemsetAsync(T.rl_count, 0, sizeof(int), st);
         cudaMemsetAsync(T.rl_next, 0, (size_t)T.rl_nlmax * sizeof(int), st);
     }
-    if (T.rl_long2) {
-        cudaMemsetAsync(T.rl_count2, 0, sizeof(int), st);
-        cudaMemsetAsync(T.rl_next2, 0, (size_t)T.rl_nlmax2 * sizeof(int), st);
-    }
     const int nb = (T.np + 255) / 256;
     k_rlist_count<<<nb, 256, 0, st>>>(B, T, mode);
     k_rlist_scan<<<1, 1024, 0, st>>>(T);
     k_rlist_fill<<<nb, 256, 0, st>>>(B, T, mode);
-    // the long pairs on the second stream, beside the short ones (both read
-    // the lists built above; they write disjoint pairs)
-    const bool fork = T.st2 && (T.rl_long || T.rl_long2);
+    if (T.launches) (*T.launches) += 3;
+    // The longer pairs' launches on the second stream, beside the shorter
+    // ones' (all read the lists built above; they write disjoint pairs)
+    const bool fork = T.st2 && (T.rl_long || T.nml[2] > 0);
     cudaStream_t sl = fork ? T.st2 : st;
     KtScope kts(T, KF_REFINE, st);   // on st, after the join: both streams' time
     if (fork) {
         cudaEventRecord(T.evfork, st);
         cudaStreamWaitEvent(T.st2, T.evfork, 0);
     }
-    if (few) launch_refine_k<32, false>(mode, B, T, st);
-    else launch_refine_k<16, false>(mode, B, T, st);
-    if (T.launches) (*T.launches) += 4;
     if (T.rl_long) {
         if (T.rl_nlmax <= RLW_WIDE_MAX) launch_refine_k<32, true, true>(mode, B, T, sl);
         else launch_refine_k<32, true>(mode, B, T, sl);
         launch_refine_long_fin(mode, B, T, sl);
         if (T.launches) (*T.launches) += 2;
+    } else if (T.nml[3] > 0) {
+        launch_refine_k<16, false>(mode, B, T, sl, T.nml[3], RL_LONG, 0);
+        GTB_LAUNCHED(T);
     }
-    if (T.rl_long2) {
-        // the second tier through the same kernels, on its own list
-        Bat T2 = T;
-        T2.rl_long = T.rl_long2; T2.rl_count = T.rl_count2; T2.rl_next = T.rl_next2;
-        T2.rl_cand = T.rl_cand2; T2.rl_nlmax = T.rl_nlmax2; T2.rlw_ctas = T.rlw_ctas2;
-        launch_refine_k<32, true>(mode, B, T2, sl);
-        launch_refine_long_fin(mode, B, T2, sl);
-        if (T.launches) (*T.launches) += 2;
+    const bool coop = few || T.np <= RC_SMALL;
+    launch_refine_coop(mode, B, T, sl, T.nml[2], RC_N2, RL_LONG, 8);
+    if (coop) {
+        const int c = T.np <= RC_NP8 ? 8 : T.np <= RC_NP4 ? 4 : T.np <= RC_NP2 ? 2 : 1;
+        launch_refine_coop(mode, B, T, st, T.nml[1], RC_N1, RC_N2, c < 4 ? 4 : c);
+        launch_refine_coop(mode, B, T, st, T.np, 0, RC_N1, c);
+    } else {
+        launch_refine_k<16, false>(mode, B, T, st, T.np, 0, RC_N2);
+        GTB_LAUNCHED(T);
     }
     if (fork) {
         cudaEventRecord(T.evjoin, T.st2);

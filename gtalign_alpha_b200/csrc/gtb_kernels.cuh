@@ -13,16 +13,25 @@ namespace gtb {
 // 16/R consecutive steps into one 32-bit word, words of a strip stored
 // [step / (16/R)][lane].
 // refinement: pairs with at least RL_LONG positions get RLW_CTAS CTAs of 4
-// warps; in the launches where few pairs take part, the pairs below that
-// with at least RL_LONG_FEW positions get RLW_CTAS_FEW; a long-pair launch
-// has at most RLW_GRID CTAs (they walk the long pairs).  When a sub-batch
-// has few pairs of a tier, each gets more CTAs (rlw_ctas_for), up to
-// RLW_CTAS_MAX: a lone long pair has variants for many more warps.
+// warps; a long-pair launch has at most RLW_GRID CTAs (they walk the long
+// pairs).  When a sub-batch has few long pairs, each gets more CTAs
+// (rlw_ctas_for), up to RLW_CTAS_MAX: a lone long pair has variants for many
+// more warps.
 constexpr int RL_LONG = 1536;
-constexpr int RL_LONG_FEW = 384;
+// The warp-a-pass form (k_refine_coop).  It takes every pair where few take
+// part or the batch has at most RC_SMALL pairs: a solve serves 8 variants there
+// against the lane form's 32, so that with the GPU full the lane form is the
+// faster (all launches of 16 x 500 by warps 58 against 54 ms, of 2 x 20,000
+// 123 against 100; of 1 x 1,000 by lanes 12.4 against 11.4).  From RC_N2
+// positions it always does (the lane form's slowest pair sets the launch's
+// time).  CTAs per pair: 8 from RC_N2, at least 4 from RC_N1 (2 and 8: within
+// 4% either way), else by the pairs of the batch (with one CTA instead of two
+// 16 x 500 takes twice as long; 4 for 1,000 pairs 13.9 against 11.4 ms).
+constexpr int RC_N1 = 256, RC_N2 = 512;
+constexpr int RC_SMALL = 2048, RC_NP8 = 64, RC_NP4 = 256, RC_NP2 = 4096;
+constexpr int RC_GRID = 1184;         // CTAs of a launch at most
 constexpr int RL_NBUCKET = 65536 >> 4;   // work-list buckets; rhist[RL_NBUCKET] = list length
 constexpr int RLW_CTAS = 16;
-constexpr int RLW_CTAS_FEW = 4;
 constexpr int RLW_GRID = 1024;
 constexpr int RLW_CTAS_MAX = 256;
 constexpr int RLW_CTA_WARPS = 4;     // warps of a long-pair CTA (one candidate each)
@@ -121,18 +130,15 @@ struct Bat {
     int *rlist, *rhist;              // refinement work list [np], buckets [4097]
     // long pairs of a refinement launch (null: none possible): list, count,
     // per-pair variant counter, per-warp candidates; rl_nlmax = capacity;
-    // this launch's threshold and CTAs per long pair.  The second set (the
-    // same fields with 2) is a lower tier, pairs from rl_min2 positions with
-    // rlw_ctas2 CTAs each, used in the launches after the --pre-score filter
-    // (null rl_long2: no second tier in this launch).  The caller's rlw_ctas
-    // is the first tier's CTAs per pair (0: RLW_CTAS)
+    // this launch's threshold and CTAs per long pair.  The caller's rlw_ctas
+    // is the CTAs per pair (0: RLW_CTAS)
     int rl_nlmax;
     int rl_min, rlw_ctas;
     int *rl_long, *rl_count, *rl_next;
     float* rl_cand;
-    int rl_nlmax2, rl_min2, rlw_ctas2;
-    int *rl_long2, *rl_count2, *rl_next2;
-    float* rl_cand2;
+    // host: pairs whose shorter structure has at least 0, RC_N1, RC_N2, RL_LONG
+    // residues (bounds of the refinement launches' grids)
+    int nml[4];
     int plog_round;                  // round of an RM_PLOG launch (0 .. PLOG_ROUNDS-1)
     // host: a second stream for a refinement launch's long pairs, which then
     // run beside its short pairs (fork and join events; null: one stream)

@@ -173,8 +173,11 @@ extern "C" gtb_status gtb_process_block_noalloc(int device, const gtb_options* o
     long long* oaln = h_offs + 2 * (np + 1);
     long long* ostr = h_offs + 3 * (np + 1);
     obt[0] = orow[0] = oaln[0] = ostr[0] = 0;
+    int nml[4] = {np, 0, 0, 0};      // pairs of the refinement's length classes
     for (int i = 0; i < np; i++) {
         int lq = q->lens[i / r->n], lr = r->lens[i % r->n];
+        const int ml = lq < lr ? lq : lr;
+        nml[1] += ml >= RC_N1; nml[2] += ml >= RC_N2; nml[3] += ml >= RL_LONG;
         obt[i + 1] = obt[i] + gtb::bt_words(lq, lr);
         orow[i + 1] = orow[i] + lr;
         oaln[i + 1] = oaln[i] + (lq < lr ? lq : lr);
@@ -278,6 +281,7 @@ extern "C" gtb_status gtb_process_block_noalloc(int device, const gtb_options* o
     T.nff = np; T.ff_pair = nullptr; T.ff_chunk = nullptr; T.ff_nch = nullptr; T.ff_key = nullptr;
     T.launches = nullptr;
     T.alt_rci = -1;
+    for (int k = 0; k < 4; k++) T.nml[k] = nml[k];
 
     // the host offsets are copied from the static host array (no allocation)
     e = cudaMemcpyAsync(offs, h_offs, (size_t)(np + 1) * 4 * sizeof(long long), cudaMemcpyHostToDevice, st);

@@ -337,3 +337,22 @@ def test_far_residues(oracle, far):
     r.y[r.offs[3] + 11] = -far
     res, ora = run_both(oracle, q, r, OPTSETS["speed13"])
     assert_same(res, ora, q.n, r.n)
+
+
+@pytest.mark.parametrize("lens,fill", [((31, 32, 33, 127, 128, 129, 255, 256, 257), 0),
+                                       ((511, 512, 513), 70), ((129, 257, 513), 300),
+                                       ((33, 255, 512), 2100), ((1535, 1536), 0)])
+def test_refinement_length_classes(oracle, lens, fill):
+    """Pairs whose alignments end at the edges of blocks and of the
+    refinement's length classes, in batches of each size class (`fill` short
+    structures make up the number): GPU against the oracle bit for bit."""
+    from gtalign_alpha_b200 import synth
+    rng = np.random.default_rng(sum(lens))
+    q = synth.random_chains(rng, [max(lens)], "q")
+    r = [synth.homolog(rng, synth.Chain(q[0].xyz[:n], q[0].seq[:n], "t"), 1.0, 0.0, "h%d" % n) for n in lens]
+    r += synth.random_chains(rng, rng.integers(20, 30, fill), "f")
+    q, r = synth.pack(q), synth.pack(r)
+    d = dict(OPTSETS["speed13" if max(lens) > 600 or fill else "default"], convergence=2)
+    res, ora = run_both(oracle, q, r, d)
+    assert_same(res, ora, q.n, r.n)
+    assert (res.alndata[0, :len(lens), 4] >= np.array(lens) - 2).all()
