@@ -853,7 +853,7 @@ static gtb_status upload_block(gtb_handle* h, const HostSoA& S, gtb_block* b,
     CK(cudaMemcpyAsync(b->z, S.z, S.npos * 4, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(b->rsd, S.rsd, S.npos, cudaMemcpyHostToDevice, st));
     long long nl = 0;
-    launch_pack4(b->c4, b->x, b->y, b->z, S.npos, st);
+    launch_pack4_structs(b->c4, b->x, b->y, b->z, b->doff, b->dlen, b->doff, b->n, st);
     launch_secstr(b->ss, b->x, b->y, b->z, b->dlen, b->doff, b->dmol, b->n, st, &nl);
     if (ndx)
         launch_pack_nodes(b->nd, b->nc, b->nx, b->ny, b->nz, b->nl, b->nr, b->no, b->doff, b->dlen,

@@ -167,25 +167,31 @@ void launch_secstr(char* ss, const float* x, const float* y, const float* z,
 }
 
 // ---------------------------------------------------------------------------
-__global__ void k_pack4(float4* out, const float* x, const float* y, const float* z, long long n) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = make_float4(x[i], y[i], z[i], 0.f);
-}
-
-void launch_pack4(float4* out, const float* x, const float* y, const float* z, long long n,
-                  cudaStream_t st) {
-    if (n <= 0) return;
-    k_pack4<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(out, x, y, z, n);
-}
-
+// A structure's residues as (x, y, z, 0); its first residue's w is 1 when some
+// coordinate is not ordinary: not a number, or above 10^9, from where on squared
+// distances could leave the range that the DP's fast form takes.
 __global__ void k_pack4s(float4* out, const float* x, const float* y, const float* z,
                          const int* off, const int* len, const int* coff, int n) {
     int si = blockIdx.x;
     if (si >= n) return;
     int o = off[si], L = len[si], c = coff[si];
-    for (int p = threadIdx.x; p < L; p += blockDim.x)
-        out[c + p] = make_float4(x[o + p], y[o + p], z[o + p], 0.f);
+    float4 v0 = make_float4(0.f, 0.f, 0.f, 0.f);
+    bool odd = false;
+    for (int p = threadIdx.x; p < L; p += blockDim.x) {
+        const float4 v = make_float4(x[o + p], y[o + p], z[o + p], 0.f);
+        odd = odd || !(fabsf(v.x) <= 1.e9f && fabsf(v.y) <= 1.e9f && fabsf(v.z) <= 1.e9f);
+        if (p == 0) v0 = v;
+        else out[c + p] = v;
+    }
+    odd = __syncthreads_or(odd);
+    if (threadIdx.x == 0) {
+        v0.w = odd ? 1.f : 0.f;
+        out[c] = v0;
+    }
 }
+
+// c4: a structure's first residue
+__device__ __forceinline__ bool coords_ordinary(const float4* c4) { return __ldg(&c4->w) == 0.f; }
 
 void launch_pack4_structs(float4* out, const float* x, const float* y, const float* z,
                           const int* off, const int* len, const int* coff, int n,
@@ -2134,6 +2140,8 @@ void launch_refine(int mode, const Blk& B, const Bat& T0, cudaStream_t st, bool 
 // value + DPSS_C, a reader takes the offset off again, the gap cost is paid
 // once when leaving such a cell; the border reads as a diagonal cell of 0).
 // SCOREONLY: no traceback words; the last cell's value goes to *fin.
+// This form takes any coordinates and the --add-search-by-ss score; the others
+// run dp_pair_fast.
 template <int R, bool gap0, int SC, bool WAVE, bool SCOREONLY = false>
 __device__ __forceinline__ bool dp_pair(const float* t, float d02, float gcost, int lq, int lr,
                                         const float* qx, const float* qy, const float* qz,
@@ -2220,14 +2228,14 @@ __device__ __forceinline__ bool dp_pair(const float* t, float d02, float gcost, 
                             if (ssrr && (!CHK || r < nv)) {
                                 float v = __fmaf_rn(gonnet(qaa[r], cra), 0.2f, (float)(qss[r] == css));
                                 v = __fadd_rn(v, dg < DPSS_CMP ? __fsub_rn(dg, DPSS_C) : dg);
-                                int bk = BT_DIAG;
+                                int bk = BTW_DIAG;
                                 float l = h[r];
                                 if (l < DPSS_CMP) l = __fsub_rn(__fadd_rn(gcost, l), DPSS_C);
-                                if (v < l) { v = l; bk = BT_LEFT; }
+                                if (v < l) { v = l; bk = BTW_LEFT; }
                                 float uu = up;
                                 if (uu < DPSS_CMP) uu = __fsub_rn(__fadd_rn(gcost, uu), DPSS_C);
-                                if (v < uu) { v = uu; bk = BT_UP; }
-                                float w = bk == BT_DIAG ? __fadd_rn(v, DPSS_C) : v;
+                                if (v < uu) { v = uu; bk = BTW_UP; }
+                                float w = bk == BTW_DIAG ? __fadd_rn(v, DPSS_C) : v;
                                 dg = h[r];
                                 up = w;
                                 h[r] = w;
@@ -2236,14 +2244,14 @@ __device__ __forceinline__ bool dp_pair(const float* t, float d02, float gcost, 
                                 float v = tmterm(d02, dist2(tx[r], ty[r], tz[r], c4.x, c4.y, c4.z));
                                 if (usess) v = __fadd_rn(v, __fmul_rn((float)(qss[r] == css), 0.5f));
                                 v = __fadd_rn(v, gap0 ? dg : fabsf(dg));
-                                int bk = BT_DIAG;
+                                int bk = BTW_DIAG;
                                 float l = h[r];
                                 if (!gap0 && l < 0.f) l = __fsub_rn(gcost, l);
-                                if (v < l) { v = l; bk = BT_LEFT; }
+                                if (v < l) { v = l; bk = BTW_LEFT; }
                                 float uu = up;
                                 if (!gap0 && uu < 0.f) uu = __fsub_rn(gcost, uu);
-                                if (v < uu) { v = uu; bk = BT_UP; }
-                                float w = (gap0 || bk != BT_DIAG) ? v : -v;
+                                if (v < uu) { v = uu; bk = BTW_UP; }
+                                float w = (gap0 || bk != BTW_DIAG) ? v : -v;
                                 dg = h[r];   // (row r, j-1): the next row's diagonal
                                 up = w;      // (row r, j):   the next row's up
                                 h[r] = w;
@@ -2273,6 +2281,181 @@ __device__ __forceinline__ bool dp_pair(const float* t, float d02, float gcost, 
     return true;
 }
 
+// The DP of a pair whose coordinates are ordinary (coords_ordinary), cell
+// scores DP_SC_TFM and DP_SC_TFMSS: the values and directions of dp_pair.
+// A lone warp of dp_pair took ~600 cycles a step (R cells a lane): each cell's
+// score was computed inside the chain of cell values.  Here the score terms
+// of a group of steps (16 cells a lane) come first, two steps to a packed
+// FP32 operation, and the chain that is left is a shuffle and, per row, one
+// maximum (and, with a gap cost, the choice of what a neighbour sees).
+//  * The reference's coordinates go through a ring of 64 columns in shared
+//    memory, kept twice, the second time shifted by one, so that every lane
+//    reads the pairs of columns (j, j+1) of its steps as 8 aligned bytes.
+//  * Rows past the query's end and columns past the reference's are computed
+//    and never read; before the first column the terms are -inf (stored negated), which leaves
+//    the zeros of the border in place.
+//  * With a gap cost a cell keeps its value and what its right and lower
+//    neighbours see: the value + gap cost if it was reached diagonally.  In the
+//    row buffer a diagonally reached value is negative, as in dp_pair.
+// What bounds it: a lone pair, the chain; a full GPU, issue.
+constexpr int DPR_W = 64;                    // columns of a warp's ring
+struct DpRing { float c[2][3][DPR_W]; };
+
+template <int R, bool gap0, int SC, bool WAVE, bool SCOREONLY>
+__device__ __forceinline__ bool dp_pair_fast(const float* t, float d02, float gcost, int lq, int lr,
+                                             const float4* q4, const float4* r4, const char* qs,
+                                             const char* rs, float* row, unsigned* bt, DpRing& ring,
+                                             int lane, int s_first = 0, int s_step = 1,
+                                             volatile int* prog = nullptr,
+                                             volatile int* err = nullptr,
+                                             long long spin = DP_WAVE_SPIN_DEFAULT,
+                                             float* fin = nullptr, bool cta_wave = false) {
+    constexpr bool usess = SC == DP_SC_TFMSS;
+    constexpr int ROWS = 32 * R, SPW = 16 / R;
+    const unsigned FULL = 0xffffffffu;
+    const float INF = __int_as_float(0x7f800000);
+    const int ngrp = (lr + 31 + SPW - 1) / SPW;
+    const int nstrips = (lq + ROWS - 1) / ROWS;
+    const f32x2 D02 = pack2(d02, d02), ONE = pack2(1.f, 1.f);
+    const float* cx = ring.c[lane & 1][0];
+    const int codd = (lane & 1) - lane;      // a lane's column pairs in its copy: t + codd, even
+    for (int s = s_first; s < nstrips; s += s_step) {
+        f32x2 nx[R], ny[R], nz[R];
+        float h[R], e[R];                    // (row, j-1): value; what a neighbour sees (gap cost)
+        char qss[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const int irow = s * ROWS + lane * R + r;
+            float x = 0.f, y = 0.f, z = 0.f;
+            qss[r] = 0;
+            h[r] = e[r] = 0.f;
+            if (irow < lq) {
+                const float4 q = __ldg(q4 + irow);
+                xform(t, q.x, q.y, q.z, x, y, z);
+                if (usess) qss[r] = qs[irow];
+            }
+            nx[r] = pack2(-x, -x); ny[r] = pack2(-y, -y); nz[r] = pack2(-z, -z);
+        }
+        float hup = 0.f;                     // (first row - 1, j-1)
+        float rb = 0.f;
+        float4 cn = lane < lr ? __ldg(r4 + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+        unsigned* bts = SCOREONLY ? nullptr : bt + (long long)s * ngrp * 32 + lane;
+        const int lastr = (lq - 1) - s * ROWS - lane * R;   // the last row among this lane's (if 0..R-1)
+        __syncwarp();
+        for (int g = 0; g < ngrp; g++) {
+            const int t0 = g * SPW;
+            if ((t0 & 31) == 0) {
+                if (WAVE && s > 0) {
+                    // row[t0 .. t0+31] of strip s-1: written up to its step t0+62
+                    const int need = t0 + 64 < ngrp * SPW ? t0 + 64 : ngrp * SPW;
+                    int ok = 1;
+                    if (lane == 0) {
+                        long long it = 0;
+                        while (prog[s - 1] < need) {
+                            if (*err || ++it > spin) { *err = 1; ok = 0; break; }
+                            __nanosleep(32);
+                        }
+                    }
+                    ok = __shfl_sync(FULL, ok, 0);
+                    if (cta_wave) __threadfence_block();
+                    else __threadfence();
+                    if (!ok) return false;
+                }
+                const int jj = t0 + lane;
+                if (s > 0) rb = jj < lr ? (WAVE ? __ldcg(row + jj) : row[jj]) : 0.f;
+                // these 32 columns into the ring, the next 32 on their way
+                const int a = jj & (DPR_W - 1), b = (jj + 1) & (DPR_W - 1);
+                ring.c[0][0][a] = cn.x; ring.c[0][1][a] = cn.y; ring.c[0][2][a] = cn.z;
+                ring.c[1][0][b] = cn.x; ring.c[1][1][b] = cn.y; ring.c[1][2][b] = cn.z;
+                __syncwarp();
+                if (jj + 32 < lr) cn = __ldg(r4 + jj + 32);
+            }
+            float nt[SPW][R];                // the negated score terms
+#pragma unroll
+            for (int u = 0; u < SPW; u += 2) {
+                const int o = (t0 + u + codd) & (DPR_W - 1);
+                const float2 x2 = *(const float2*)(cx + o), y2 = *(const float2*)(cx + DPR_W + o),
+                             z2 = *(const float2*)(cx + 2 * DPR_W + o);
+                const f32x2 X = pack2(x2.x, x2.y), Y = pack2(y2.x, y2.y), Z = pack2(z2.x, z2.y);
+                char c0 = 0, c1 = 0;
+                if (usess) {
+                    const int j = t0 + u - lane;
+                    c0 = j >= 0 && j < lr ? rs[j] : 0;
+                    c1 = j + 1 >= 0 && j + 1 < lr ? rs[j + 1] : 0;
+                }
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    const f32x2 dx = add2(X, nx[r]), dy = add2(Y, ny[r]), dz = add2(Z, nz[r]);
+                    const f32x2 b = add2(D02, fma2(dx, dx, fma2(dy, dy, mul2(dz, dz))));
+                    unpack2(div2_neg(D02, b, ONE), nt[u][r], nt[u + 1][r]);
+                    if (usess) {
+                        nt[u][r] = __fsub_rn(nt[u][r], qss[r] == c0 ? 0.5f : 0.f);
+                        nt[u + 1][r] = __fsub_rn(nt[u + 1][r], qss[r] == c1 ? 0.5f : 0.f);
+                    }
+                }
+            }
+            if (t0 < 31) {
+#pragma unroll
+                for (int u = 0; u < SPW; u++)
+                    if (t0 + u < lane) {
+#pragma unroll
+                        for (int r = 0; r < R; r++) nt[u][r] = INF;
+                    }
+            }
+            unsigned acc = 0u;
+#pragma unroll
+            for (int u = 0; u < SPW; u++) {
+                const int tt = t0 + u;
+                const float r0 = __shfl_sync(FULL, rb, tt & 31);
+                float hu = __shfl_up_sync(FULL, h[R - 1], 1), eu = 0.f;
+                if (gap0) {
+                    if (lane == 0) hu = r0;
+                } else {
+                    eu = __shfl_up_sync(FULL, e[R - 1], 1);
+                    if (lane == 0) { hu = fabsf(r0); eu = r0 < 0.f ? __fsub_rn(gcost, r0) : r0; }
+                }
+                float dg = hup;
+                hup = hu;
+                float up = gap0 ? hu : eu;
+                bool diag = false;           // the last row's cell was reached diagonally
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    const float v = __fsub_rn(dg, nt[u][r]);
+                    const float l = gap0 ? h[r] : e[r];
+                    const bool p1 = v < l;                        // left rather than diagonal
+                    const float m = fmaxf(v, l);
+                    const bool p2 = m < up;                       // up rather than either
+                    const float w = fmaxf(m, up);
+                    if (!SCOREONLY) {
+                        if (p1) acc |= 1u << (2 * R * u + 2 * r);
+                        if (p2) acc |= 2u << (2 * R * u + 2 * r);
+                    }
+                    dg = h[r];
+                    h[r] = w;
+                    if (gap0) up = w;
+                    else {
+                        diag = !(p1 || p2);
+                        e[r] = diag ? __fadd_rn(gcost, w) : w;
+                        up = e[r];
+                    }
+                    if (SCOREONLY && t0 + SPW >= lr && r == lastr && tt - lane == lr - 1) *fin = w;
+                }
+                if (lane == 31 && tt >= 31 && tt - 31 < lr) row[tt - 31] = diag ? -h[R - 1] : h[R - 1];
+            }
+            if (!SCOREONLY) bts[g * 32] = acc;
+            // the count is published at every 32nd step, when the next strip
+            // may read 32 more columns, and at the end
+            if (WAVE && lane == 31 && (((t0 + SPW) & 31) == 0 || g == ngrp - 1)) {
+                if (cta_wave) __threadfence_block();       // the row values before the count
+                else __threadfence();
+                prog[s] = t0 + SPW;
+            }
+        }
+        __syncwarp();
+    }
+    return true;
+}
+
 // The DP work list (k_dlist_*, largest matrices first): its first dp_kc
 // pairs take a CTA each, whose 4 warps run the pair's strips as a wavefront
 // (strip s on warp s mod 4, each strip waiting with a bounded spin until the
@@ -2282,6 +2465,7 @@ template <int GAP0, int SC>
 __global__ void __launch_bounds__(128) k_dp(Blk B, Bat T, int tfmsrc, float gcost, int dpscan,
                                             int skipmode) {
     __shared__ int s_prog[DP_CTA_MAXSTRIPS];
+    __shared__ DpRing s_ring[4];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int len = T.rhist[RL_NB];
     const int dkc = T.dw_err ? T.dp_kc : 0;
@@ -2304,7 +2488,9 @@ __global__ void __launch_bounds__(128) k_dp(Blk B, Bat T, int tfmsrc, float gcos
     const float* qx = B.qx + B.qoff[qi];
     const float* qy = B.qy + B.qoff[qi];
     const float* qz = B.qz + B.qoff[qi];
+    const float4* q4 = B.q4 + B.q4off[qi];
     const float4* r4 = B.r4 + B.r4off[ri];
+    const bool fast = SC != DP_SC_SSRR && coords_ordinary(q4) && coords_ordinary(r4);
     const char* qs = B.qs + B.qoff[qi];
     const char* rs = B.rs + B.roff[ri];
     float* row = T.row + T.off_row[i];
@@ -2316,6 +2502,17 @@ __global__ void __launch_bounds__(128) k_dp(Blk B, Bat T, int tfmsrc, float gcos
         if (dp_strips(lq) > 1) {
             for (int k = threadIdx.x; k < DP_CTA_MAXSTRIPS; k += blockDim.x) s_prog[k] = 0;
             __syncthreads();
+            if (fast) {
+                if (dp_r(lq) == 4)
+                    dp_pair_fast<4, GAP0 != 0, SC, true, false>(t, d02, gcost, lq, lr, q4, r4, qs, rs, row, bt,
+                                                                s_ring[w], lane, w, blockDim.x >> 5, s_prog,
+                                                                T.dw_err, T.dw_spin, nullptr, true);
+                else
+                    dp_pair_fast<2, GAP0 != 0, SC, true, false>(t, d02, gcost, lq, lr, q4, r4, qs, rs, row, bt,
+                                                                s_ring[w], lane, w, blockDim.x >> 5, s_prog,
+                                                                T.dw_err, T.dw_spin, nullptr, true);
+                return;
+            }
             if (dp_r(lq) == 4)
                 dp_pair<4, GAP0 != 0, SC, true>(t, d02, gcost, lq, lr, qx, qy, qz, r4, qs, rs, qa, ra, row,
                                                 bt, lane, w, blockDim.x >> 5, s_prog, T.dw_err, T.dw_spin,
@@ -2330,6 +2527,15 @@ __global__ void __launch_bounds__(128) k_dp(Blk B, Bat T, int tfmsrc, float gcos
     } else if (lane == 0) {
         work_add(T, WK_DPCELL, (unsigned long long)lq * (unsigned long long)lr);
     }
+    if (fast) {
+        if (dp_r(lq) == 4)
+            dp_pair_fast<4, GAP0 != 0, SC, false, false>(t, d02, gcost, lq, lr, q4, r4, qs, rs, row, bt,
+                                                         s_ring[w], lane);
+        else
+            dp_pair_fast<2, GAP0 != 0, SC, false, false>(t, d02, gcost, lq, lr, q4, r4, qs, rs, row, bt,
+                                                         s_ring[w], lane);
+        return;
+    }
     if (dp_r(lq) == 4)
         dp_pair<4, GAP0 != 0, SC, false>(t, d02, gcost, lq, lr, qx, qy, qz, r4, qs, rs, qa, ra, row, bt, lane);
     else
@@ -2341,6 +2547,7 @@ __global__ void __launch_bounds__(128) k_dp(Blk B, Bat T, int tfmsrc, float gcos
 template <int GAP0, int SC>
 __global__ void __launch_bounds__(32) k_dp_wave(Blk B, Bat T, int tfmsrc, float gcost, int dpscan,
                                                 int skipmode) {
+    __shared__ DpRing s_ring;
     const int lane = threadIdx.x & 31;
     const int item = blockIdx.x;
     if (item >= T.ndw) return;
@@ -2364,7 +2571,9 @@ __global__ void __launch_bounds__(32) k_dp_wave(Blk B, Bat T, int tfmsrc, float 
     const float* qx = B.qx + B.qoff[qi];
     const float* qy = B.qy + B.qoff[qi];
     const float* qz = B.qz + B.qoff[qi];
+    const float4* q4 = B.q4 + B.q4off[qi];
     const float4* r4 = B.r4 + B.r4off[ri];
+    const bool fast = SC != DP_SC_SSRR && coords_ordinary(q4) && coords_ordinary(r4);
     const char* qs = B.qs + B.qoff[qi];
     const char* rs = B.rs + B.roff[ri];
     float* row = T.row + T.off_row[i];
@@ -2373,6 +2582,15 @@ __global__ void __launch_bounds__(32) k_dp_wave(Blk B, Bat T, int tfmsrc, float 
     const unsigned char* qa = B.qa + B.qoff[qi];
     const unsigned char* ra = B.ra + B.roff[ri];
     if (lane == 0 && c == 0) work_add(T, WK_DPCELL, (unsigned long long)lq * (unsigned long long)lr);
+    if (fast) {
+        if (dp_r(lq) == 4)
+            dp_pair_fast<4, GAP0 != 0, SC, true, false>(t, d02, gcost, lq, lr, q4, r4, qs, rs, row, bt, s_ring,
+                                                        lane, c, G, prog, T.dw_err, T.dw_spin);
+        else
+            dp_pair_fast<2, GAP0 != 0, SC, true, false>(t, d02, gcost, lq, lr, q4, r4, qs, rs, row, bt, s_ring,
+                                                        lane, c, G, prog, T.dw_err, T.dw_spin);
+        return;
+    }
     if (dp_r(lq) == 4)
         dp_pair<4, GAP0 != 0, SC, true>(t, d02, gcost, lq, lr, qx, qy, qz, r4, qs, rs, qa, ra, row,
                                         bt, lane, c, G, prog, T.dw_err, T.dw_spin);
@@ -2453,7 +2671,9 @@ void launch_pair_list(const Blk& B, const Bat& T, int skipmask, cudaStream_t st)
 // (largest pairs first); each slot's DP keeps its strip row in the pair's
 // detailed-search region (the local score matrix is no longer read).
 __global__ void __launch_bounds__(128) k_f3_dpscore(Blk B, Bat T) {
+    __shared__ DpRing s_ring[4];
     const int lane = threadIdx.x & 31;
+    DpRing& ring = s_ring[threadIdx.x >> 5];
     const int nsl = B.f3nsec * F3_NTOP;          // slots per pair
     const long long nitems = (long long)T.rhist[RL_NB] * nsl;
     const long long wstride = (long long)gridDim.x * (blockDim.x >> 5);
@@ -2475,13 +2695,23 @@ __global__ void __launch_bounds__(128) k_f3_dpscore(Blk B, Bat T) {
         const float* qx = B.qx + B.qoff[qi];
         const float* qy = B.qy + B.qoff[qi];
         const float* qz = B.qz + B.qoff[qi];
+        const float4* q4 = B.q4 + B.q4off[qi];
         const float4* r4 = B.r4 + B.r4off[ri];
         float* row = (float*)(T.lsm + T.off_lsm[i]) + (long long)k * lr;
         float t[12];
 #pragma unroll
         for (int f = 0; f < 12; f++) t[f] = sl[1 + f];
         if (lane == 0) work_add(T, WK_F3CELL, (unsigned long long)lq * (unsigned long long)lr);
-        if (dp_r(lq) == 4)
+        if (coords_ordinary(q4) && coords_ordinary(r4)) {
+            if (dp_r(lq) == 4)
+                dp_pair_fast<4, true, DP_SC_TFM, false, true>(t, d02, 0.f, lq, lr, q4, r4, nullptr, nullptr, row,
+                                                              nullptr, ring, lane, 0, 1, nullptr, nullptr,
+                                                              DP_WAVE_SPIN_DEFAULT, fin);
+            else
+                dp_pair_fast<2, true, DP_SC_TFM, false, true>(t, d02, 0.f, lq, lr, q4, r4, nullptr, nullptr, row,
+                                                              nullptr, ring, lane, 0, 1, nullptr, nullptr,
+                                                              DP_WAVE_SPIN_DEFAULT, fin);
+        } else if (dp_r(lq) == 4)
             dp_pair<4, true, DP_SC_TFM, false, true>(t, d02, 0.f, lq, lr, qx, qy, qz, r4, nullptr,
                                                      nullptr, nullptr, nullptr, row, nullptr, lane,
                                                      0, 1, nullptr, nullptr, DP_WAVE_SPIN_DEFAULT, fin);
@@ -2567,9 +2797,9 @@ __global__ void k_btck(Blk B, Bat T, int constrained) {
             w = bt[wi];
             cwi = wi;
         }
-        int b = (int)((w >> (2 * R * (tt % spw) + 2 * (yy % R))) & 3u);
-        if (b == BT_UP) { y--; continue; }
-        if (b == BT_LEFT) { x--; continue; }
+        const unsigned b = (w >> (2 * R * (tt % spw) + 2 * (yy % R))) & 3u;
+        if (b >= BTW_UP) { y--; continue; }
+        if (b == BTW_LEFT) { x--; continue; }
         float4 cq = __ldg(q4 + y), cr = __ldg(r4 + x);
         float cqx = cq.x, cqy = cq.y, cqz = cq.z, crx = cr.x, cry = cr.y, crz = cr.z;
         bool keep = true;

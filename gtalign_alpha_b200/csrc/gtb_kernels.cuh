@@ -231,11 +231,9 @@ enum DpTfm { DP_TFM_IBEST = 0, DP_TFM_GRAND = 1, DP_TFM_ALT = 2, DP_TFM_2ND = 3 
 void launch_secstr(char* ss, const float* x, const float* y, const float* z,
                    const int* len, const int* off, const int* mol, int nstr,
                    cudaStream_t st, long long* launches);
-// (x, y, z, 0) copies of n coordinates, for single 16-byte loads in the passes
-void launch_pack4(float4* out, const float* x, const float* y, const float* z, long long n,
-                  cudaStream_t st);
-// the same per structure into a back-to-back copy: structure i's residues
-// [off[i], off[i]+len[i]) go to out[coff[i] ...]
+// (x, y, z, 0) copies of the coordinates, for single 16-byte loads in the
+// passes: structure i's residues [off[i], off[i]+len[i]) go to out[coff[i] ...]
+// (its first residue's w marks coordinates that are not ordinary)
 void launch_pack4_structs(float4* out, const float* x, const float* y, const float* z,
                           const int* off, const int* len, const int* coff, int n,
                           cudaStream_t st);

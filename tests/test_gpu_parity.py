@@ -356,3 +356,19 @@ def test_refinement_length_classes(oracle, lens, fill):
     res, ora = run_both(oracle, q, r, d)
     assert_same(res, ora, q.n, r.n)
     assert (res.alndata[0, :len(lens), 4] >= np.array(lens) - 2).all()
+
+
+@pytest.mark.parametrize("opt", ["filters", "ssrr", "frg3"])
+def test_dp_strip_edges(oracle, opt):
+    """Queries that end at and beside the DP's strips and its change of rows
+    per lane, references that end at and beside 32 columns (the column ring,
+    the row buffer, the traceback's windows): GPU against the oracle bit for
+    bit, at the options that use every cell score."""
+    from gtalign_alpha_b200 import synth
+    rng = np.random.default_rng(77)
+    q = synth.random_chains(rng, [21, 63, 64, 65, 127, 129, 383, 384, 385, 513], "q")
+    r = synth.random_chains(rng, [20, 31, 32, 33, 63, 64, 65, 95, 97, 128], "r")
+    r += [synth.homolog(rng, c, 1.0, 0.05, "h") for c in q]
+    q, r = synth.pack(q), synth.pack(r)
+    res, ora = run_both(oracle, q, r, OPTSETS[opt])
+    assert_same(res, ora, q.n, r.n)
