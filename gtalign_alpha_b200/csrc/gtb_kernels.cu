@@ -23,7 +23,7 @@
 //    shuffles, each lane packs the 2-bit directions of its cells into
 //    traceback words.  A long pair's strips run as a wavefront over several
 //    single-warp CTAs (cooperative launch, bounded waits on progress counters).
-//  * traceback, alignment rows, bookkeeping: one thread per pair.
+//  * traceback: a warp per pair; alignment rows, bookkeeping: a thread per pair.
 // All floating-point reductions are sequential per thread in forward position
 // order (blocks of BLK positions, Neumaier-compensated), so results do not
 // depend on the launch geometry.
@@ -2736,19 +2736,95 @@ void launch_f3_dpscore(const Blk& B, const Bat& T, cudaStream_t st) {
 
 // ---------------------------------------------------------------------------
 // traceback: MpDPHub.cpp:1515-1660 (plain) and 1699-1905 (constrained)
-constexpr int BTCK_AHEAD = 4;     // step groups the traceback loads ahead
+//
+// A warp per pair.  The walk is one chain of dependent steps, the same on every
+// lane; a thread per pair paid a load from L2 for most of them (580 cycles a
+// step: 0.73 ms for a pair of 1,200 residues).  Here the 32 words of a (strip,
+// step group), one 128-byte line, come in for BT_WIN groups at a time into
+// shared memory, and the lines the path enters next (the groups below, and the
+// previous strip's around the path's column) are on their way to L1.  32
+// aligned pairs at a time are written out, a pair per lane.
+constexpr int BT_WIN = 16;        // groups of a window
+constexpr int BT_WARPS = 4;
 __device__ __forceinline__ void bt_prefetch(const unsigned* p) {
     asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
 }
 
-__global__ void k_btck(Blk B, Bat T, int constrained) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+template <int R>
+__device__ __forceinline__ int btck_walk(const unsigned* bt, int lq, int lr, const float4* q4,
+                                         const float4* r4, bool constrained, const float* t,
+                                         float d82, unsigned* aln, float* alc, unsigned* win,
+                                         int lane) {
+    const unsigned FULL = 0xffffffffu;
+    constexpr int ROWS = 32 * R, SPW = 16 / R;
+    const long long sw = bt_strip_words(lr, R);
+    int y = lq - 1, x = lr - 1, n = 0, pend = 0;
+    unsigned mine = 0;                        // this lane's aligned pair among the last 32
+    auto flush = [&](int cnt) {
+        float4 cq = make_float4(0.f, 0.f, 0.f, 0.f), cr = cq;
+        bool keep = lane < cnt;
+        if (keep) {
+            cq = __ldg(q4 + (mine >> 16));
+            cr = __ldg(r4 + (mine & 0xffffu));
+            if (constrained) keep = dist2_tf(t, cq.x, cq.y, cq.z, cr.x, cr.y, cr.z) <= d82;
+        }
+        const unsigned m = __ballot_sync(FULL, keep);
+        if (keep) {
+            const int k = n + __popc(m & ((1u << lane) - 1u));
+            aln[k] = mine;
+            float2* c2 = (float2*)(alc + 6 * (long long)k);
+            c2[0] = make_float2(cq.x, cq.y); c2[1] = make_float2(cq.z, cr.x); c2[2] = make_float2(cr.y, cr.z);
+        }
+        n += __popc(m);
+    };
+    int cs = -1, wlo = 0, cg = -1, cl = -1;   // the window's strip and lowest group; the word in w
+    unsigned w = 0;
+    while (x >= 0 && y >= 0) {
+        const int s = y / ROWS, yy = y % ROWS, l = yy / R, tt = x + l, g = tt / SPW;
+        if (s != cs || g < wlo) {
+            cs = s;
+            wlo = g - BT_WIN + 1 > 0 ? g - BT_WIN + 1 : 0;
+            const unsigned* line = bt + s * sw;
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < BT_WIN; k++)
+                if (g - k >= 0) win[((g - k) & (BT_WIN - 1)) * 32 + lane] = line[(g - k) * 32 + lane];
+            if (lane < BT_WIN) {
+                if (wlo - 1 - lane >= 0) bt_prefetch(line + (wlo - 1 - lane) * 32);
+            } else if (s > 0) {
+                const int gp = (x + 31) / SPW - (lane - BT_WIN);
+                if (gp >= 0) bt_prefetch(line - sw + gp * 32);
+            }
+            __syncwarp();
+            cg = -1;
+        }
+        if (g != cg || l != cl) {
+            w = win[(g & (BT_WIN - 1)) * 32 + l];
+            cg = g; cl = l;
+        }
+        const unsigned b = (w >> (2 * R * (tt % SPW) + 2 * (yy % R))) & 3u;
+        if (b == BTW_DIAG) {
+            if (lane == pend) mine = ((unsigned)y << 16) | (unsigned)x;
+            if (++pend == 32) { flush(32); pend = 0; }
+        }
+        // down is 2 or 3, left 1, diagonal 0
+        y -= b != BTW_LEFT;
+        x -= b < BTW_UP;
+    }
+    if (pend > 0) flush(pend);
+    return n;
+}
+
+__global__ void __launch_bounds__(BT_WARPS * 32) k_btck(Blk B, Bat T, int constrained) {
+    __shared__ unsigned s_win[BT_WARPS][BT_WIN * 32];
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const int i = blockIdx.x * BT_WARPS + wp;
     if (i >= T.np) return;
     int flags = T.flags[i];
     if (constrained) {
         if (flags & CONV_LOWTMSC) return;
     } else if ((flags & (CONV_LOWTMSC | CONV_SCOREDP)) || alt_empty(T, i)) {
-        T.naln[i] = 0;
+        if (lane == 0) T.naln[i] = 0;
         return;
     }
     int qi = pair_qi(B, T, i), ri = pair_ri(B, T, i);
@@ -2757,66 +2833,20 @@ __global__ void k_btck(Blk B, Bat T, int constrained) {
     const unsigned* bt = T.bt + T.off_bt[i];
     unsigned* aln = T.aln + T.off_aln[i];
     float* alc = T.alc + 6 * T.off_aln[i];
-    const int R = dp_r(lq), rows = 32 * R, spw = 16 / R;
-    const long long sw = bt_strip_words(lr, R);
     float t[12];
     float d82 = B.t_d82[ml];
     const float4* q4 = B.q4 + B.q4off[qi];
     const float4* r4 = B.r4 + B.r4off[ri];
-    if (constrained) {
 #pragma unroll
-        for (int f = 0; f < 12; f++) t[f] = T.tfm_gr[i * 12 + f];
-    }
-    int y = lq - 1, x = lr - 1, n = 0;
-    // The walk is a chain of dependent loads.  The 32 words of a (strip, step
-    // group) are one 128-byte line and the path only moves to lower groups and
-    // strips, so each new group starts the loads of the BTCK_AHEAD groups
-    // below it (and, near a strip's top, of the previous strip's groups the
-    // path enters next); the last word read is kept.
-    long long cwi = -1;
-    unsigned w = 0;
-    int cs = -1, cg = -1, prevs = -1;
-    while (x >= 0 && y >= 0) {
-        int yy = y % rows, l = yy / R, tt = x + l;
-        const int s = y / rows, g = tt / spw;
-        const long long wi = (long long)s * sw + (long long)g * 32 + l;
-        if (wi != cwi) {
-            if (s != cs) {              // a new strip (or the start): its next groups
-                for (int k = 1; k <= BTCK_AHEAD && g - k >= 0; k++)
-                    bt_prefetch(bt + (long long)s * sw + (long long)(g - k) * 32);
-            } else if (g != cg && g >= BTCK_AHEAD) {
-                bt_prefetch(bt + (long long)s * sw + (long long)(g - BTCK_AHEAD) * 32);
-            }
-            cs = s; cg = g;
-            if (l <= 2 && s > 0 && prevs != s) {
-                const int gp = (x + 31) / spw;
-                for (int k = 0; k < BTCK_AHEAD && gp - k >= 0; k++)
-                    bt_prefetch(bt + (long long)(s - 1) * sw + (long long)(gp - k) * 32);
-                prevs = s;
-            }
-            w = bt[wi];
-            cwi = wi;
-        }
-        const unsigned b = (w >> (2 * R * (tt % spw) + 2 * (yy % R))) & 3u;
-        if (b >= BTW_UP) { y--; continue; }
-        if (b == BTW_LEFT) { x--; continue; }
-        float4 cq = __ldg(q4 + y), cr = __ldg(r4 + x);
-        float cqx = cq.x, cqy = cq.y, cqz = cq.z, crx = cr.x, cry = cr.y, crz = cr.z;
-        bool keep = true;
-        if (constrained) keep = dist2_tf(t, cqx, cqy, cqz, crx, cry, crz) <= d82;
-        if (keep) {
-            aln[n] = ((unsigned)y << 16) | (unsigned)x;
-            float2* c2 = (float2*)(alc + 6 * (long long)n);
-            c2[0] = make_float2(cqx, cqy); c2[1] = make_float2(cqz, crx); c2[2] = make_float2(cry, crz);
-            n++;
-        }
-        x--; y--;
-    }
-    T.naln[i] = n;
+    for (int f = 0; f < 12; f++) t[f] = constrained ? T.tfm_gr[i * 12 + f] : 0.f;
+    const int n = dp_r(lq) == 4
+        ? btck_walk<4>(bt, lq, lr, q4, r4, constrained != 0, t, d82, aln, alc, s_win[wp], lane)
+        : btck_walk<2>(bt, lq, lr, q4, r4, constrained != 0, t, d82, aln, alc, s_win[wp], lane);
+    if (lane == 0) T.naln[i] = n;
 }
 
 void launch_btck(const Blk& B, const Bat& T, int constrained, cudaStream_t st) {
-    k_btck<<<(T.np + 127) / 128, 128, 0, st>>>(B, T, constrained);
+    k_btck<<<(T.np + BT_WARPS - 1) / BT_WARPS, BT_WARPS * 32, 0, st>>>(B, T, constrained);
     GTB_LAUNCHED(T);
 }
 
