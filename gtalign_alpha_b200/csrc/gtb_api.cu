@@ -341,6 +341,37 @@ static gtb_status run_block(gtb_handle* h, const DevBlock& D, float scorethld,
     struct StrBat { char* base; long long p0; int np; long long* soff; unsigned long long* cnt; char* str; };
     std::vector<StrBat> strbat;
 
+    // A copy to pageable host memory holds the host until it is done, and with
+    // it the launches of the next sub-batch: such results are copied once all
+    // sub-batches are launched (400 structures all against all 198 -> 113 ms).
+    auto pageable = [](const void* p) {
+        cudaPointerAttributes a{};
+        if (!p) return false;
+        if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return true; }
+        return a.type == cudaMemoryTypeUnregistered;
+    };
+    const bool late = pageable(h_alndata) || pageable(h_tfm) || pageable(h_err);
+    struct LateBat { char* base; long long p0; int np; const float *out, *tfm, *err; cudaStream_t st; };
+    std::vector<LateBat> latebat;
+    auto copy_out = [&](long long q0, int np, const float* out, const float* tfm, const float* err,
+                        cudaStream_t st) -> gtb_status {
+        if (h_alndata)
+            CK(cudaMemcpyAsync(h_alndata + q0 * 16, out, (size_t)np * 16 * sizeof(float), cudaMemcpyDefault, st));
+        if (h_tfm)
+            CK(cudaMemcpyAsync(h_tfm + q0 * 12, tfm, (size_t)np * 12 * sizeof(float), cudaMemcpyDefault, st));
+        if (h_err)
+            CK(cudaMemcpyAsync(h_err + q0 * 4, err, (size_t)np * 4 * sizeof(float), cudaMemcpyDefault, st));
+        return GTB_OK;
+    };
+    // frees the memory of sub-batches kept past their launches
+    auto drop_kept = [&](bool sync) {
+        if (sync) for (int k = 0; k < gtb_handle::NSUB; k++) cudaStreamSynchronize(h->sub[k]);
+        if (strings) for (const StrBat& sb : strbat) cudaFreeAsync(sb.base, h->st);
+        else for (const LateBat& lb : latebat) cudaFreeAsync(lb.base, lb.st);
+        strbat.clear();
+        latebat.clear();
+    };
+
     // One sub-batch [q0, q0 + np): plan, carve one allocation, upload the
     // offsets, launch the stage sequence and the result copies on stream st.
     auto launch_sub = [&](long long q0, int np, int j, int evset) -> gtb_status {
@@ -546,18 +577,17 @@ static gtb_status run_block(gtb_handle* h, const DevBlock& D, float scorethld,
                       scorethld, st, h->sev[evset], o.polish_steps);
         CK(lerr);
         CK(cudaGetLastError());
-        if (h_alndata)
-            CK(cudaMemcpyAsync(h_alndata + q0 * 16, T.out, (size_t)np * 16 * sizeof(float), cudaMemcpyDefault, st));
-        if (h_tfm)
-            CK(cudaMemcpyAsync(h_tfm + q0 * 12, T.tfm_gr, (size_t)np * 12 * sizeof(float), cudaMemcpyDefault, st));
-        if (h_err)
-            CK(cudaMemcpyAsync(h_err + q0 * 4, T.err, (size_t)np * 4 * sizeof(float), cudaMemcpyDefault, st));
+        if (!late) {
+            gtb_status s2 = copy_out(q0, np, T.out, T.tfm_gr, T.err, st);
+            if (s2 != GTB_OK) return s2;
+        }
         CK(cudaMemcpyAsync(h->h_flag + evset, T.dw_err, sizeof(int), cudaMemcpyDeviceToHost, st));
         if (strings) {
             // read after the batch: only the bytes the rows took
             strbat.push_back({base, q0, np, T.str_off, T.str_cnt, T.str});
-            return GTB_OK;
         }
+        if (late) latebat.push_back({base, q0, np, T.out, T.tfm_gr, T.err, st});
+        if (strings || late) return GTB_OK;
         CK(cudaFreeAsync(base, st));
         return GTB_OK;
     };
@@ -605,13 +635,21 @@ static gtb_status run_block(gtb_handle* h, const DevBlock& D, float scorethld,
             long long q1 = p0 + nb * (j + 1) / nsub;
             gtb_status s = launch_sub(q0, (int)(q1 - q0), j % gtb_handle::NSUB, j);
             if (s != GTB_OK) {
-                for (int k = 0; k < gtb_handle::NSUB; k++) cudaStreamSynchronize(h->sub[k]);
-                for (const StrBat& sb : strbat) cudaFreeAsync(sb.base, h->st);
+                drop_kept(true);
                 return s;
             }
             q0 = q1;
         }
+        for (const LateBat& lb : latebat) {
+            gtb_status s = copy_out(lb.p0, lb.np, lb.out, lb.tfm, lb.err, lb.st);
+            if (s != GTB_OK) {
+                drop_kept(true);
+                return s;
+            }
+        }
         for (int j = 0; j < std::min(nsub, gtb_handle::NSUB); j++) CK(cudaStreamSynchronize(h->sub[j]));
+        if (!strings) drop_kept(false);
+        latebat.clear();
         if (!strbat.empty()) {
             gtb_status s2 = GTB_OK;
             for (const StrBat& sb : strbat) {
