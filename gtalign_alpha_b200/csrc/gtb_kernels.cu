@@ -591,6 +591,157 @@ __device__ float findfrag_variant(const PairGeom& G, float d02, float d0s, int s
     return best;
 }
 
+// The same for ordinary coordinates (coords_ordinary), without branches in the
+// sweeps.  findfrag_variant's fused pass kept the six smallest distances with
+// their positions and added to the covariance as it went: with 32 offsets a
+// warp, some lane took nearly every branch (about 60 issued instructions a
+// visit).  Here a pass scores and keeps the three smallest distances by five
+// minima and maxima; the threshold then known, a second sweep marks the
+// positions within it in a 32-bit mask per block and only the marked ones are
+// added.  What bounds it: issue, and the L1 reads of 32 offsets' residues.
+struct SeedCov {                       // covariance sums, CovAcc's order of operations
+    float s[15], c[15], b[15];
+    int n;
+    __device__ __forceinline__ void init() {
+#pragma unroll
+        for (int f = 0; f < 15; f++) { s[f] = 0.f; c[f] = 0.f; b[f] = 0.f; }
+        n = 0;
+    }
+    __device__ __forceinline__ void add(const float4& u, const float4& v) {
+        b[0] = __fmaf_rn(u.x, v.x, b[0]); b[1] = __fmaf_rn(u.x, v.y, b[1]); b[2] = __fmaf_rn(u.x, v.z, b[2]);
+        b[3] = __fmaf_rn(u.y, v.x, b[3]); b[4] = __fmaf_rn(u.y, v.y, b[4]); b[5] = __fmaf_rn(u.y, v.z, b[5]);
+        b[6] = __fmaf_rn(u.z, v.x, b[6]); b[7] = __fmaf_rn(u.z, v.y, b[7]); b[8] = __fmaf_rn(u.z, v.z, b[8]);
+        b[9] = __fadd_rn(b[9], u.x); b[10] = __fadd_rn(b[10], u.y); b[11] = __fadd_rn(b[11], u.z);
+        b[12] = __fadd_rn(b[12], v.x); b[13] = __fadd_rn(b[13], v.y); b[14] = __fadd_rn(b[14], v.z);
+    }
+    __device__ __forceinline__ void fold() {
+#pragma unroll
+        for (int f = 0; f < 15; f++) { tfold(s[f], c[f], b[f]); b[f] = 0.f; }
+    }
+    __device__ __forceinline__ void final(float* v) const {
+#pragma unroll
+        for (int f = 0; f < 15; f++) v[f] = __fadd_rn(s[f], c[f]);
+        v[15] = (float)n;
+    }
+};
+
+__device__ __forceinline__ float seed_d2(const float* tfm, const float4& u, const float4& v) {
+    return dist2_tf(tfm, u.x, u.y, u.z, v.x, v.y, v.z);
+}
+
+// score under tfm and, M3, the three smallest distances (a multiset)
+template <bool M3>
+__device__ __forceinline__ float seed_score(const float4* q, const float4* r, int n, const float* tfm,
+                                            float d02, float& m1, float& m2, float& m3) {
+    float ss = 0.f, sc = 0.f;
+    m1 = m2 = m3 = LARGEDST;
+    auto visit = [&](int k, float& sb) {
+        const float d = seed_d2(tfm, __ldg(q + k), __ldg(r + k));
+        sb = __fadd_rn(sb, div_ord(d02, __fadd_rn(d02, d)));
+        if (M3) {
+            const float a = fmaxf(m1, d);
+            m1 = fminf(m1, d);
+            m3 = fminf(m3, fmaxf(m2, a));
+            m2 = fminf(m2, a);
+        }
+    };
+    int b0 = 0;
+    for (; b0 + BLK <= n; b0 += BLK) {
+        float sb = 0.f;
+#pragma unroll 8
+        for (int k = 0; k < BLK; k++) visit(b0 + k, sb);
+        tfold(ss, sc, sb);
+    }
+    float sb = 0.f;
+#pragma unroll 2
+    for (int k = b0; k < n; k++) visit(k, sb);
+    tfold(ss, sc, sb);
+    return __fadd_rn(ss, sc);
+}
+
+// covariance of the positions with d <= thr
+__device__ __forceinline__ void seed_cov(const float4* q, const float4* r, int n, const float* tfm,
+                                         float thr, float* v) {
+    SeedCov A;
+    A.init();
+    for (int b0 = 0; b0 < n; b0 += BLK) {
+        unsigned mask = 0u;
+        if (b0 + BLK <= n) {
+#pragma unroll 1
+            for (int k = 0; k < BLK; k += 8) {
+                unsigned m8 = 0u;
+#pragma unroll
+                for (int e = 0; e < 8; e++)
+                    if (seed_d2(tfm, __ldg(q + b0 + k + e), __ldg(r + b0 + k + e)) <= thr) m8 |= 1u << e;
+                mask |= m8 << k;
+            }
+        } else {
+#pragma unroll 2
+            for (int k = b0; k < n; k++)
+                if (seed_d2(tfm, __ldg(q + k), __ldg(r + k)) <= thr) mask |= 1u << (k - b0);
+        }
+        if (mask) {
+            A.n += __popc(mask);
+            do {
+                const int k = b0 + __ffs(mask) - 1;
+                mask &= mask - 1;
+                A.add(__ldg(q + k), __ldg(r + k));
+            } while (mask);
+            A.fold();
+        }
+    }
+    A.final(v);
+}
+
+// the third smallest distinct distance (ties among the smallest: rare)
+__device__ __noinline__ float seed_third_distinct(const float4* q, const float4* r, int n, const float* tfm) {
+    float m1 = LARGEDST, m2 = LARGEDST, m3 = LARGEDST;
+    for (int k = 0; k < n; k++) track3(1, seed_d2(tfm, __ldg(q + k), __ldg(r + k)), m1, m2, m3);
+    return m3;
+}
+
+__device__ __forceinline__ float findfrag_variant_fast(const float4* q, const float4* r, int n, float d02,
+                                                       float d0s, int swap, unsigned long long& vis) {
+    float v[16], tfm[12], best = 0.f;
+    const float d02s0 = __fmul_rn(d0s, d0s);
+    {
+        SeedCov A;
+        A.init();
+        for (int b0 = 0; b0 < n; b0 += BLK) {
+            const int b1 = b0 + BLK < n ? b0 + BLK : n;
+#pragma unroll 4
+            for (int k = b0; k < b1; k++) A.add(__ldg(q + k), __ldg(r + k));
+            A.fold();
+        }
+        A.n = n;
+        A.final(v);
+    }
+    vis += n;
+#pragma unroll 1
+    for (int it = 0; it < 3; it++) {
+        solve_sums(v, swap, tfm);
+        float m1, m2, m3;
+        vis += n;
+        if (it == 2) {
+            const float sc = seed_score<false>(q, r, n, tfm, d02, m1, m2, m3);
+            if (best < sc) best = sc;
+            break;
+        }
+        const float d02s = __fadd_rn(d02s0, (it == 1 ? 1.0f : 0.0f));
+        const float sc = seed_score<true>(q, r, n, tfm, d02, m1, m2, m3);
+        if (best < sc) best = sc;
+        if ((m1 == m2 || m2 == m3) && m1 < LARGEDST) m3 = seed_third_distinct(q, r, n, tfm);
+        float dst32;
+        if (LARGEDST_CMP < m3 || m3 < d02s || n <= 3) dst32 = d02s;
+        else dst32 = __fadd_rn(d02s, __fmul_rn(ceilf(__fmul_rn(__fsub_rn(m3, d02s), 2.0f)), 0.5f));
+        seed_cov(q, r, n, tfm, dst32, v);
+        vis += n;
+        if (v[15] < 1.0f) break;
+        if ((int)v[15] == n) break;
+    }
+    return best;
+}
+
 __global__ void __launch_bounds__(128) k_findfrag(Blk B, Bat T) {
     const int item = blockIdx.x;
     int i = item, c = 0, nch = 1;
@@ -623,6 +774,7 @@ __global__ void __launch_bounds__(128) k_findfrag(Blk B, Bat T) {
     PairGeom G;
     G.q4 = B.q4 + B.q4off[qi]; G.r4 = B.r4 + B.r4off[ri];
     G.alc = nullptr;
+    const bool fast = coords_ordinary(G.q4) && coords_ordinary(G.r4);
     float lbest = 0.f;
     int lsi = 0x7fffffff;
     unsigned long long vis = 0;
@@ -639,7 +791,8 @@ __global__ void __launch_bounds__(128) k_findfrag(Blk B, Bat T) {
         if (lq - qpos < prv || lr - rpos < prv) continue;
         G.q0 = qpos; G.r0 = rpos;
         G.n = (lq - qpos) < (lr - rpos) ? (lq - qpos) : (lr - rpos);
-        float b = findfrag_variant(G, d02, d0s, swap, vis);
+        const float b = fast ? findfrag_variant_fast(G.q4 + qpos, G.r4 + rpos, G.n, d02, d0s, swap, vis)
+                             : findfrag_variant(G, d02, d0s, swap, vis);
         if (b > 0.f && lbest < b) { lbest = b; lsi = si; }
     }
     __shared__ float sb[128];
@@ -1565,15 +1718,6 @@ struct alignas(16) CoopSmem {
 };
 inline size_t coop_smem_bytes(int nmax) {
     return sizeof(CoopSmem) + (size_t)((nmax + BLK - 1) / BLK * BLK) * (sizeof(float4) + sizeof(float2));
-}
-
-// the exact error of s + b added to the compensation (Knuth's TwoSum): the
-// same c as nfold's, whose comparison only orders the operands
-__device__ __forceinline__ void tfold(float& s, float& c, float b) {
-    const float t = __fadd_rn(s, b);
-    const float bb = __fsub_rn(t, s);
-    c = __fadd_rn(c, __fadd_rn(__fsub_rn(s, __fsub_rn(t, bb)), __fsub_rn(b, bb)));
-    s = t;
 }
 
 __device__ __forceinline__ void keep3(float d, float& m1, float& m2, float& m3) {
