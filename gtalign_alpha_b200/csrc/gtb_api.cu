@@ -475,7 +475,7 @@ static gtb_status run_block(gtb_handle* h, const DevBlock& D, float scorethld,
         size_t o_sto = strings ? carve((size_t)np * sizeof(long long) + sizeof(unsigned long long)) : 0;
         size_t o_alc = carve((size_t)off_aln[np] * 6 * sizeof(float));
         size_t o_rl = carve((size_t)np * sizeof(int));
-        size_t o_rh = carve((size_t)4097 * sizeof(int));
+        size_t o_rh = carve((size_t)gtb::RL_NHIST * sizeof(int));
         size_t o_ffi = split ? carve((size_t)nitems * 2 * sizeof(int)) : 0;
         size_t o_ffn = split ? carve((size_t)np * sizeof(int)) : 0;
         size_t o_ffk = split ? carve((size_t)np * sizeof(unsigned long long)) : 0;

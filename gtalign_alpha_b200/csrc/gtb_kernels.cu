@@ -1696,7 +1696,8 @@ __global__ void k_refine_long_fin(Blk B, Bat T) {
 // of the pass -> solve chain (about 800 + 2,800 cycles at 150 positions).
 // Refinement launches of a call, before -> after: one pair of 150 residues
 // 3.5 -> 1.0 ms, 16 x 500 29 -> 16 ms, all against all of 400 structures
-// 114 -> 78 ms, 2 x 20,000 115 -> 62 ms (three streams).
+// 114 -> 78 ms, 2 x 20,000 115 -> 62 ms (three streams).  Four CTAs a SM (128
+// registers) against three: 2 x 8,000 41.8 -> 36.9 ms, 1 x 1,000 4.0 -> 3.5.
 constexpr int CM_WARPS = 4;
 constexpr int CM_MAX = 8;                    // variants a warp holds at most
 constexpr int CM_CMAX = 8;                   // CTAs per cluster at most
@@ -1714,7 +1715,7 @@ struct alignas(16) CoopSmem {
     CoopWarp w[CM_WARPS];
     float win[CM_CMAX * 32];                 // the CTAs' winners (first CTA)
     float cand[CM_WARPS * 32];               // the warps' winners
-    int next;
+    int next, slot;
 };
 inline size_t coop_smem_bytes(int nmax) {
     return sizeof(CoopSmem) + (size_t)((nmax + BLK - 1) / BLK * BLK) * (sizeof(float4) + sizeof(float2));
@@ -1850,7 +1851,7 @@ __device__ float coop_rmsd(CoopWarp& w, int n, const float4* cA, const float2* c
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(CM_WARPS * 32) k_refine_coop(Blk B, Bat T, int lo, int hi) {
+__global__ void __launch_bounds__(CM_WARPS * 32, 4) k_refine_coop(Blk B, Bat T, int lo, int hi, int cls) {
     extern __shared__ __align__(16) unsigned char cm_smem[];
     CoopSmem& S = *(CoopSmem*)cm_smem;
     float4* cA = (float4*)(cm_smem + sizeof(CoopSmem));
@@ -1862,7 +1863,10 @@ __global__ void __launch_bounds__(CM_WARPS * 32) k_refine_coop(Blk B, Bat T, int
     int first, last;
     rlist_range(T, lo, hi, first, last);
     for (int e = 0; e < CM_CHUNK; e++) w.buf[e * CM_BLKW + 7 * CM_BST + lane] = 1.f;
-    for (int slot = first + (int)blockIdx.x / C; slot < last; slot += (int)gridDim.x / C) {
+    // the first pair by position, the next ones as clusters come free
+    int* ctr = T.rhist + RL_NB + 1 + cls;
+    const int ncl = (int)gridDim.x / C;
+    for (int slot = first + (int)blockIdx.x / C; slot < last;) {
         const int i = T.rlist[slot];
         const int qi = pair_qi(B, T, i), ri = pair_ri(B, T, i);
         const int lq = B.qlen[qi], lr = B.rlen[ri];
@@ -1878,7 +1882,6 @@ __global__ void __launch_bounds__(CM_WARPS * 32) k_refine_coop(Blk B, Bat T, int
             n = T.naln[i];
         }
         float2* cB = (float2*)(cA + (n + BLK - 1) / BLK * BLK);
-        __syncthreads();                                      // the last pair's shared data is done with
         if (MODE == RM_INIT) {
             for (int p = threadIdx.x; p < n; p += blockDim.x) {
                 const float4 u = __ldg(q4 + sq + p), v = __ldg(r4 + sr + p);
@@ -2099,9 +2102,14 @@ __global__ void __launch_bounds__(CM_WARPS * 32) k_refine_coop(Blk B, Bat T, int
                 refine_commit<MODE>(B, T, i, lq, lr, x[0] > 0.f, x[0], x[2], __float_as_int(x[3]),
                                     __float_as_int(x[4]), x + 5, 1);
             }
-            cl.sync();                 // the winners are read before the next pair's arrive
         }
+        if (crank == 0 && threadIdx.x == 0) S.slot = first + ncl + atomicAdd(ctr, 1);
+        // the next pair is known; this one's shared data is done with
+        if (C > 1) cl.sync();
+        else __syncthreads();
+        slot = *cl.map_shared_rank(&S.slot, 0);
     }
+    if (C > 1) cl.sync();              // the first CTA's shared memory is read until here
 }
 
 // npair: pairs the launch may have at most (a lane form's grid)
@@ -2128,7 +2136,7 @@ static void launch_refine_k(int mode, const Blk& B, const Bat& T, cudaStream_t s
 // A warp to a pass: the listed pairs with lo <= n < hi (at most npair of
 // them), a cluster of C CTAs a pair.
 static void launch_refine_coop(int mode, const Blk& B, const Bat& T, cudaStream_t st, int npair,
-                               int lo, int hi, int C) {
+                               int lo, int hi, int C, int cls) {
     const int nmax = std::min(hi - 1, std::min(B.qmax, B.rmax));
     if (npair <= 0 || nmax < lo) return;
     cudaLaunchConfig_t cfg{};
@@ -2144,13 +2152,13 @@ static void launch_refine_coop(int mode, const Blk& B, const Bat& T, cudaStream_
     cfg.numAttrs = C > 1 ? 1 : 0;
     cudaError_t e = cudaErrorInvalidValue;
     switch (mode) {
-        case RM_INIT:  e = cudaLaunchKernelEx(&cfg, k_refine_coop<RM_INIT>, B, T, lo, hi); break;
-        case RM_DP:    e = cudaLaunchKernelEx(&cfg, k_refine_coop<RM_DP>, B, T, lo, hi); break;
-        case RM_FIN1:  e = cudaLaunchKernelEx(&cfg, k_refine_coop<RM_FIN1>, B, T, lo, hi); break;
-        case RM_FIN2:  e = cudaLaunchKernelEx(&cfg, k_refine_coop<RM_FIN2>, B, T, lo, hi); break;
-        case RM_PROD1: e = cudaLaunchKernelEx(&cfg, k_refine_coop<RM_PROD1>, B, T, lo, hi); break;
-        case RM_PROD2: e = cudaLaunchKernelEx(&cfg, k_refine_coop<RM_PROD2>, B, T, lo, hi); break;
-        case RM_PLOG:  e = cudaLaunchKernelEx(&cfg, k_refine_coop<RM_PLOG>, B, T, lo, hi); break;
+        case RM_INIT:  e = cudaLaunchKernelEx(&cfg, k_refine_coop<RM_INIT>, B, T, lo, hi, cls); break;
+        case RM_DP:    e = cudaLaunchKernelEx(&cfg, k_refine_coop<RM_DP>, B, T, lo, hi, cls); break;
+        case RM_FIN1:  e = cudaLaunchKernelEx(&cfg, k_refine_coop<RM_FIN1>, B, T, lo, hi, cls); break;
+        case RM_FIN2:  e = cudaLaunchKernelEx(&cfg, k_refine_coop<RM_FIN2>, B, T, lo, hi, cls); break;
+        case RM_PROD1: e = cudaLaunchKernelEx(&cfg, k_refine_coop<RM_PROD1>, B, T, lo, hi, cls); break;
+        case RM_PROD2: e = cudaLaunchKernelEx(&cfg, k_refine_coop<RM_PROD2>, B, T, lo, hi, cls); break;
+        case RM_PLOG:  e = cudaLaunchKernelEx(&cfg, k_refine_coop<RM_PLOG>, B, T, lo, hi, cls); break;
     }
     if (e != cudaSuccess && T.lerr && *T.lerr == cudaSuccess) *T.lerr = e;
     GTB_LAUNCHED(T);
@@ -2219,7 +2227,7 @@ void launch_refine(int mode, const Blk& B, const Bat& T0, cudaStream_t st, bool 
     Bat T = T0;
     T.rl_min = RL_LONG;
     T.rlw_ctas = T0.rlw_ctas > 0 && T0.rlw_ctas <= RLW_CTAS_MAX ? T0.rlw_ctas : RLW_CTAS;
-    cudaMemsetAsync(T.rhist, 0, (RL_NB + 1) * sizeof(int), st);
+    cudaMemsetAsync(T.rhist, 0, RL_NHIST * sizeof(int), st);
     if (T.rl_long) {
         cudaMemsetAsync(T.rl_count, 0, sizeof(int), st);
         cudaMemsetAsync(T.rl_next, 0, (size_t)T.rl_nlmax * sizeof(int), st);
@@ -2248,11 +2256,11 @@ void launch_refine(int mode, const Blk& B, const Bat& T0, cudaStream_t st, bool 
         GTB_LAUNCHED(T);
     }
     const bool coop = few || T.np <= RC_SMALL;
-    launch_refine_coop(mode, B, T, sl, T.nml[2], RC_N2, RL_LONG, 8);
+    launch_refine_coop(mode, B, T, sl, T.nml[2], RC_N2, RL_LONG, 8, 2);
     if (coop) {
         const int c = T.np <= RC_NP8 ? 8 : T.np <= RC_NP4 ? 4 : T.np <= RC_NP2 ? 2 : 1;
-        launch_refine_coop(mode, B, T, st, T.nml[1], RC_N1, RC_N2, c < 4 ? 4 : c);
-        launch_refine_coop(mode, B, T, st, T.np, 0, RC_N1, c);
+        launch_refine_coop(mode, B, T, st, T.nml[1], RC_N1, RC_N2, c < 4 ? 4 : c, 1);
+        launch_refine_coop(mode, B, T, st, T.np, 0, RC_N1, c, 0);
     } else {
         launch_refine_k<16, false>(mode, B, T, st, T.np, 0, RC_N2);
         GTB_LAUNCHED(T);
@@ -2771,7 +2779,7 @@ static void launch_dp_wave(const Blk& B, const Bat& T, int tfmsrc, float gcost, 
 void launch_dp(const Blk& B, const Bat& T, int tfmsrc, int gap0, float gcost, int usess,
                int dpscan, int skipmode, cudaStream_t st) {
     {
-        cudaMemsetAsync(T.rhist, 0, (RL_NB + 1) * sizeof(int), st);
+        cudaMemsetAsync(T.rhist, 0, RL_NHIST * sizeof(int), st);
         const int nb = (T.np + 255) / 256;
         k_dlist_count<<<nb, 256, 0, st>>>(B, T, skipmode);
         k_rlist_scan<<<1, 1024, 0, st>>>(T);
@@ -2799,7 +2807,7 @@ void launch_dp(const Blk& B, const Bat& T, int tfmsrc, int gap0, float gcost, in
 }
 
 void launch_pair_list(const Blk& B, const Bat& T, int skipmask, cudaStream_t st) {
-    cudaMemsetAsync(T.rhist, 0, (RL_NB + 1) * sizeof(int), st);
+    cudaMemsetAsync(T.rhist, 0, RL_NHIST * sizeof(int), st);
     const int nb = (T.np + 255) / 256;
     k_plist_count<<<nb, 256, 0, st>>>(B, T, skipmask);
     k_rlist_scan<<<1, 1024, 0, st>>>(T);

@@ -29,8 +29,9 @@ constexpr int RL_LONG = 1536;
 // 16 x 500 takes twice as long; 4 for 1,000 pairs 13.9 against 11.4 ms).
 constexpr int RC_N1 = 256, RC_N2 = 512;
 constexpr int RC_SMALL = 2048, RC_NP8 = 64, RC_NP4 = 256, RC_NP2 = 4096;
-constexpr int RC_GRID = 1184;         // CTAs of a launch at most
+constexpr int RC_GRID = 592;          // CTAs of a launch at most (4 per SM)
 constexpr int RL_NBUCKET = 65536 >> 4;   // work-list buckets; rhist[RL_NBUCKET] = list length
+constexpr int RL_NHIST = RL_NBUCKET + 5; // and after it the launches' counters of pairs taken
 constexpr int RLW_CTAS = 16;
 constexpr int RLW_GRID = 1024;
 constexpr int RLW_CTAS_MAX = 256;
@@ -127,7 +128,7 @@ struct Bat {
     // last byte of a row its NUL; str_cnt: bytes used
     long long* str_off;
     unsigned long long* str_cnt;
-    int *rlist, *rhist;              // refinement work list [np], buckets [4097]
+    int *rlist, *rhist;              // refinement work list [np], buckets [RL_NHIST]
     // long pairs of a refinement launch (null: none possible): list, count,
     // per-pair variant counter, per-warp candidates; rl_nlmax = capacity;
     // this launch's threshold and CTAs per long pair.  The caller's rlw_ctas

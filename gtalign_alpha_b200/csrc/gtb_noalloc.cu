@@ -203,7 +203,7 @@ extern "C" gtb_status gtb_process_block_noalloc(int device, const gtb_options* o
     size_t o_r4 = carve((size_t)rres * sizeof(float4));
     size_t o_co = carve((size_t)(q->n + r->n) * sizeof(int));
     size_t o_rl = carve((size_t)np * sizeof(int));
-    size_t o_rh = carve((size_t)4097 * sizeof(int));
+    size_t o_rh = carve((size_t)RL_NHIST * sizeof(int));
     size_t o_na = carve(2 * sizeof(int));
     if (sz > SCRATCH_BYTES) {
         setmsg(errbuf, errlen, "block needs %lld bytes of working memory; the static scratch holds %lld",
