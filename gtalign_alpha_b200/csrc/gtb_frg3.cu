@@ -14,7 +14,7 @@
 //     structure's 3-d tree (first among residues of the same secondary
 //     structure) and re-superposed; the final superposition's order-dependent
 //     score goes to fragment slot (configuration count mod 32), which keeps
-//     its best (k_f3_search, a warp per pair);
+//     its best (k_f3_search, a cluster per pair);
 //  3. each slot's transform is scored by a gap-0 DP (k_f3_dpscore), the
 //     slots ordered by that score, and the best --nbranches refined by DP +
 //     fragment refinement (the stage-1 kernels), keeping the best branch;
@@ -23,6 +23,8 @@
 // position slots in blocks of 32 reduced by xor-shuffle trees and folded into
 // Neumaier totals, FP64 rotation solve.  Bit-identical to the oracle's
 // frg3_stage.
+#include <algorithm>
+#include <cooperative_groups.h>
 #include "gtb200.h"
 #include "gtb_device.cuh"
 #include "gtb_kernels.cuh"
@@ -40,11 +42,31 @@ constexpr int F3_LENTHR = 150;      // MpStageFrg3.cpp:48: longer structures thi
 constexpr float F3_SSDST2 = 64.f;   // an SS-matched neighbour farther than 8 A is none
 constexpr int F3_MAXWIN = 512;      // the largest --window
 constexpr int F3_WARPS = 4;         // warps per CTA of the search
-constexpr int F3_PERWARP = 4;       // configurations per warp in a round of the search
-constexpr int F3_ROUND = F3_WARPS * F3_PERWARP;
-// the search's dynamic shared memory: a round's results (scored flags, then
-// score + transform per configuration and fragment)
-constexpr int F3_ROUND_BYTES = F3_ROUND * 2 * (int)sizeof(int) + F3_ROUND * 2 * 13 * (int)sizeof(float);
+// CTAs per pair of the search (a cluster) by the pairs of the batch: 8, 4, else
+// 2.  More spread a pair wider, fewer wait less for one another at a round's end;
+// twice as many from 4,096 pairs: the same times within 2%.
+constexpr int F3_NP8 = 256, F3_NP4 = 4096;
+constexpr int F3_GRID = 592;        // CTAs of the search at most (4 per SM)
+constexpr int F3_ENT = 256;         // results of a round (configuration x fragment)
+constexpr unsigned short F3_NONE = 0xffff;   // no residue (an index is below 65535)
+struct F3Walk {                     // a warp's tree walks
+    float diff[F3_MAXSTACK * 32];
+    unsigned short node[F3_MAXSTACK * 32];
+    unsigned char dim[F3_MAXSTACK * 32];
+};
+struct F3Chain {                    // a warp's chain score
+    float max[F3_HASH], ndx[F3_HASH];
+};
+struct alignas(16) F3Smem {
+    unsigned short pq[F3_WARPS][F3_MAXWIN], pr[F3_WARPS][F3_MAXWIN];
+    union { F3Walk walk; F3Chain chain; } u[F3_WARPS];   // never both at once
+    // in the cluster's first CTA: the next configuration of the round, per
+    // entry scored (1) or not, and score and transform
+    int next, slot;
+    unsigned char got[F3_ENT];
+    unsigned short list[F3_ENT];    // the scored entries, in order
+    float res[F3_ENT * 13];
+};
 
 __device__ __forceinline__ int pair_q(const Blk& B, const Bat& T, int i) { return (int)((T.p0 + i) / B.nr); }
 __device__ __forceinline__ int pair_r(const Blk& B, const Bat& T, int i) { return (int)((T.p0 + i) % B.nr); }
@@ -54,14 +76,21 @@ __device__ __forceinline__ int pair_r(const Blk& B, const Bat& T, int i) { retur
 // MpDPHub.cpp:1256-1480): +1 for equal, -1 for different SS, floored at 0
 // (STOP), gap cost per step; the byte per cell is the truncated score
 // rounded down to a multiple of 4 (mod 256) with the direction in its low
-// two bits.  A warp per pair sweeps strips of 32 rows (a row per lane)
-// along anti-diagonals; the previous strip's last row is kept in the pair's
-// row buffer.
-__global__ void __launch_bounds__(128) k_f3_localdp(Blk B, Bat T) {
+// two bits.  A CTA per pair; its warps run the strips of 32 rows (a row per
+// lane) along anti-diagonals as a wavefront: strip s on warp s mod 4, 32 steps
+// at a time, each chunk waiting (a bounded spin) until the previous strip has
+// left the row values it reads in the pair's row buffer.  A chunk's bytes are
+// kept in shared memory and written a row at a time; the columns' letters and
+// the previous strip's row move from lane to lane.  What bounds it: the chain of
+// steps.  (One warp a pair storing a byte per lane and row at each step, with the
+// row buffer read in the chain: 4.3 ms for 2 x 3,000 references; now 1.0.)
+__global__ void __launch_bounds__(F3_WARPS * 32) k_f3_localdp(Blk B, Bat T) {
+    __shared__ volatile int s_prog[F3_WARPS];            // chunks done: strip * nchunks + chunk
+    __shared__ unsigned char s_tile[F3_WARPS][32 * 36];
     const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const int slot = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (slot >= T.rhist[RL_NBUCKET]) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int slot = blockIdx.x;
+    if (slot >= T.rhist[RL_NBUCKET]) return;             // the same for the whole CTA
     const int i = T.rlist[slot];
     const int qi = pair_q(B, T, i), ri = pair_r(B, T, i);
     const int lq = B.qlen[qi], lr = B.rlen[ri];
@@ -69,37 +98,76 @@ __global__ void __launch_bounds__(128) k_f3_localdp(Blk B, Bat T) {
     const char* rs = B.rs + B.roff[ri];
     unsigned char* m = T.lsm + T.off_lsm[i];
     float* row = T.row + T.off_row[i];
+    volatile int* err = T.dw_err;
     const float g = B.f3gapcost;
-    const int nstrips = (lq + 31) >> 5;
-    for (int s = 0; s < nstrips; s++) {
+    const int nstrips = (lq + 31) >> 5, nchunks = (lr + 31 + 31) >> 5;
+    if (threadIdx.x < F3_WARPS) s_prog[threadIdx.x] = 0;
+    __syncthreads();
+    unsigned char* tile = s_tile[w];
+    for (int s = w; s < nstrips; s += F3_WARPS) {
         const int y = s * 32 + lane;
         const bool valid = y < lq;
         const char qss = valid ? qs[y] : 0;
         float h = 0.f;          // this lane's cell of the previous step: (y, j-1)
         float uplast = 0.f;     // (y-1, j-1)
-        unsigned char* my = m + (long long)(valid ? y : 0) * lr;
-        for (int t = 0; t < lr + 31; t++) {
-            const int j = t - lane;
-            float up = __shfl_up_sync(FULL, h, 1);          // lane-1's (y-1, j)
-            if (lane == 0) up = (s > 0 && 0 <= j && j < lr) ? row[j] : 0.f;
-            if (valid && 0 <= j && j < lr) {
-                float dg = j > 0 ? uplast : 0.f;
-                float v = __fadd_rn(__fsub_rn((float)((qss == rs[j]) * 2), 1.0f), dg);
-                int bk = BT_DIAG;
-                if (v < 0.f) { v = 0.f; bk = BT_STOP; }
-                const float l = __fadd_rn(j > 0 ? h : 0.f, g);
-                if (v < l) { v = l; bk = BT_LEFT; }
-                const float u = __fadd_rn(up, g);
-                if (v < u) { v = u; bk = BT_UP; }
-                h = v;
-                my[j] = (unsigned char)((((unsigned)v) & 0xfcu) | (unsigned)bk);
-                // lane 31's row is the next strip's "up" (lane 0 of this strip
-                // read row[j] 31 steps ago)
-                if (lane == 31) row[j] = v;
+        int css = 0;            // the letter of this lane's column
+        for (int c = 0; c < nchunks; c++) {
+            const int t0 = c * 32;
+            if (s > 0) {
+                // row[t0 .. t0+31] of strip s-1: written up to its step t0+62
+                const int need = (s - 1) * nchunks + (c + 2 < nchunks ? c + 2 : nchunks);
+                int ok = 1;
+                if (lane == 0) {
+                    long long it = 0;
+                    while (s_prog[(w + F3_WARPS - 1) % F3_WARPS] < need) {
+                        if (*err || ++it > T.dw_spin) { *err = 1; ok = 0; break; }
+                        __nanosleep(32);
+                    }
+                }
+                if (!__shfl_sync(FULL, ok, 0)) return;
+                __threadfence_block();
             }
-            uplast = up;
+            const int jj = t0 + lane;
+            const float rb = s > 0 && jj < lr ? row[jj] : 0.f;
+            const int cb = jj < lr ? rs[jj] : 0;
+            __syncwarp();
+#pragma unroll 8
+            for (int u = 0; u < 32; u++) {
+                const int j = t0 + u - lane;
+                const float r0 = __shfl_sync(FULL, rb, u);
+                const int c0 = __shfl_sync(FULL, cb, u);
+                float up = __shfl_up_sync(FULL, h, 1);          // lane-1's (y-1, j)
+                css = __shfl_up_sync(FULL, css, 1);
+                if (lane == 0) { up = r0; css = c0; }
+                if (0 <= j && j < lr) {
+                    float v = __fadd_rn(__fsub_rn((float)((qss == (char)css) * 2), 1.0f), j > 0 ? uplast : 0.f);
+                    int bk = BT_DIAG;
+                    if (v < 0.f) { v = 0.f; bk = BT_STOP; }
+                    const float l = __fadd_rn(j > 0 ? h : 0.f, g);
+                    if (v < l) { v = l; bk = BT_LEFT; }
+                    const float x = __fadd_rn(up, g);
+                    if (v < x) { v = x; bk = BT_UP; }
+                    h = v;
+                    tile[lane * 36 + u] = (unsigned char)((((unsigned)v) & 0xfcu) | (unsigned)bk);
+                    // lane 31's row is the next strip's "up"
+                    if (lane == 31) row[j] = v;
+                }
+                uplast = up;
+            }
+            __syncwarp();
+            // row r's bytes of this chunk: columns t0 - r ...
+            const int nrow = lq - s * 32 < 32 ? lq - s * 32 : 32;
+#pragma unroll 4
+            for (int r = 0; r < nrow; r++) {
+                const int j = t0 - r + lane;
+                if (0 <= j && j < lr) m[(long long)(s * 32 + r) * lr + j] = tile[r * 36 + lane];
+            }
+            __syncwarp();
+            if (lane == 31) {
+                __threadfence_block();                   // the row values before the count
+                s_prog[w] = s * nchunks + c + 1;
+            }
         }
-        __syncwarp();           // the row buffer before the next strip reads it
     }
 }
 
@@ -176,7 +244,8 @@ __device__ bool f3_similar(const unsigned char* m, int lq, int lr, int qrypos, i
 // rectangle from (qrypos, rfnpos); the pairs go to pq/pr in increasing order.
 // Returns their number (0: too few), the same on every lane.
 __device__ int f3_seed_local(const unsigned char* m, int lq, int lr, int trig, int fraglen,
-                             int qrypos, int rfnpos, int* pq, int* pr, int lane) {
+                             int qrypos, int rfnpos, unsigned short* pq,
+                             unsigned short* pr, int lane) {
     int n = 0;
     if (lane == 0) {
         if (lq < qrypos + fraglen && lr < rfnpos + fraglen)
@@ -196,13 +265,13 @@ __device__ int f3_seed_local(const unsigned char* m, int lq, int lr, int trig, i
             if (b == BT_STOP) break;
             if (b == BT_UP) { y--; continue; }
             if (b == BT_LEFT) { x--; continue; }
-            pq[n] = y; pr[n] = x; n++;
+            pq[n] = (unsigned short)y; pr[n] = (unsigned short)x; n++;
             x--; y--;
         }
         const int minf = fraglen < 16 ? fraglen : 16;
         if (n < 1 || (trig && n < minf)) n = 0;
         for (int a = 0, b = n - 1; a < b; a++, b--) {
-            int t = pq[a]; pq[a] = pq[b]; pq[b] = t;
+            unsigned short t = pq[a]; pq[a] = pq[b]; pq[b] = t;
             t = pr[a]; pr[a] = pr[b]; pr[b] = t;
         }
     }
@@ -210,21 +279,21 @@ __device__ int f3_seed_local(const unsigned char* m, int lq, int lr, int trig, i
     return __shfl_sync(0xffffffffu, n, 0);
 }
 
-// Covariance sums over position slots 0..n-1 (pq/pr; a negative index: no
+// Covariance sums over position slots 0..n-1 (pq/pr; F3_NONE: no
 // pair): lane k of block b takes slot 32b + k; each block's values are
 // summed by the xor-shuffle tree and folded into Neumaier totals in block
 // order.  Every lane gets the 16 values (15 sums and the count).
 __device__ void f3_cov(const float* qx, const float* qy, const float* qz, const float* rx,
-                       const float* ry, const float* rz, const int* pq, const int* pr, int n,
-                       float* v, int lane) {
+                       const float* ry, const float* rz, const unsigned short* pq,
+                       const unsigned short* pr, int n, float* v, int lane) {
     float s[15], c[15];
 #pragma unroll
     for (int f = 0; f < 15; f++) { s[f] = 0.f; c[f] = 0.f; }
     int cnt = 0;
     for (int b0 = 0; b0 < n; b0 += 32) {
         const int k = b0 + lane;
-        const int a = k < n ? pq[k] : -1, b = k < n ? pr[k] : -1;
-        const bool ok = a >= 0 && b >= 0;
+        const int a = k < n ? pq[k] : F3_NONE, b = k < n ? pr[k] : F3_NONE;
+        const bool ok = a != F3_NONE && b != F3_NONE;
         const float x0 = ok ? qx[a] : 0.f, y0 = ok ? qy[a] : 0.f, z0 = ok ? qz[a] : 0.f;
         const float x1 = ok ? rx[b] : 0.f, y1 = ok ? ry[b] : 0.f, z1 = ok ? rz[b] : 0.f;
         float t[15] = {__fmul_rn(x0, x1), __fmul_rn(x0, y1), __fmul_rn(x0, z1),
@@ -307,11 +376,11 @@ struct F3Pair {
 
 // Neighbours over the window of the shorter structure
 // (ProduceAlignmentUsingIndex2Reference/Query, MpStageFrg3.h:500-680), a
-// window slot per lane per round; fills pq/pr (-1: empty), returns the
+// window slot per lane per round; fills pq/pr (F3_NONE: empty), returns the
 // window length.
 __device__ int f3_window(const F3Pair& P, const float* tfm, bool ssfilt, int window, int qrypos,
-                         int rfnpos, int stacksize, int* pq, int* pr, int lane, unsigned short* sn,
-                         float* sd, unsigned char* sm) {
+                         int rfnpos, int stacksize, unsigned short* pq, unsigned short* pr, int lane,
+                         unsigned short* sn, float* sd, unsigned char* sm) {
     const int lq = P.lq, lr = P.lr;
     int n;
     if (lq < lr) {
@@ -325,8 +394,8 @@ __device__ int f3_window(const F3Pair& P, const float* tfm, bool ssfilt, int win
             float x, y, z;
             xform(tfm, P.qx[q], P.qy[q], P.qz[q], x, y, z);
             const int r = f3_nn(P.rnd, P.rnc, lr, ssfilt, P.qs[q], x, y, z, stacksize, sn, sd, sm);
-            pq[pi] = q;
-            pr[pi] = r > 0 ? r : -1;
+            pq[pi] = (unsigned short)q;
+            pr[pi] = r > 0 ? (unsigned short)r : F3_NONE;
         }
     } else {
         const int fl = lq < window ? lq : window;
@@ -339,8 +408,8 @@ __device__ int f3_window(const F3Pair& P, const float* tfm, bool ssfilt, int win
             float x, y, z;
             xform(tfm, P.rx[r], P.ry[r], P.rz[r], x, y, z);
             const int q = f3_nn(P.qnd, P.qnc, lq, ssfilt, P.rs[r], x, y, z, stacksize, sn, sd, sm);
-            pq[pi] = q > 0 ? q : -1;
-            pr[pi] = r;
+            pq[pi] = q > 0 ? (unsigned short)q : F3_NONE;
+            pr[pi] = (unsigned short)r;
         }
     }
     __syncwarp();
@@ -358,8 +427,8 @@ __device__ int f3_window(const F3Pair& P, const float* tfm, bool ssfilt, int win
 // running maximum of the entries below the partner's: the table is then
 // kept as prefix maxima (pm[k] = max of entries 0..k), read with one load
 // and raised by every lane for its own entries at or above the partner's.
-__device__ float f3_progressive(const F3Pair& P, const float* tfm, float d02, const int* pq,
-                                const int* pr, int cnt, bool partner_is_r, float* omax,
+__device__ float f3_progressive(const F3Pair& P, const float* tfm, float d02, const unsigned short* pq,
+                                const unsigned short* pr, int cnt, bool partner_is_r, float* omax,
                                 float* ondx, int lane) {
     if ((partner_is_r ? P.lr : P.lq) <= F3_HASH) {
         float* pm = omax;
@@ -367,7 +436,7 @@ __device__ float f3_progressive(const F3Pair& P, const float* tfm, float d02, co
         __syncwarp();
         for (int pi = 0; pi < cnt; pi++) {
             const int a = pq[pi], b = pr[pi];
-            if (a < 0 || b < 0) continue;          // the same on every lane
+            if (a == F3_NONE || b == F3_NONE) continue;   // the same on every lane
             const float d = dist2_tf(tfm, P.qx[a], P.qy[a], P.qz[a], P.rx[b], P.ry[b], P.rz[b]);
             const float sco = tmterm(d02, d);
             if (!(0.f < sco)) continue;
@@ -386,7 +455,7 @@ __device__ float f3_progressive(const F3Pair& P, const float* tfm, float d02, co
     __syncwarp();
     for (int pi = 0; pi < cnt; pi++) {
         const int a = pq[pi], b = pr[pi];
-        if (a < 0 || b < 0) continue;          // the same on every lane
+        if (a == F3_NONE || b == F3_NONE) continue;   // the same on every lane
         const float d = dist2_tf(tfm, P.qx[a], P.qy[a], P.qz[a], P.rx[b], P.ry[b], P.rz[b]);
         const float sco = tmterm(d02, d);
         if (!(0.f < sco)) continue;
@@ -420,146 +489,175 @@ __device__ __forceinline__ int f3_stacksize(int lq, int lr) {
     return b < F3_MAXSTACK ? b : F3_MAXSTACK;
 }
 
-// A CTA per listed pair; a round is F3_ROUND consecutive configurations,
-// F3_PERWARP per warp (interleaved, so that cheap and dear ones mix); a
-// scored configuration's slot is the pair's count of scored configurations
-// before it mod 32, and the slot keeps its best: after each round the
-// round's results are applied in configuration order, as one warp going
-// through the configurations in order would.
-__global__ void __launch_bounds__(F3_WARPS * 32, 3) k_f3_search(Blk B, Bat T, int depth) {
-    __shared__ int s_pq[F3_WARPS][F3_MAXWIN], s_pr[F3_WARPS][F3_MAXWIN];
-    __shared__ float s_omax[F3_WARPS][F3_HASH], s_ondx[F3_WARPS][F3_HASH];
-    __shared__ unsigned short s_stkn[F3_WARPS][F3_MAXSTACK * 32];
-    __shared__ float s_stkd[F3_WARPS][F3_MAXSTACK * 32];
-    __shared__ unsigned char s_stkm[F3_WARPS][F3_MAXSTACK * 32];
-    // a round's results (F3_ROUND_BYTES, dynamic): per configuration of the
-    // round and fragment, scored (1) or not; score and transform
-    extern __shared__ float s_dyn[];
-    int* s_got = (int*)s_dyn;
-    float* s_res = s_dyn + F3_ROUND * 2;
+__device__ __forceinline__ void f3_sync(cooperative_groups::cluster_group& cl, int C) {
+    if (C > 1) cl.sync();
+    else __syncthreads();
+}
+
+// A cluster of CTAs per listed pair (the grid's clusters walk the list,
+// largest pairs first).  A round is F3_ENT consecutive entries (configuration
+// x fragment); the cluster's warps draw the round's configurations one at a
+// time and leave their results in the first CTA's shared memory.  A scored
+// entry's slot is the pair's count of scored entries before it mod 32, and the
+// slot keeps its best: after the round, lane j of one warp goes through the
+// entries of slot j in order, as one warp going through all configurations
+// would.  What bounds it: the latency of the tree walks.  With one CTA a pair
+// and rounds of 16 configurations a launch lasted as long as its largest pair,
+// SMs busy a fifth of the time: 42 ms for 2 x 3,000 references, now 10; for
+// 2 x 8,000 the stage's own kernels took 61 ms, now 36 (with 3 CTAs a SM 66).
+__global__ void __launch_bounds__(F3_WARPS * 32, 4) k_f3_search(Blk B, Bat T, int depth) {
+    extern __shared__ __align__(16) unsigned char f3_smem[];
+    F3Smem& S = *(F3Smem*)f3_smem;
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    const int C = (int)cl.num_blocks(), crank = (int)cl.block_rank();
+    F3Smem& S0 = *cl.map_shared_rank(&S, 0);       // the first CTA's
+    const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int slot = blockIdx.x;
-    if (slot >= T.rhist[RL_NBUCKET]) return;       // the same for the whole CTA
-    const int i = T.rlist[slot];
-    const int qi = pair_q(B, T, i), ri = pair_r(B, T, i);
-    F3Pair P;
-    P.lq = B.qlen[qi]; P.lr = B.rlen[ri];
-    const int qo = B.qoff[qi], ro = B.roff[ri];
-    P.qx = B.qx + qo; P.qy = B.qy + qo; P.qz = B.qz + qo;
-    P.rx = B.rx + ro; P.ry = B.ry + ro; P.rz = B.rz + ro;
-    P.qs = B.qs + qo; P.rs = B.rs + ro;
-    P.qnd = B.qnd + qo; P.qnc = B.qnc + qo;
-    P.rnd = B.rnd + ro; P.rnc = B.rnc + ro;
-    const int lq = P.lq, lr = P.lr;
-    const int ml = lq < lr ? lq : lr;
-    const float d0 = B.t_d0[ml];
-    const float d02 = __fmul_rn(d0, d0);
-    const unsigned char* m = T.lsm + T.off_lsm[i];
-    int* pq = s_pq[w];
-    int* pr = s_pr[w];
-    unsigned short* sn = s_stkn[w] + lane;
-    float* sd = s_stkd[w] + lane;
-    unsigned char* sm = s_stkm[w] + lane;
-    const int nsec = B.f3nsec;
-    float* slots = T.f3slot + (long long)i * nsec * F3_NTOP * 13;
-    for (int k = threadIdx.x; k < nsec * F3_NTOP; k += blockDim.x) slots[k * 13] = 0.f;
-    const float thr = __fdiv_rn((float)B.f3trigger, 100.0f);
-    const int seedrule = B.f3seedrule;
-    const int qstep = f3_step(depth, lq), rstep = f3_step(depth, lr);
-    const int minn = depth == 3 ? 5 : 10;
-    int nsy = lq / qstep + 1; if (nsy < minn) nsy = minn;
-    int nsx = lr / rstep + 1; if (nsx < minn) nsx = minn;
-    const int nconf = nsy * nsx;
-    const int stacksize = f3_stacksize(lq, lr);
-    const int f0 = f3_fraglen(lq, lr, 0, 0), f1 = f3_fraglen(lq, lr, 1, 0);
-    const int nfr = seedrule ? 1 : 2;
-    int nscored = 0;                              // kept by thread 0
-    for (int c0 = 0; c0 < nconf; c0 += F3_ROUND)
-    for (int jj = 0; jj <= F3_PERWARP; jj++) {
-      if (jj == F3_PERWARP) {
-        // the round's results in configuration order
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int rr = 0; rr < F3_ROUND; rr++) {
-                // the sections this configuration feeds: section 0 all; at
-                // --depth 1 and 0 sections 1 and 2 those on every second /
-                // third grid row and column of a structure longer than
-                // F3_LENTHR (sec2met, sec3met: MpStageFrg3.cpp:204-212)
-                const int cc = c0 + rr, ys = cc / nsx, xs = cc % nsx;
-                const bool sec1 = nsec > 1 && (lq <= F3_LENTHR || (ys & 1) == 0) &&
-                                  (lr <= F3_LENTHR || (xs & 1) == 0);
-                const bool sec2 = nsec > 2 && (lq <= F3_LENTHR || ys % 3 == 0) &&
-                                  (lr <= F3_LENTHR || xs % 3 == 0);
-                for (int fi = 0; fi < 2; fi++) {
-                    if (!s_got[rr * 2 + fi]) continue;
-                    const int k = nscored % F3_NTOP;
-                    nscored++;
-                    const float* res = s_res + (rr * 2 + fi) * 13;
-                    const float sc = res[0];
-                    if (!(0.0f < sc)) continue;
-                    for (int sec = 0; sec < nsec; sec++) {
-                        if ((sec == 1 && !sec1) || (sec == 2 && !sec2)) continue;
-                        float* sl = slots + (sec * F3_NTOP + k) * 13;
-                        if (sl[0] < sc) {
-                            sl[0] = sc;
-                            for (int f = 0; f < 12; f++) sl[1 + f] = res[1 + f];
-                        }
-                    }
-                }
+    unsigned short* pq = S.pq[w];
+    unsigned short* pr = S.pr[w];
+    unsigned short* sn = S.u[w].walk.node + lane;
+    float* sd = S.u[w].walk.diff + lane;
+    unsigned char* sm = S.u[w].walk.dim + lane;
+    const int nlist = T.rhist[RL_NBUCKET], ncl = (int)gridDim.x / C;
+    int* ctr = T.rhist + RL_NBUCKET + 1;
+    for (int slot = (int)blockIdx.x / C; slot < nlist;) {
+        const int i = T.rlist[slot];
+        const int qi = pair_q(B, T, i), ri = pair_r(B, T, i);
+        F3Pair P;
+        P.lq = B.qlen[qi]; P.lr = B.rlen[ri];
+        const int qo = B.qoff[qi], ro = B.roff[ri];
+        P.qx = B.qx + qo; P.qy = B.qy + qo; P.qz = B.qz + qo;
+        P.rx = B.rx + ro; P.ry = B.ry + ro; P.rz = B.rz + ro;
+        P.qs = B.qs + qo; P.rs = B.rs + ro;
+        P.qnd = B.qnd + qo; P.qnc = B.qnc + qo;
+        P.rnd = B.rnd + ro; P.rnc = B.rnc + ro;
+        const int lq = P.lq, lr = P.lr;
+        const int ml = lq < lr ? lq : lr;
+        const float d0 = B.t_d0[ml];
+        const float d02 = __fmul_rn(d0, d0);
+        const unsigned char* m = T.lsm + T.off_lsm[i];
+        const int nsec = B.f3nsec;
+        float* slots = T.f3slot + (long long)i * nsec * F3_NTOP * 13;
+        if (crank == 0)
+            for (int k = threadIdx.x; k < nsec * F3_NTOP; k += blockDim.x) slots[k * 13] = 0.f;
+        const float thr = __fdiv_rn((float)B.f3trigger, 100.0f);
+        const int seedrule = B.f3seedrule;
+        const int qstep = f3_step(depth, lq), rstep = f3_step(depth, lr);
+        const int minn = depth == 3 ? 5 : 10;
+        int nsy = lq / qstep + 1; if (nsy < minn) nsy = minn;
+        int nsx = lr / rstep + 1; if (nsx < minn) nsx = minn;
+        const int nconf = nsy * nsx;
+        const int stacksize = f3_stacksize(lq, lr);
+        const int f0 = f3_fraglen(lq, lr, 0, 0), f1 = f3_fraglen(lq, lr, 1, 0);
+        const int nfr = seedrule ? 1 : 2;
+        const int rconf = F3_ENT / nfr;               // configurations of a round
+        int nscored = 0;                              // kept by the first CTA's first warp
+        for (int c0 = 0; c0 < nconf; c0 += rconf) {
+            const int nc = nconf - c0 < rconf ? nconf - c0 : rconf;
+            if (crank == 0) {
+                for (int k = threadIdx.x; k < F3_ENT; k += blockDim.x) S.got[k] = 0;
+                if (threadIdx.x == 0) S.next = 0;
             }
-        }
-        __syncthreads();
-        continue;
-      }
-        const int rix = w + F3_WARPS * jj;        // this configuration's place in the round
-        const int c = c0 + rix;
-        if (lane < 2) s_got[rix * 2 + lane] = 0;
-        __syncwarp();
-        if (c < nconf) {
-            const int qrypos = (c / nsx) * qstep, rfnpos = (c % nsx) * rstep;
-            bool go = !(lq < qrypos + f0 || lr < rfnpos + f0 || f0 < 1);
-            const bool conv1 = (lq < qrypos + f1 || lr < rfnpos + f1 || f1 < 1);
-            if (go && 0.0f < thr && !f3_similar(m, lq, lr, qrypos, rfnpos, f1, thr, lane)) go = false;
-            for (int fi = 0; go && fi < nfr; fi++) {
-                if (fi == 1 && conv1) continue;
-                const int fraglen = fi == 0 ? f0 : f1;
-                if (lq < qrypos + fraglen || lr < rfnpos + fraglen) continue;
-                float v[16], tfm[12];
-                int n;
-                if (seedrule) {
-                    n = f3_seed_local(m, lq, lr, B.f3trigger > 0, f3_fraglen(lq, lr, fi, seedrule),
-                                      qrypos, rfnpos, pq, pr, lane);
-                } else {
-                    for (int k = lane; k < fraglen; k += 32) { pq[k] = qrypos + k; pr[k] = rfnpos + k; }
+            f3_sync(cl, C);
+            for (;;) {
+                int k = 0;
+                if (lane == 0) k = atomicAdd(&S0.next, 1);
+                k = __shfl_sync(FULL, k, 0);
+                if (k >= nc) break;
+                const int c = c0 + k;
+                const int qrypos = (c / nsx) * qstep, rfnpos = (c % nsx) * rstep;
+                bool go = !(lq < qrypos + f0 || lr < rfnpos + f0 || f0 < 1);
+                const bool conv1 = (lq < qrypos + f1 || lr < rfnpos + f1 || f1 < 1);
+                if (go && 0.0f < thr && !f3_similar(m, lq, lr, qrypos, rfnpos, f1, thr, lane)) go = false;
+                for (int fi = 0; go && fi < nfr; fi++) {
+                    if (fi == 1 && conv1) continue;
+                    const int fraglen = fi == 0 ? f0 : f1;
+                    if (lq < qrypos + fraglen || lr < rfnpos + fraglen) continue;
+                    float v[16], tfm[12];
+                    int n;
+                    if (seedrule) {
+                        n = f3_seed_local(m, lq, lr, B.f3trigger > 0, f3_fraglen(lq, lr, fi, seedrule),
+                                          qrypos, rfnpos, pq, pr, lane);
+                    } else {
+                        for (int p = lane; p < fraglen; p += 32) { pq[p] = (unsigned short)(qrypos + p); pr[p] = (unsigned short)(rfnpos + p); }
+                        __syncwarp();
+                        n = fraglen;
+                    }
+                    if (n < 1) continue;
+                    f3_cov(P.qx, P.qy, P.qz, P.rx, P.ry, P.rz, pq, pr, n, v, lane);
                     __syncwarp();
-                    n = fraglen;
-                }
-                if (n < 1) continue;
-                f3_cov(P.qx, P.qy, P.qz, P.rx, P.ry, P.rz, pq, pr, n, v, lane);
-                __syncwarp();
-                if (v[15] < 1.0f) continue;
-                solve_sums(v, lq < lr ? 0 : 2, tfm);
-                for (int it = 0; it < 2; it++) {
-                    const int cw = f3_window(P, tfm, it == 0, B.f3window, qrypos, rfnpos, stacksize,
-                                             pq, pr, lane, sn, sd, sm);
-                    f3_cov(P.qx, P.qy, P.qz, P.rx, P.ry, P.rz, pq, pr, cw, v, lane);
-                    if (v[15] < 1.0f) { __syncwarp(); continue; }
-                    if (it == 0) { solve_sums(v, lq < lr ? 0 : 2, tfm); __syncwarp(); continue; }
-                    solve_sums(v, 0, tfm);
-                    const float sc = f3_progressive(P, tfm, d02, pq, pr, (int)v[15], lq < lr,
-                                                    s_omax[w], s_ondx[w], lane);
-                    if (lane == 0) {
-                        float* res = s_res + (rix * 2 + fi) * 13;
-                        s_got[rix * 2 + fi] = 1;
-                        res[0] = sc;
+                    if (v[15] < 1.0f) continue;
+                    solve_sums(v, lq < lr ? 0 : 2, tfm);
+                    for (int it = 0; it < 2; it++) {
+                        const int cw = f3_window(P, tfm, it == 0, B.f3window, qrypos, rfnpos, stacksize,
+                                                 pq, pr, lane, sn, sd, sm);
+                        f3_cov(P.qx, P.qy, P.qz, P.rx, P.ry, P.rz, pq, pr, cw, v, lane);
+                        if (v[15] < 1.0f) { __syncwarp(); continue; }
+                        solve_sums(v, it == 0 ? (lq < lr ? 0 : 2) : 0, tfm);
+                        if (it == 0) { __syncwarp(); continue; }
+                        const float sc = f3_progressive(P, tfm, d02, pq, pr, (int)v[15], lq < lr,
+                                                        S.u[w].chain.max, S.u[w].chain.ndx, lane);
+                        if (lane == 0) {
+                            float* res = S0.res + (k * nfr + fi) * 13;
+                            S0.got[k * nfr + fi] = 1;
+                            res[0] = sc;
 #pragma unroll
-                        for (int f = 0; f < 12; f++) res[1 + f] = tfm[f];
+                            for (int f = 0; f < 12; f++) res[1 + f] = tfm[f];
+                        }
+                        __syncwarp();
                     }
-                    __syncwarp();
                 }
             }
+            f3_sync(cl, C);
+            if (crank == 0) {
+                if (w == 0) {
+                    int cnt = 0;
+                    for (int e0 = 0; e0 < nc * nfr; e0 += 32) {
+                        const bool g = e0 + lane < nc * nfr && S.got[e0 + lane];
+                        const unsigned gm = __ballot_sync(FULL, g);
+                        if (g) S.list[cnt + __popc(gm & ((1u << lane) - 1u))] = (unsigned short)(e0 + lane);
+                        cnt += __popc(gm);
+                    }
+                    __syncwarp();
+                    // the sections an entry feeds: section 0 all; at --depth 1 and
+                    // 0 sections 1 and 2 the configurations on every second /
+                    // third grid row and column of a structure longer than
+                    // F3_LENTHR (sec2met, sec3met: MpStageFrg3.cpp:204-212)
+                    float best[F3_NSEC];
+                    int src[F3_NSEC];
+#pragma unroll
+                    for (int sec = 0; sec < F3_NSEC; sec++) {
+                        best[sec] = sec < nsec ? slots[(sec * F3_NTOP + lane) * 13] : 0.f;
+                        src[sec] = -1;
+                    }
+                    for (int e = (lane - nscored) & (F3_NTOP - 1); e < cnt; e += F3_NTOP) {
+                        const int en = S.list[e];
+                        const float sc = S.res[en * 13];
+                        if (!(0.0f < sc)) continue;
+                        const int cc = c0 + en / nfr, ys = cc / nsx, xs = cc % nsx;
+                        const bool in[F3_NSEC] = {true,
+                                                  (lq <= F3_LENTHR || (ys & 1) == 0) && (lr <= F3_LENTHR || (xs & 1) == 0),
+                                                  (lq <= F3_LENTHR || ys % 3 == 0) && (lr <= F3_LENTHR || xs % 3 == 0)};
+#pragma unroll
+                        for (int sec = 0; sec < F3_NSEC; sec++)
+                            if (sec < nsec && in[sec] && best[sec] < sc) { best[sec] = sc; src[sec] = en; }
+                    }
+                    nscored += cnt;
+#pragma unroll
+                    for (int sec = 0; sec < F3_NSEC; sec++)
+                        if (src[sec] >= 0)
+                            for (int f = 0; f < 13; f++)
+                                slots[(sec * F3_NTOP + lane) * 13 + f] = S.res[src[sec] * 13 + f];
+                }
+                __syncthreads();
+            }
         }
+        // the first pair by position, the next ones as clusters come free
+        if (crank == 0 && threadIdx.x == 0) S.slot = ncl + atomicAdd(ctr, 1);
+        f3_sync(cl, C);
+        slot = S0.slot;
     }
+    f3_sync(cl, C);                    // the first CTA's shared memory is read until here
 }
 
 // ---------------------------------------------------------------------------
@@ -628,19 +726,30 @@ __global__ void k_f3_second(Blk B, Bat T, int rci) {
 // own lists, so the frg3 list is rebuilt before each frg3 kernel that
 // reads it.
 void launch_frg3(const Blk& B, const Bat& T, cudaStream_t st) {
-    const int nb = (T.np + 3) / 4;
     auto plist = [&]() { launch_pair_list(B, T, CONV_LOWTMSC, st); };
     plist();
     const int nbr = B.f3nbranches < F3_NBMAX ? B.f3nbranches : F3_NBMAX;
     {
         KtScope kts(T, KF_FRG3, st);
         if (0 < B.f3trigger || B.f3seedrule) {
-            k_f3_localdp<<<nb, 128, 0, st>>>(B, T);
+            k_f3_localdp<<<T.np, F3_WARPS * 32, 0, st>>>(B, T);
             if (T.launches) (*T.launches)++;
         }
-        // static arrays (~48 kB) + the round's results go past the default 48 kB
-        cudaFuncSetAttribute(k_f3_search, cudaFuncAttributeMaxDynamicSharedMemorySize, F3_ROUND_BYTES);
-        k_f3_search<<<T.np, F3_WARPS * 32, F3_ROUND_BYTES, st>>>(B, T, B.depth);
+        cudaFuncSetAttribute(k_f3_search, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(F3Smem));
+        cudaLaunchConfig_t cfg{};
+        const int C = T.np <= F3_NP8 ? 8 : T.np <= F3_NP4 ? 4 : 2;
+        cfg.gridDim = dim3(std::min(T.np, F3_GRID / C) * C);
+        cfg.blockDim = dim3(F3_WARPS * 32);
+        cfg.dynamicSmemBytes = sizeof(F3Smem);
+        cfg.stream = st;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = C;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, k_f3_search, B, T, B.depth);
+        if (e != cudaSuccess && T.lerr && *T.lerr == cudaSuccess) *T.lerr = e;
         if (T.launches) (*T.launches)++;
         launch_f3_dpscore(B, T, st);
         k_f3_select<<<(T.np + 255) / 256, 256, 0, st>>>(B, T, nbr);

@@ -372,3 +372,19 @@ def test_dp_strip_edges(oracle, opt):
     q, r = synth.pack(q), synth.pack(r)
     res, ora = run_both(oracle, q, r, OPTSETS[opt])
     assert_same(res, ora, q.n, r.n)
+
+
+@pytest.mark.parametrize("fill,depth", [(300, 2), (300, 0), (4200, 3)])
+def test_detailed_search_batches(oracle, fill, depth):
+    """The detailed search in batches of each size class (its CTAs per pair),
+    with pairs of few and of many configurations (several rounds at --depth 0):
+    GPU against the oracle bit for bit."""
+    from gtalign_alpha_b200 import synth
+    rng = np.random.default_rng(fill + depth)
+    q = synth.random_chains(rng, [320 if fill < 1000 else 90], "q")
+    r = [synth.homolog(rng, q[0], s, 0.05, "h") for s in (1.0, 2.5)]
+    r += synth.random_chains(rng, rng.integers(20, 30, fill), "f")
+    q, r = synth.pack(q), synth.pack(r)
+    d = dict(OPTSETS["frg3s12"], depth=depth, prescore=0.2)
+    res, ora = run_both(oracle, q, r, d)
+    assert_same(res, ora, q.n, r.n)
