@@ -81,6 +81,18 @@ class TMScore(torch.autograd.Function):
         q, tfm, off, n, g, gq = ctx.saved_tensors
         P = tfm.shape[0]
         N = q.shape[0]
+        # one kernel, unless the backward pass itself is to be differentiated
+        if P and not torch.is_grad_enabled():
+            grad_q = torch.zeros_like(gq)
+            grad_tfm = torch.empty(P, 12, dtype=torch.float32, device=q.device)
+            qc, tc, go = q.contiguous(), tfm.contiguous(), gout.contiguous()
+            st = load_library().gtb_tm_backward(
+                None, P, _ptr(off), _ptr(n), _ptr(qc), _ptr(gq), _ptr(tc), _ptr(g), _ptr(go),
+                _ptr(grad_q), _ptr(grad_tfm),
+                ctypes.c_void_p(torch.cuda.current_stream(q.device).cuda_stream))
+            if st != 0:
+                raise GTBError(st, "gtb_tm_backward failed")
+            return grad_q, grad_tfm, None, None, None, None
         # pair index and residue row of every aligned position, on the device:
         # row = off[pair] + (position - first position of the pair)
         nl = n.long()

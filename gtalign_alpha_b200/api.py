@@ -189,6 +189,8 @@ def load_library():
     L.gtb_tm_adjoint.restype = ctypes.c_int
     L.gtb_polish.argtypes = [vp, ctypes.c_int, vp, vp, vp, vp, vp, vp, ctypes.c_int, vp, vp, vp]
     L.gtb_polish.restype = ctypes.c_int
+    L.gtb_tm_backward.argtypes = [vp, ctypes.c_int] + [vp] * 10
+    L.gtb_tm_backward.restype = ctypes.c_int
     _lib = L
     return L
 

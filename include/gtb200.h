@@ -231,6 +231,16 @@ gtb_status gtb_tm_adjoint(gtb_handle* h, int npairs, const long long* off,
                           const float* tfm, const float* d0,
                           float* tm, float* grad, float* gq, void* stream);
 
+/* Backward pass of the scores as a function of the query coordinates and the
+ * transforms: from gtb_tm_adjoint's grad and gq and the incoming gradient
+ * gout[p] of tm[p], grad_q[row] = gout * gq[row] for the rows of the pairs
+ * (others are left as they are) and grad_tfm[p*12..] = gout * (dTM/dR row-major,
+ * dTM/dt).  Device pointers, stream. */
+gtb_status gtb_tm_backward(gtb_handle* h, int npairs, const long long* off, const int* n,
+                           const float* qxyz, const float* gq, const float* tfm,
+                           const float* grad, const float* gout, float* grad_q,
+                           float* grad_tfm, void* stream);
+
 /* Projected-gradient polishing of transforms on SO(3) x R^3 for fixed
  * alignments: `steps` ascent steps with backtracking; a step is only
  * accepted when it does not lower the TM-score.  Device pointers, stream.

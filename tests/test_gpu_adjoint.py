@@ -178,3 +178,35 @@ def test_polishing_in_the_search_never_lowers_the_score():
     gain = short[1] - short[0]
     assert (gain > 1e-5).sum() > 5
     assert float(np.max(res[10].numerr[0][:, :2])) < 1e-5  # FP32 vs FP64 of the polished transform
+
+
+@pytest.mark.parametrize("lens", [(1, 31, 32, 33, 600), (0, 64, 5)])
+def test_autograd_rows_weights_and_layouts(lens):
+    """The backward kernel on short, empty and long pairs with rows that belong
+    to no pair, an expanded incoming gradient and a strided q, against the
+    backward pass that can itself be differentiated (torch operations)."""
+    import torch
+    from gtalign_alpha_b200.adjoint import TMScore
+    rng = np.random.default_rng(len(lens))
+    P, gap = len(lens), 3
+    off = np.cumsum([0] + [n + gap for n in lens[:-1]])
+    N = int(off[-1] + lens[-1] + gap)
+    T = lambda a, t=torch.float32: torch.from_numpy(np.ascontiguousarray(a)).to("cuda", t)
+    q2 = T(rng.normal(0, 10, (N, 6)))
+    r = q2[:, :3].contiguous() + T(rng.normal(0, 2, (N, 3)))
+    tfm = T(np.tile(np.concatenate([np.eye(3).ravel(), [0.3, -0.2, 0.1]]), (P, 1)))
+    args = (r, T(off, torch.int64), T(np.array(lens), torch.int32), T(np.full(P, 3.0)))
+    out = []
+    for create in (False, True):
+        q = q2[:, ::2].detach().requires_grad_(True)          # rows of 6 floats, every second
+        t = tfm.clone().requires_grad_(True)
+        tm = TMScore.apply(q, t, *args)
+        out.append(torch.autograd.grad(tm, (q, t), torch.tensor(0.7, device="cuda").expand(P),
+                                       create_graph=create))
+    for a, b in zip(*out):
+        # sums of up to 600 terms in FP32, in two orders
+        assert (a - b).abs().max() <= 600 * 2.0 ** -24 * b.abs().max()
+    covered = torch.zeros(N, dtype=torch.bool)
+    for o, n in zip(off, lens):
+        covered[o:o + n] = True
+    assert (out[0][0].cpu()[~covered] == 0).all()
