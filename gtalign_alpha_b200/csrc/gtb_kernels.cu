@@ -882,6 +882,9 @@ void launch_findfrag(const Blk& B, const Bat& T, cudaStream_t st) {
 // finished pairs cost nothing.  Pairs left out get the mode's outputs for
 // "no variant scored" here.
 constexpr int RL_SHIFT = 4;
+// up to here one CTA builds a list (4 pairs a thread): one pair 4.9 -> 4.2 ms,
+// 1 x 1,000 at the fastest preset 7.5 -> 7.2
+constexpr int LIST_SMALL = 4096;
 constexpr int RL_NB = 65536 >> RL_SHIFT;   // buckets; rhist[RL_NB] = list length
 
 // position count of pair i in mode `mode`, or -1 when the pair is skipped
@@ -896,23 +899,28 @@ __device__ __forceinline__ int refine_span(const Blk& B, const Bat& T, int mode,
     return (lq - sq) < (lr - sr) ? (lq - sq) : (lr - sr);
 }
 
-__global__ void k_rlist_count(Blk B, Bat T, int mode) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= T.np) return;
+// pair i's bucket, or -1: left out (with its outputs for "no variant scored"
+// here), or put on the long pairs' list
+__device__ __forceinline__ int rlist_bucket(const Blk& B, const Bat& T, int i, int mode) {
     int n = refine_span(B, T, mode, i);
     if (n >= T.rl_min && T.rl_long) {          // many warps for this pair
         int slot = atomicAdd(T.rl_count, 1);
-        if (slot < T.rl_nlmax) { T.rl_long[slot] = i; return; }
+        if (slot < T.rl_nlmax) { T.rl_long[slot] = i; return -1; }
     }
-    if (n > 0) {
-        atomicAdd(&T.rhist[RL_NB - 1 - (n >> RL_SHIFT)], 1);
-        return;
-    }
+    if (n > 0) return RL_NB - 1 - (n >> RL_SHIFT);
     // no variant: MpStage1.cpp:700-716 with nothing scored
     bool skipped = n < 0;
     if (mode == RM_INIT || mode == RM_DP || (!skipped && (mode == RM_FIN1 || mode == RM_FIN2)))
         T.best[i] = 0.f;
     if (!skipped && mode == RM_FIN1) { T.sfndx[i] = T.sfndx_cur[i]; T.sfpos[i] = T.sfpos_cur[i]; }
+    return -1;
+}
+
+__global__ void k_rlist_count(Blk B, Bat T, int mode) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= T.np) return;
+    int b = rlist_bucket(B, T, i, mode);
+    if (b >= 0) atomicAdd(&T.rhist[b], 1);
 }
 
 // exclusive scan of the bucket counts (one CTA of 1024 threads)
@@ -990,6 +998,59 @@ __global__ void k_rlist_fill(Blk B, Bat T, int mode) {
     int n = refine_span(B, T, mode, i);
     if (n >= T.rl_min && T.rl_long) return;      // listed by k_rlist_count
     if (n > 0) T.rlist[atomicAdd(&T.rhist[RL_NB - 1 - (n >> RL_SHIFT)], 1)] = i;
+}
+
+// The work list of a batch of at most LIST_SMALL pairs by one CTA, buckets in
+// shared memory, in place of a memset and three launches (KIND: LK_*; arg: the
+// refinement mode, the DP's skip mode or the flag mask).
+enum ListKind { LK_REFINE = 0, LK_DP = 1, LK_PAIRS = 2 };
+template <int KIND>
+__global__ void __launch_bounds__(1024) k_list_small(Blk B, Bat T, int arg) {
+    __shared__ int hist[RL_NB], part[1024];
+    constexpr int PER = RL_NB / 1024, IPT = LIST_SMALL / 1024;
+    const int t = threadIdx.x;
+#pragma unroll
+    for (int j = 0; j < PER; j++) hist[t * PER + j] = 0;
+    if (KIND == LK_REFINE && T.rl_long) {
+        if (t == 0) *T.rl_count = 0;
+        for (int k = t; k < T.rl_nlmax; k += 1024) T.rl_next[k] = 0;
+    }
+    __syncthreads();
+    int b[IPT];
+#pragma unroll
+    for (int j = 0; j < IPT; j++) {
+        const int i = t + 1024 * j;
+        b[j] = -1;
+        if (i < T.np) {
+            b[j] = KIND == LK_REFINE ? rlist_bucket(B, T, i, arg)
+                 : KIND == LK_DP ? dlist_bucket(B, T, i, arg) : plist_bucket(B, T, i, arg);
+            if (b[j] >= 0) atomicAdd(&hist[b[j]], 1);
+        }
+    }
+    __syncthreads();
+    int loc[PER], s = 0;
+#pragma unroll
+    for (int j = 0; j < PER; j++) { loc[j] = hist[t * PER + j]; s += loc[j]; }
+    part[t] = s;
+    __syncthreads();
+    for (int o = 1; o < 1024; o <<= 1) {
+        const int v = t >= o ? part[t - o] : 0;
+        __syncthreads();
+        part[t] += v;
+        __syncthreads();
+    }
+    int run = part[t] - s;
+#pragma unroll
+    for (int j = 0; j < PER; j++) { hist[t * PER + j] = run; run += loc[j]; }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < IPT; j++)
+        if (b[j] >= 0) T.rlist[atomicAdd(&hist[b[j]], 1)] = t + 1024 * j;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < PER; j++) T.rhist[t * PER + j] = hist[t * PER + j];
+    if (t == 0) T.rhist[RL_NB] = part[1023];
+    if (t < RL_NHIST - RL_NB - 1) T.rhist[RL_NB + 1 + t] = 0;
 }
 
 // Variant list of one pair, enumerated compactly (admissible variants only).
@@ -2227,16 +2288,21 @@ void launch_refine(int mode, const Blk& B, const Bat& T0, cudaStream_t st, bool 
     Bat T = T0;
     T.rl_min = RL_LONG;
     T.rlw_ctas = T0.rlw_ctas > 0 && T0.rlw_ctas <= RLW_CTAS_MAX ? T0.rlw_ctas : RLW_CTAS;
-    cudaMemsetAsync(T.rhist, 0, RL_NHIST * sizeof(int), st);
-    if (T.rl_long) {
-        cudaMemsetAsync(T.rl_count, 0, sizeof(int), st);
-        cudaMemsetAsync(T.rl_next, 0, (size_t)T.rl_nlmax * sizeof(int), st);
+    if (T.np <= LIST_SMALL) {
+        k_list_small<LK_REFINE><<<1, 1024, 0, st>>>(B, T, mode);
+        GTB_LAUNCHED(T);
+    } else {
+        cudaMemsetAsync(T.rhist, 0, RL_NHIST * sizeof(int), st);
+        if (T.rl_long) {
+            cudaMemsetAsync(T.rl_count, 0, sizeof(int), st);
+            cudaMemsetAsync(T.rl_next, 0, (size_t)T.rl_nlmax * sizeof(int), st);
+        }
+        const int nb = (T.np + 255) / 256;
+        k_rlist_count<<<nb, 256, 0, st>>>(B, T, mode);
+        k_rlist_scan<<<1, 1024, 0, st>>>(T);
+        k_rlist_fill<<<nb, 256, 0, st>>>(B, T, mode);
+        if (T.launches) (*T.launches) += 3;
     }
-    const int nb = (T.np + 255) / 256;
-    k_rlist_count<<<nb, 256, 0, st>>>(B, T, mode);
-    k_rlist_scan<<<1, 1024, 0, st>>>(T);
-    k_rlist_fill<<<nb, 256, 0, st>>>(B, T, mode);
-    if (T.launches) (*T.launches) += 3;
     // The longer pairs' launches on the second stream, beside the shorter
     // ones' (all read the lists built above; they write disjoint pairs)
     const bool fork = T.st2 && (T.rl_long || T.nml[2] > 0);
@@ -2778,7 +2844,10 @@ static void launch_dp_wave(const Blk& B, const Bat& T, int tfmsrc, float gcost, 
 
 void launch_dp(const Blk& B, const Bat& T, int tfmsrc, int gap0, float gcost, int usess,
                int dpscan, int skipmode, cudaStream_t st) {
-    {
+    if (T.np <= LIST_SMALL) {
+        k_list_small<LK_DP><<<1, 1024, 0, st>>>(B, T, skipmode);
+        GTB_LAUNCHED(T);
+    } else {
         cudaMemsetAsync(T.rhist, 0, RL_NHIST * sizeof(int), st);
         const int nb = (T.np + 255) / 256;
         k_dlist_count<<<nb, 256, 0, st>>>(B, T, skipmode);
@@ -2807,6 +2876,11 @@ void launch_dp(const Blk& B, const Bat& T, int tfmsrc, int gap0, float gcost, in
 }
 
 void launch_pair_list(const Blk& B, const Bat& T, int skipmask, cudaStream_t st) {
+    if (T.np <= LIST_SMALL) {
+        k_list_small<LK_PAIRS><<<1, 1024, 0, st>>>(B, T, skipmask);
+        GTB_LAUNCHED(T);
+        return;
+    }
     cudaMemsetAsync(T.rhist, 0, RL_NHIST * sizeof(int), st);
     const int nb = (T.np + 255) / 256;
     k_plist_count<<<nb, 256, 0, st>>>(B, T, skipmask);
