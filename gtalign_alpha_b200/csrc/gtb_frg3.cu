@@ -762,15 +762,13 @@ void launch_frg3(const Blk& B, const Bat& T, cudaStream_t st) {
     for (int rci = 0; rci < B.f3nsec * nbr; rci++) {
         Bat TA = T;
         TA.alt_rci = rci;
-        launch_dp(B, TA, DP_TFM_ALT, 1, 0.0f, 0, 0, 0, st);
-        launch_btck(B, TA, 0, st);
+        launch_dp(B, TA, DP_TFM_ALT, 1, 0.0f, 0, 0, 0, 0, st);
         launch_refine(RM_DP, B, T, st, true);
         plist();
         k_f3_second<<<(T.np + 255) / 256, 256, 0, st>>>(B, T, rci);
         if (T.launches) (*T.launches)++;
         if (B.depth <= 1) {
-            launch_dp(B, T, DP_TFM_IBEST, 1, 0.0f, 0, 0, 0, st);
-            launch_btck(B, T, 0, st);
+            launch_dp(B, T, DP_TFM_IBEST, 1, 0.0f, 0, 0, 0, 0, st);
             launch_refine(RM_DP, B, T, st, true);
             plist();
             k_f3_second<<<(T.np + 255) / 256, 256, 0, st>>>(B, T, rci);

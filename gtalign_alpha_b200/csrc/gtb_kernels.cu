@@ -944,11 +944,14 @@ __global__ void __launch_bounds__(1024) k_rlist_scan(Bat T) {
     if (t == 1023) T.rhist[RL_NB] = part[1023];
 }
 
+// skipmode & DL_KEEPALN: the pairs left out keep their aligned pairs (before a
+// constrained traceback); else they have none
+constexpr int DL_KEEPALN = 2;
 // DP work list: the pairs a DP launch works on (flags clear, not on the
 // wavefront path), largest matrices first; kept in the same buffers as the
 // refinement list (a DP launch is over before the next list is built).
 __device__ __forceinline__ int dlist_bucket(const Blk& B, const Bat& T, int i, int skipmode) {
-    int skipmask = skipmode == 0 ? (CONV_LOWTMSC | CONV_SCOREDP) : CONV_LOWTMSC;
+    int skipmask = (skipmode & 1) == 0 ? (CONV_LOWTMSC | CONV_SCOREDP) : CONV_LOWTMSC;
     if (T.flags[i] & skipmask) return -1;
     if (T.dw_mark && T.dw_mark[i]) return -1;
     if (alt_empty(T, i)) return -1;
@@ -963,6 +966,7 @@ __global__ void k_dlist_count(Blk B, Bat T, int skipmode) {
     if (i >= T.np) return;
     int b = dlist_bucket(B, T, i, skipmode);
     if (b >= 0) atomicAdd(&T.rhist[b], 1);
+    else if (!(skipmode & DL_KEEPALN)) T.naln[i] = 0;
 }
 
 __global__ void k_dlist_fill(Blk B, Bat T, int skipmode) {
@@ -1025,6 +1029,7 @@ __global__ void __launch_bounds__(1024) k_list_small(Blk B, Bat T, int arg) {
             b[j] = KIND == LK_REFINE ? rlist_bucket(B, T, i, arg)
                  : KIND == LK_DP ? dlist_bucket(B, T, i, arg) : plist_bucket(B, T, i, arg);
             if (b[j] >= 0) atomicAdd(&hist[b[j]], 1);
+            else if (KIND == LK_DP && !(arg & DL_KEEPALN)) T.naln[i] = 0;
         }
     }
     __syncthreads();
@@ -2674,6 +2679,108 @@ __device__ __forceinline__ bool dp_pair_fast(const float* t, float d02, float gc
     return true;
 }
 
+// traceback: MpDPHub.cpp:1515-1660 (plain) and 1699-1905 (constrained)
+//
+// A warp per pair.  The walk is one chain of dependent steps, the same on every
+// lane; a thread per pair paid a load from L2 for most of them (580 cycles a
+// step: 0.73 ms for a pair of 1,200 residues).  The warp that ran the pair's DP
+// (the first of its CTA's) makes the walk right after it, beside other pairs' DPs.
+// The 32 words of a (strip,
+// step group), one 128-byte line, come in for BT_WIN groups at a time into
+// shared memory, and the lines the path enters next (the groups below, and the
+// previous strip's around the path's column) are on their way to L1.  32
+// aligned pairs at a time are written out, a pair per lane.
+constexpr int BT_WIN = 16;        // groups of a window
+constexpr int BT_WARPS = 4;
+__device__ __forceinline__ void bt_prefetch(const unsigned* p) {
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+}
+
+template <int R>
+__device__ __forceinline__ int btck_walk(const unsigned* bt, int lq, int lr, const float4* q4,
+                                         const float4* r4, bool constrained, const float* t,
+                                         float d82, unsigned* aln, float* alc, unsigned* win,
+                                         int lane) {
+    const unsigned FULL = 0xffffffffu;
+    constexpr int ROWS = 32 * R, SPW = 16 / R;
+    const long long sw = bt_strip_words(lr, R);
+    int y = lq - 1, x = lr - 1, n = 0, pend = 0;
+    unsigned mine = 0;                        // this lane's aligned pair among the last 32
+    auto flush = [&](int cnt) {
+        float4 cq = make_float4(0.f, 0.f, 0.f, 0.f), cr = cq;
+        bool keep = lane < cnt;
+        if (keep) {
+            cq = __ldg(q4 + (mine >> 16));
+            cr = __ldg(r4 + (mine & 0xffffu));
+            if (constrained) keep = dist2_tf(t, cq.x, cq.y, cq.z, cr.x, cr.y, cr.z) <= d82;
+        }
+        const unsigned m = __ballot_sync(FULL, keep);
+        if (keep) {
+            const int k = n + __popc(m & ((1u << lane) - 1u));
+            aln[k] = mine;
+            float2* c2 = (float2*)(alc + 6 * (long long)k);
+            c2[0] = make_float2(cq.x, cq.y); c2[1] = make_float2(cq.z, cr.x); c2[2] = make_float2(cr.y, cr.z);
+        }
+        n += __popc(m);
+    };
+    int cs = -1, wlo = 0;                     // the window's strip and lowest group
+    while ((x | y) >= 0) {
+        const int s = y / ROWS, l = y % ROWS / R, tt = x + l, g = tt / SPW;
+        if (s != cs || g < wlo) {
+            cs = s;
+            wlo = g - BT_WIN + 1 > 0 ? g - BT_WIN + 1 : 0;
+            const unsigned* line = bt + s * sw;
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < BT_WIN; k++)
+                if (g - k >= 0) win[((g - k) & (BT_WIN - 1)) * 32 + lane] = line[(g - k) * 32 + lane];
+            if (lane < BT_WIN) {
+                if (wlo - 1 - lane >= 0) bt_prefetch(line + (wlo - 1 - lane) * 32);
+            } else if (s > 0) {
+                const int gp = (x + 31) / SPW - (lane - BT_WIN);
+                if (gp >= 0) bt_prefetch(line - sw + gp * 32);
+            }
+            __syncwarp();
+        }
+        // the path through one word: R rows x SPW steps
+        const unsigned w = win[(g & (BT_WIN - 1)) * 32 + l];
+        int rr = y % R, uu = tt % SPW;
+        do {
+            const unsigned b = (w >> (2 * R * uu + 2 * rr)) & 3u;
+            if (b == BTW_DIAG) {
+                if (lane == pend) mine = ((unsigned)y << 16) | (unsigned)x;
+                if (++pend == 32) { flush(32); pend = 0; }
+            }
+            const int dy = b != BTW_LEFT, dx = b < BTW_UP;    // up is 2 or 3, left 1, diagonal 0
+            y -= dy; rr -= dy;
+            x -= dx; uu -= dx;
+        } while ((rr | uu | x) >= 0);
+    }
+    if (pend > 0) flush(pend);
+    return n;
+}
+
+// the traceback of pair i by a warp: its aligned pairs and their number
+__device__ __forceinline__ void btck_pair(const Blk& B, const Bat& T, int i, int flags, int lq, int lr,
+                                          const float4* q4, const float4* r4, int constrained,
+                                          unsigned* win, int lane) {
+    if (!constrained && (flags & CONV_SCOREDP)) {
+        if (lane == 0) T.naln[i] = 0;
+        return;
+    }
+    const unsigned* bt = T.bt + T.off_bt[i];
+    unsigned* aln = T.aln + T.off_aln[i];
+    float* alc = T.alc + 6 * T.off_aln[i];
+    const float d82 = B.t_d82[lq < lr ? lq : lr];
+    float t[12];
+#pragma unroll
+    for (int f = 0; f < 12; f++) t[f] = constrained ? T.tfm_gr[i * 12 + f] : 0.f;
+    const int n = dp_r(lq) == 4
+        ? btck_walk<4>(bt, lq, lr, q4, r4, constrained != 0, t, d82, aln, alc, win, lane)
+        : btck_walk<2>(bt, lq, lr, q4, r4, constrained != 0, t, d82, aln, alc, win, lane);
+    if (lane == 0) T.naln[i] = n;
+}
+
 // The DP work list (k_dlist_*, largest matrices first): its first dp_kc
 // pairs take a CTA each, whose 4 warps run the pair's strips as a wavefront
 // (strip s on warp s mod 4, each strip waiting with a bounded spin until the
@@ -2681,9 +2788,10 @@ __device__ __forceinline__ bool dp_pair_fast(const float* t, float d02, float gc
 // shared memory); the other pairs take a warp each.
 template <int GAP0, int SC>
 __global__ void __launch_bounds__(128) k_dp(Blk B, Bat T, int tfmsrc, float gcost, int dpscan,
-                                            int skipmode) {
+                                            int constrained) {
     __shared__ int s_prog[DP_CTA_MAXSTRIPS];
     __shared__ DpRing s_ring[4];
+    __shared__ unsigned s_win[4][BT_WIN * 32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int len = T.rhist[RL_NB];
     const int dkc = T.dw_err ? T.dp_kc : 0;
@@ -2729,9 +2837,7 @@ __global__ void __launch_bounds__(128) k_dp(Blk B, Bat T, int tfmsrc, float gcos
                     dp_pair_fast<2, GAP0 != 0, SC, true, false>(t, d02, gcost, lq, lr, q4, r4, qs, rs, row, bt,
                                                                 s_ring[w], lane, w, blockDim.x >> 5, s_prog,
                                                                 T.dw_err, T.dw_spin, nullptr, true);
-                return;
-            }
-            if (dp_r(lq) == 4)
+            } else if (dp_r(lq) == 4)
                 dp_pair<4, GAP0 != 0, SC, true>(t, d02, gcost, lq, lr, qx, qy, qz, r4, qs, rs, qa, ra, row,
                                                 bt, lane, w, blockDim.x >> 5, s_prog, T.dw_err, T.dw_spin,
                                                 nullptr, true);
@@ -2739,6 +2845,8 @@ __global__ void __launch_bounds__(128) k_dp(Blk B, Bat T, int tfmsrc, float gcos
                 dp_pair<2, GAP0 != 0, SC, true>(t, d02, gcost, lq, lr, qx, qy, qz, r4, qs, rs, qa, ra, row,
                                                 bt, lane, w, blockDim.x >> 5, s_prog, T.dw_err, T.dw_spin,
                                                 nullptr, true);
+            __syncthreads();                       // every strip's words
+            if (w == 0) btck_pair(B, T, i, T.flags[i], lq, lr, q4, r4, constrained, s_win[w], lane);
             return;
         }
         if (w != 0) return;                        // one strip: one warp
@@ -2752,12 +2860,12 @@ __global__ void __launch_bounds__(128) k_dp(Blk B, Bat T, int tfmsrc, float gcos
         else
             dp_pair_fast<2, GAP0 != 0, SC, false, false>(t, d02, gcost, lq, lr, q4, r4, qs, rs, row, bt,
                                                          s_ring[w], lane);
-        return;
-    }
-    if (dp_r(lq) == 4)
+    } else if (dp_r(lq) == 4)
         dp_pair<4, GAP0 != 0, SC, false>(t, d02, gcost, lq, lr, qx, qy, qz, r4, qs, rs, qa, ra, row, bt, lane);
     else
         dp_pair<2, GAP0 != 0, SC, false>(t, d02, gcost, lq, lr, qx, qy, qz, r4, qs, rs, qa, ra, row, bt, lane);
+    __syncwarp();
+    btck_pair(B, T, i, T.flags[i], lq, lr, q4, r4, constrained, s_win[w], lane);
 }
 
 // One warp per CTA; the CTAs of a long pair take its strips round robin.
@@ -2842,17 +2950,36 @@ static void launch_dp_wave(const Blk& B, const Bat& T, int tfmsrc, float gcost, 
     if (e != cudaSuccess && T.lerr && *T.lerr == cudaSuccess) *T.lerr = e;
 }
 
+// the pairs whose DP ran on several CTAs (dw_mark); the others' walks are in k_dp
+__global__ void __launch_bounds__(BT_WARPS * 32) k_btck(Blk B, Bat T, int constrained) {
+    __shared__ unsigned s_win[BT_WARPS][BT_WIN * 32];
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const int i = blockIdx.x * BT_WARPS + wp;
+    if (i >= T.np || !T.dw_mark[i]) return;
+    const int flags = T.flags[i];
+    if (constrained) {
+        if (flags & CONV_LOWTMSC) return;
+    } else if ((flags & CONV_LOWTMSC) || alt_empty(T, i)) {
+        if (lane == 0) T.naln[i] = 0;
+        return;
+    }
+    const int qi = pair_qi(B, T, i), ri = pair_ri(B, T, i);
+    btck_pair(B, T, i, flags, B.qlen[qi], B.rlen[ri], B.q4 + B.q4off[qi], B.r4 + B.r4off[ri], constrained,
+              s_win[wp], lane);
+}
+
 void launch_dp(const Blk& B, const Bat& T, int tfmsrc, int gap0, float gcost, int usess,
-               int dpscan, int skipmode, cudaStream_t st) {
+               int dpscan, int skipmode, int constrained, cudaStream_t st) {
+    const int lmode = skipmode | (constrained ? DL_KEEPALN : 0);
     if (T.np <= LIST_SMALL) {
-        k_list_small<LK_DP><<<1, 1024, 0, st>>>(B, T, skipmode);
+        k_list_small<LK_DP><<<1, 1024, 0, st>>>(B, T, lmode);
         GTB_LAUNCHED(T);
     } else {
         cudaMemsetAsync(T.rhist, 0, RL_NHIST * sizeof(int), st);
         const int nb = (T.np + 255) / 256;
-        k_dlist_count<<<nb, 256, 0, st>>>(B, T, skipmode);
+        k_dlist_count<<<nb, 256, 0, st>>>(B, T, lmode);
         k_rlist_scan<<<1, 1024, 0, st>>>(T);
-        k_dlist_fill<<<nb, 256, 0, st>>>(B, T, skipmode);
+        k_dlist_fill<<<nb, 256, 0, st>>>(B, T, lmode);
         if (T.launches) (*T.launches) += 3;
     }
     KtScope kts(T, KF_DP, st);
@@ -2867,12 +2994,16 @@ void launch_dp(const Blk& B, const Bat& T, int tfmsrc, int gap0, float gcost, in
     }
     // dp_kc CTAs for the largest listed pairs, then a warp per pair
     const int nb = (T.dw_err ? T.dp_kc : 0) + (T.np + 3) / 4;
-    if (usess == DP_SC_SSRR) k_dp<0, DP_SC_SSRR><<<nb, 128, 0, st>>>(B, T, tfmsrc, gcost, dpscan, skipmode);
-    else if (gap0 && !usess) k_dp<1, DP_SC_TFM><<<nb, 128, 0, st>>>(B, T, tfmsrc, gcost, dpscan, skipmode);
-    else if (!gap0 && !usess) k_dp<0, DP_SC_TFM><<<nb, 128, 0, st>>>(B, T, tfmsrc, gcost, dpscan, skipmode);
-    else if (!gap0 && usess) k_dp<0, DP_SC_TFMSS><<<nb, 128, 0, st>>>(B, T, tfmsrc, gcost, dpscan, skipmode);
-    else k_dp<1, DP_SC_TFMSS><<<nb, 128, 0, st>>>(B, T, tfmsrc, gcost, dpscan, skipmode);
+    if (usess == DP_SC_SSRR) k_dp<0, DP_SC_SSRR><<<nb, 128, 0, st>>>(B, T, tfmsrc, gcost, dpscan, constrained);
+    else if (gap0 && !usess) k_dp<1, DP_SC_TFM><<<nb, 128, 0, st>>>(B, T, tfmsrc, gcost, dpscan, constrained);
+    else if (!gap0 && !usess) k_dp<0, DP_SC_TFM><<<nb, 128, 0, st>>>(B, T, tfmsrc, gcost, dpscan, constrained);
+    else if (!gap0 && usess) k_dp<0, DP_SC_TFMSS><<<nb, 128, 0, st>>>(B, T, tfmsrc, gcost, dpscan, constrained);
+    else k_dp<1, DP_SC_TFMSS><<<nb, 128, 0, st>>>(B, T, tfmsrc, gcost, dpscan, constrained);
     GTB_LAUNCHED(T);
+    if (T.ndw > 0) {
+        k_btck<<<(T.np + BT_WARPS - 1) / BT_WARPS, BT_WARPS * 32, 0, st>>>(B, T, constrained);
+        GTB_LAUNCHED(T);
+    }
 }
 
 void launch_pair_list(const Blk& B, const Bat& T, int skipmask, cudaStream_t st) {
@@ -2961,121 +3092,6 @@ void launch_f3_dpscore(const Blk& B, const Bat& T, cudaStream_t st) {
 }
 
 // ---------------------------------------------------------------------------
-// traceback: MpDPHub.cpp:1515-1660 (plain) and 1699-1905 (constrained)
-//
-// A warp per pair.  The walk is one chain of dependent steps, the same on every
-// lane; a thread per pair paid a load from L2 for most of them (580 cycles a
-// step: 0.73 ms for a pair of 1,200 residues).  Here the 32 words of a (strip,
-// step group), one 128-byte line, come in for BT_WIN groups at a time into
-// shared memory, and the lines the path enters next (the groups below, and the
-// previous strip's around the path's column) are on their way to L1.  32
-// aligned pairs at a time are written out, a pair per lane.
-constexpr int BT_WIN = 16;        // groups of a window
-constexpr int BT_WARPS = 4;
-__device__ __forceinline__ void bt_prefetch(const unsigned* p) {
-    asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
-}
-
-template <int R>
-__device__ __forceinline__ int btck_walk(const unsigned* bt, int lq, int lr, const float4* q4,
-                                         const float4* r4, bool constrained, const float* t,
-                                         float d82, unsigned* aln, float* alc, unsigned* win,
-                                         int lane) {
-    const unsigned FULL = 0xffffffffu;
-    constexpr int ROWS = 32 * R, SPW = 16 / R;
-    const long long sw = bt_strip_words(lr, R);
-    int y = lq - 1, x = lr - 1, n = 0, pend = 0;
-    unsigned mine = 0;                        // this lane's aligned pair among the last 32
-    auto flush = [&](int cnt) {
-        float4 cq = make_float4(0.f, 0.f, 0.f, 0.f), cr = cq;
-        bool keep = lane < cnt;
-        if (keep) {
-            cq = __ldg(q4 + (mine >> 16));
-            cr = __ldg(r4 + (mine & 0xffffu));
-            if (constrained) keep = dist2_tf(t, cq.x, cq.y, cq.z, cr.x, cr.y, cr.z) <= d82;
-        }
-        const unsigned m = __ballot_sync(FULL, keep);
-        if (keep) {
-            const int k = n + __popc(m & ((1u << lane) - 1u));
-            aln[k] = mine;
-            float2* c2 = (float2*)(alc + 6 * (long long)k);
-            c2[0] = make_float2(cq.x, cq.y); c2[1] = make_float2(cq.z, cr.x); c2[2] = make_float2(cr.y, cr.z);
-        }
-        n += __popc(m);
-    };
-    int cs = -1, wlo = 0, cg = -1, cl = -1;   // the window's strip and lowest group; the word in w
-    unsigned w = 0;
-    while (x >= 0 && y >= 0) {
-        const int s = y / ROWS, yy = y % ROWS, l = yy / R, tt = x + l, g = tt / SPW;
-        if (s != cs || g < wlo) {
-            cs = s;
-            wlo = g - BT_WIN + 1 > 0 ? g - BT_WIN + 1 : 0;
-            const unsigned* line = bt + s * sw;
-            __syncwarp();
-#pragma unroll
-            for (int k = 0; k < BT_WIN; k++)
-                if (g - k >= 0) win[((g - k) & (BT_WIN - 1)) * 32 + lane] = line[(g - k) * 32 + lane];
-            if (lane < BT_WIN) {
-                if (wlo - 1 - lane >= 0) bt_prefetch(line + (wlo - 1 - lane) * 32);
-            } else if (s > 0) {
-                const int gp = (x + 31) / SPW - (lane - BT_WIN);
-                if (gp >= 0) bt_prefetch(line - sw + gp * 32);
-            }
-            __syncwarp();
-            cg = -1;
-        }
-        if (g != cg || l != cl) {
-            w = win[(g & (BT_WIN - 1)) * 32 + l];
-            cg = g; cl = l;
-        }
-        const unsigned b = (w >> (2 * R * (tt % SPW) + 2 * (yy % R))) & 3u;
-        if (b == BTW_DIAG) {
-            if (lane == pend) mine = ((unsigned)y << 16) | (unsigned)x;
-            if (++pend == 32) { flush(32); pend = 0; }
-        }
-        // down is 2 or 3, left 1, diagonal 0
-        y -= b != BTW_LEFT;
-        x -= b < BTW_UP;
-    }
-    if (pend > 0) flush(pend);
-    return n;
-}
-
-__global__ void __launch_bounds__(BT_WARPS * 32) k_btck(Blk B, Bat T, int constrained) {
-    __shared__ unsigned s_win[BT_WARPS][BT_WIN * 32];
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-    const int i = blockIdx.x * BT_WARPS + wp;
-    if (i >= T.np) return;
-    int flags = T.flags[i];
-    if (constrained) {
-        if (flags & CONV_LOWTMSC) return;
-    } else if ((flags & (CONV_LOWTMSC | CONV_SCOREDP)) || alt_empty(T, i)) {
-        if (lane == 0) T.naln[i] = 0;
-        return;
-    }
-    int qi = pair_qi(B, T, i), ri = pair_ri(B, T, i);
-    int lq = B.qlen[qi], lr = B.rlen[ri];
-    int ml = lq < lr ? lq : lr;
-    const unsigned* bt = T.bt + T.off_bt[i];
-    unsigned* aln = T.aln + T.off_aln[i];
-    float* alc = T.alc + 6 * T.off_aln[i];
-    float t[12];
-    float d82 = B.t_d82[ml];
-    const float4* q4 = B.q4 + B.q4off[qi];
-    const float4* r4 = B.r4 + B.r4off[ri];
-#pragma unroll
-    for (int f = 0; f < 12; f++) t[f] = constrained ? T.tfm_gr[i * 12 + f] : 0.f;
-    const int n = dp_r(lq) == 4
-        ? btck_walk<4>(bt, lq, lr, q4, r4, constrained != 0, t, d82, aln, alc, s_win[wp], lane)
-        : btck_walk<2>(bt, lq, lr, q4, r4, constrained != 0, t, d82, aln, alc, s_win[wp], lane);
-    if (lane == 0) T.naln[i] = n;
-}
-
-void launch_btck(const Blk& B, const Bat& T, int constrained, cudaStream_t st) {
-    k_btck<<<(T.np + BT_WARPS - 1) / BT_WARPS, BT_WARPS * 32, 0, st>>>(B, T, constrained);
-    GTB_LAUNCHED(T);
-}
-
 // ---------------------------------------------------------------------------
 // per-iteration bookkeeping of DPRefine: MpStage1.cpp:495-513 and
 // CheckScoreConvergence / SaveLastScore0 / SetLowScoreConvergenceFlag
@@ -3322,8 +3338,7 @@ void make_tables(float* d0, float* d82, float* d0fin, int n) {
 void launch_dprefine(const Blk& B, const Bat& T, int gap0, int prescreen, int maxit,
                      float prescore, bool few, int tfm1, cudaStream_t st) {
     for (int dpi = 0; dpi < maxit; dpi++) {
-        launch_dp(B, T, dpi == 0 ? tfm1 : DP_TFM_IBEST, gap0, gap0 ? 0.0f : -0.6f, 0, 0, 0, st);
-        launch_btck(B, T, 0, st);
+        launch_dp(B, T, dpi == 0 ? tfm1 : DP_TFM_IBEST, gap0, gap0 ? 0.0f : -0.6f, 0, 0, 0, 0, st);
         launch_refine(RM_DP, B, T, st, few);
         launch_post(B, T, dpi, maxit, prescreen, prescore, st);
     }
@@ -3355,8 +3370,7 @@ void launch_stages(const Blk& B, const Bat& T, int refinement, int depth, int co
         // --add-search-by-ss (custage_ssrr.cu:43-140, CuBatch.cu:583-600): the
         // alignment of the SS and residue-scored DP, fragment refinement over it,
         // DP refinement with the gap cost and without, 2 iterations each
-        launch_dp(B, T, DP_TFM_GRAND, 0, -1.0f, DP_SC_SSRR, 0, 1, st);
-        launch_btck(B, T, 0, st);
+        launch_dp(B, T, DP_TFM_GRAND, 0, -1.0f, DP_SC_SSRR, 0, 1, 0, st);
         launch_refine(RM_DP, B, T, st, few);
         dprefine(0, 0, 2, few);
         dprefine(1, 0, 2, few);
@@ -3366,8 +3380,7 @@ void launch_stages(const Blk& B, const Bat& T, int refinement, int depth, int co
     // two stage-2 passes: MpStage2.h:63-83, CuBatch.cu:627-650
     for (int call = 0; call < 2; call++) {
         int gap0 = call == 1;
-        launch_dp(B, T, DP_TFM_GRAND, gap0, gap0 ? 0.0f : -1.0f, !gap0, !gap0, 1, st);
-        launch_btck(B, T, 0, st);
+        launch_dp(B, T, DP_TFM_GRAND, gap0, gap0 ? 0.0f : -1.0f, !gap0, !gap0, 1, 0, st);
         launch_refine(RM_DP, B, T, st, few);
         dprefine(0, 0, 2, few);
         dprefine(1, 0, call == 0 ? 2 : convergence, few);
@@ -3375,12 +3388,10 @@ void launch_stages(const Blk& B, const Bat& T, int refinement, int depth, int co
     }
     mark(3);
     // final stage: MpStageFin.h:63-96
-    launch_dp(B, T, DP_TFM_GRAND, 1, 0.0f, 0, 0, 1, st);
-    launch_btck(B, T, 0, st);
+    launch_dp(B, T, DP_TFM_GRAND, 1, 0.0f, 0, 0, 1, 0, st);
     launch_refine(RM_FIN1, B, T, st, few);
     if (!(depth == 3 || refinement == GTB_REFINEMENT_COARSE)) launch_refine(RM_FIN2, B, T, st, few);
-    launch_dp(B, T, DP_TFM_GRAND, 1, 0.0f, 0, 0, 1, st);
-    launch_btck(B, T, 1, st);
+    launch_dp(B, T, DP_TFM_GRAND, 1, 0.0f, 0, 0, 1, 1, st);
     launch_alnstr(B, T, st);
     launch_refine(RM_PROD1, B, T, st, few);
     if (refinement == GTB_REFINEMENT_LOG) {

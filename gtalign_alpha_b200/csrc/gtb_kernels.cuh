@@ -270,10 +270,11 @@ __host__ __device__ inline void seed_range(int lq, int lr, int qmax, int qmin, i
 void launch_findfrag(const Blk& B, const Bat& T, cudaStream_t st);
 // few: most pairs of the batch are already filtered out (32 lanes per pair)
 void launch_refine(int mode, const Blk& B, const Bat& T, cudaStream_t st, bool few);
-// skipmode 0: skip LOWTMSC|SCOREDP (plain), 1: skip LOWTMSC only
+// DP and traceback.  skipmode 0: skip LOWTMSC|SCOREDP (plain), 1: skip LOWTMSC
+// only; constrained: the traceback keeps the pairs within d8 of the grand best
+// transform
 void launch_dp(const Blk& B, const Bat& T, int tfmsrc, int gap0, float gcost, int usess,
-               int dpscan, int skipmode, cudaStream_t st);
-void launch_btck(const Blk& B, const Bat& T, int constrained, cudaStream_t st);
+               int dpscan, int skipmode, int constrained, cudaStream_t st);
 // CTAs that the wavefront DP may keep resident at once on this device
 int dp_wave_capacity();
 // per-device kernel attributes (shared-memory carve-outs), once per device
