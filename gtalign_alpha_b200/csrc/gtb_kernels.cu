@@ -1265,104 +1265,6 @@ __device__ __forceinline__ float lane_pass(const PairGeom& G, int kind, int k0, 
               : lane_pass_t<false, false, false>(G, kind, k0, k1, tfm, d02, chk, d82, thr, m3on, v, m3out, pl);
 }
 
-// One pass of a variant that the 32 lanes of a warp share (the long pairs'
-// refinement when few pairs are long).  Lane L sums the positions of block
-// cb + L (blocks of BLK positions, the absolute blocks of lane_pass_t) in
-// position order, exactly as lane_pass_t sums a block; the block partials
-// then go through shared memory and lane f folds field f of every block in
-// block order (the same Neumaier folds, the same closing fold), so the sums,
-// the score and the three smallest distances equal lane_pass_t's bit for
-// bit.  Every lane returns the results.  sm: 32 x 17 floats of this warp.
-__device__ float wide_pass(const PairGeom& G, int kind, int k0, int k1, const float* tfm,
-                           float d02, int chk, float d82, float thr, int m3on, float* v,
-                           float& m3out, int lane, float* sm) {
-    const unsigned FULL = 0xffffffffu;
-    const bool frag = kind == PK_FRAG;
-    const bool scr = kind == PK_SCORE || kind == PK_GSCORE;
-    const bool cov = kind == PK_SCORE || kind == PK_EXT;
-    const bool trk = kind == PK_SCORE && m3on;
-    const int n = kind == PK_IDLE ? 0 : (frag ? k1 : G.n);
-    const int bfirst = frag ? (k0 & ~(BLK - 1)) / BLK : 0;
-    const int nblk = (n + BLK - 1) / BLK;
-    float fs = 0.f, fc = 0.f;                  // lane f < 16: field f's compensated total
-    float m1 = LARGEDST, m2 = LARGEDST, m3 = LARGEDST;
-    int cnt = 0;
-    for (int cb = bfirst; cb < nblk; cb += 32) {
-        const int b = cb + lane;
-        float part[16];
-#pragma unroll
-        for (int f = 0; f < 16; f++) part[f] = 0.f;
-        if (b < nblk) {
-            const int p0 = b * BLK, p1 = p0 + BLK < n ? p0 + BLK : n;
-            for (int k = p0; k < p1; k++) {
-                float qx, qy, qz, rx, ry, rz;
-                G.at(k, qx, qy, qz, rx, ry, rz);
-                float d = dist2_tf(tfm, qx, qy, qz, rx, ry, rz);
-                if (scr) part[15] = __fadd_rn(part[15], (!chk || d <= d82) ? tmterm(d02, d) : 0.f);
-                if (trk) {
-                    bool c1 = d < m1, c2 = d < m2, c3 = d < m3;
-                    m3 = c2 ? m2 : (c3 ? d : m3);
-                    m2 = c1 ? m1 : (c2 ? d : m2);
-                    m1 = c1 ? d : m1;
-                }
-                bool inc = frag ? (k0 <= k) : (cov && d <= thr);
-                const float ax = inc ? qx : 0.f, ay = inc ? qy : 0.f, az = inc ? qz : 0.f;
-                const float bx = inc ? rx : 0.f, by = inc ? ry : 0.f, bz = inc ? rz : 0.f;
-                part[0] = __fmaf_rn(ax, bx, part[0]); part[1] = __fmaf_rn(ax, by, part[1]);
-                part[2] = __fmaf_rn(ax, bz, part[2]); part[3] = __fmaf_rn(ay, bx, part[3]);
-                part[4] = __fmaf_rn(ay, by, part[4]); part[5] = __fmaf_rn(ay, bz, part[5]);
-                part[6] = __fmaf_rn(az, bx, part[6]); part[7] = __fmaf_rn(az, by, part[7]);
-                part[8] = __fmaf_rn(az, bz, part[8]);
-                part[9] = __fadd_rn(part[9], ax); part[10] = __fadd_rn(part[10], ay);
-                part[11] = __fadd_rn(part[11], az); part[12] = __fadd_rn(part[12], bx);
-                part[13] = __fadd_rn(part[13], by); part[14] = __fadd_rn(part[14], bz);
-                cnt += inc ? 1 : 0;
-            }
-        }
-        __syncwarp();
-#pragma unroll
-        for (int f = 0; f < 16; f++) sm[lane * 17 + f] = part[f];
-        __syncwarp();
-        if (lane < 16) {
-            const int nb = nblk - cb < 32 ? nblk - cb : 32;
-            for (int L = 0; L < nb; L++) {
-                float bb = sm[L * 17 + lane];
-                nfold(fs, fc, bb);
-            }
-        }
-    }
-    // the closing fold of lane_pass_t (score) and of CovAcc::final (sums)
-    if (lane < 16) {
-        float z = 0.f;
-        nfold(fs, fc, z);
-    }
-    const float tot = __fadd_rn(fs, fc);
-#pragma unroll
-    for (int f = 0; f < 15; f++) v[f] = __shfl_sync(FULL, tot, f);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(FULL, cnt, o);
-    v[15] = (float)cnt;
-    // the three smallest distances of the pass (a multiset: merging the
-    // lanes' three smallest gives the same three as one sweep)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float o1 = __shfl_xor_sync(FULL, m1, o), o2 = __shfl_xor_sync(FULL, m2, o),
-                    o3 = __shfl_xor_sync(FULL, m3, o);
-        const float x[3] = {o1, o2, o3};
-#pragma unroll
-        for (int e = 0; e < 3; e++) {
-            const float d = x[e];
-            bool c1 = d < m1, c2 = d < m2, c3 = d < m3;
-            m3 = c2 ? m2 : (c3 ? d : m3);
-            m2 = c1 ? m1 : (c2 ? d : m2);
-            m1 = c1 ? d : m1;
-        }
-    }
-    m3out = m3;
-    __syncwarp();
-    return __shfl_sync(FULL, tot, 15);
-}
-
 // The pair's result of a refinement launch (MpStage1.cpp:700-716 and the
 // final/production copies): winner score, transform and fragment, or the
 // "nothing scored" outputs.  tb: the winner's transform, stride tstr.
@@ -1421,13 +1323,9 @@ constexpr int RF_WARPS_LONG = RLW_CTA_WARPS;
 // pair's winner among them.
 // One slot of a refinement launch: a short pair (slot of the length-sorted
 // list) or, LONG, warp `wlong` of the warps working on long pair `slot`.
-// WIDE (long pairs only): a warp works on one variant at a time, its lanes
-// sharing the passes (wide_pass); otherwise every lane has a variant.
-template <int MODE, int RF_LPP, bool LONG, bool WIDE = false>
+template <int MODE, int RF_LPP, bool LONG>
 __device__ __forceinline__ void refine_slot(const Blk& B, const Bat& T, int slot, int wlong, int slot_end = 0) {
     constexpr int RF_WARPS = LONG ? RF_WARPS_LONG : RF_WARPS_SHORT;
-    static_assert(!WIDE || (LONG && RF_LPP == 32), "a wide pass is a long pair's warp");
-    __shared__ float s_wide[WIDE ? 17 * RF_WARPS * 32 : 1];   // block partials of wide passes
     __shared__ float s_last[16 * RF_WARPS * 32];   // previous iteration's sums
     __shared__ float s_tb[12 * RF_WARPS * 32];     // best transform of the current variant
     __shared__ float s_tbest[12 * RF_WARPS * 32];  // best transform over the lane's variants
@@ -1528,25 +1426,7 @@ __device__ __forceinline__ void refine_slot(const Blk& B, const Bat& T, int slot
     unsigned long long vis = 0;                   // position visits of this lane's passes
     for (;;) {
         const unsigned nm = __ballot_sync(FULL, need) & smask;
-        if (WIDE && nm) {                         // one variant for the whole warp
-            int base = 0;
-            if (lane == 0) base = atomicAdd(T.rl_next + slot, 1);
-            const int kv = __shfl_sync(FULL, base, 0);
-            need = false;
-            kind = PK_IDLE;
-            if (kv < V.total) {
-                int fl, kf;
-                variants_get(V, vk, n, kv, si, vndx, vpos, fl, kf);
-                if (MODE == RM_DP && T.vskip && si < 32 * F3_NSEC &&
-                    ((T.vskip[(long long)i * F3_NSEC + (si >> 5)] >> (si & 31)) & 1u)) {
-                    need = true;
-                } else {
-                    kind = PK_FRAG; k0 = kf; k1 = kf + fl;
-                    best = best_init; cit = 0;
-                }
-            }
-            if (need) continue;                   // a skipped variant: the next one
-        } else if (nm) {
+        if (nm) {
             if (LONG) {                           // the pair's counter, shared by its warps
                 int base = 0;
                 if (lane == 0) base = atomicAdd(T.rl_next + slot, __popc(nm));
@@ -1576,12 +1456,8 @@ __device__ __forceinline__ void refine_slot(const Blk& B, const Bat& T, int slot
             break;
         }
         float v[16], m3;
-        const float sc = WIDE ? wide_pass(G, kind, k0, k1, tfm, pd02, pchk, d82, thr, m3mode, v, m3,
-                                          lane, s_wide + (threadIdx.x >> 5) * 32 * 17)
-                              : lane_pass(G, kind, k0, k1, tfm, pd02, pchk, d82, thr, m3mode, v, m3,
-                                          lane % RF_LPP);
-        if (!WIDE || lane == 0)
-            vis += kind == PK_IDLE ? 0u : (kind == PK_FRAG ? (unsigned)(k1 - k0) : (unsigned)n);
+        const float sc = lane_pass(G, kind, k0, k1, tfm, pd02, pchk, d82, thr, m3mode, v, m3, lane % RF_LPP);
+        vis += kind == PK_IDLE ? 0u : (kind == PK_FRAG ? (unsigned)(k1 - k0) : (unsigned)n);
         bool havev = false, done = false;
         if (kind == PK_FRAG) {
             if (v[15] < 1.0f) done = true;
@@ -1689,14 +1565,14 @@ __device__ __forceinline__ void rlist_range(const Bat& T, int lo, int hi, int& f
 // LONG: T.rlw_ctas CTAs per long pair; the grid (a multiple of that) walks
 // the long pairs listed for this launch.
 // Otherwise: the pairs of the work list with lo <= n < hi positions.
-template <int MODE, int RF_LPP, bool LONG, bool WIDE = false>
+template <int MODE, int RF_LPP, bool LONG>
 __global__ void __launch_bounds__((LONG ? RF_WARPS_LONG : RF_WARPS_SHORT) * 32) k_refine(Blk B, Bat T, int lo, int hi) {
     if (LONG) {
         const int c = T.rlw_ctas;
         const int wl = (int)(blockIdx.x % c) * RF_WARPS_LONG + (threadIdx.x >> 5);
         const int nlong = *T.rl_count;
         for (int slot = (int)(blockIdx.x / c); slot < nlong; slot += (int)(gridDim.x / c))
-            refine_slot<MODE, RF_LPP, LONG, WIDE>(B, T, slot, wl);
+            refine_slot<MODE, RF_LPP, LONG>(B, T, slot, wl);
     } else {
         constexpr int RF_PPW = 32 / RF_LPP;        // pairs per warp
         int first, last;
@@ -1881,8 +1757,10 @@ __device__ __forceinline__ void coop_pass(CoopWarp& w, int m, int n, const float
 }
 
 // The whole alignment's FP32 RMSD (production phase 1, MpStageFin.cpp): the
-// 15 covariance sums, then the 6 sums of squares, by a warp.
-__device__ float coop_rmsd(CoopWarp& w, int n, const float4* cA, const float2* cB, int lane) {
+// 15 covariance sums, then the 6 sums of squares, by a warp; at(p, q): position
+// p's six coordinates; buf: a block's components, the eighth all ones.
+template <class At>
+__device__ __forceinline__ float rmsd_warp(float* buf, int n, At at, int lane) {
     double dv[21];
     for (int part = 0; part < 2; part++) {
         float s = 0.f, c = 0.f;
@@ -1891,16 +1769,15 @@ __device__ float coop_rmsd(CoopWarp& w, int n, const float4* cA, const float2* c
         const int ay = part ? ax : (f < 9 ? 3 + f % 3 : 7);
         for (int b0 = 0; b0 * BLK < n; b0++) {
             const int p = b0 * BLK + lane;
-            float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
-            float2 v = make_float2(0.f, 0.f);
-            if (p < n) { u = cA[p]; v = cB[p]; }
-            float* o = w.buf + lane;
-            o[0] = u.x; o[CM_BST] = u.y; o[2 * CM_BST] = u.z;
-            o[3 * CM_BST] = u.w; o[4 * CM_BST] = v.x; o[5 * CM_BST] = v.y;
-            o[6 * CM_BST] = 0.f;
+            float q[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            if (p < n) at(p, q);
+#pragma unroll
+            for (int k = 0; k < 6; k++) buf[k * CM_BST + lane] = q[k];
+            buf[6 * CM_BST + lane] = 0.f;
             __syncwarp();
             float b = 0.f;
-            for (int k = 0; k < BLK; k++) b = __fmaf_rn(w.buf[ax * CM_BST + k], w.buf[ay * CM_BST + k], b);
+#pragma unroll 8
+            for (int k = 0; k < BLK; k++) b = __fmaf_rn(buf[ax * CM_BST + k], buf[ay * CM_BST + k], b);
             __syncwarp();
             tfold(s, c, b);
         }
@@ -1989,7 +1866,11 @@ __global__ void __launch_bounds__(CM_WARPS * 32, 4) k_refine_coop(Blk B, Bat T, 
         VariantList V;
         variants_init(V, vk, n, maxalnmax, phase2 ? T.sfndx[i] : 0, phase2 ? T.sfpos[i] : 0, T.plog_round);
         if (MODE == RM_PROD1 && warp == CM_WARPS - 1 && crank == 0 && V.total > 0) {
-            const float r = coop_rmsd(w, n, cA, cB, lane);
+            const float r = rmsd_warp(w.buf, n, [&](int p, float* q) {
+                const float4 u = cA[p];
+                const float2 v = cB[p];
+                q[0] = u.x; q[1] = u.y; q[2] = u.z; q[3] = u.w; q[4] = v.x; q[5] = v.y;
+            }, lane);
             if (lane == 0) T.rmsd32[i] = r;
         }
         // variants a warp holds: an even share of the pair's
@@ -2178,8 +2059,272 @@ __global__ void __launch_bounds__(CM_WARPS * 32, 4) k_refine_coop(Blk B, Bat T, 
     if (C > 1) cl.sync();              // the first CTA's shared memory is read until here
 }
 
+// ---------------------------------------------------------------------------
+// Long pairs, few of them: a CTA to a pass.  The variants of a pair of 5,000
+// positions (750) are drawn one at a time by the CTAs of the launch; a pass
+// gives each warp every CL_WARPS-th group of CM_CHUNK blocks, as coop_pass sums
+// them, the block sums meet in shared memory and 16 lanes fold them in block
+// order.  Every thread holds the variant's state.  (A warp to a variant, a block
+// per lane, took 28,000 cycles a pass at 5,000 positions; refinement of one such
+// pair 47.0 -> 14.6 ms.)
+constexpr int CL_WARPS = 4;
+constexpr int CL_SEG = 256;                  // blocks between two folds
+struct LongSmem {
+    float buf[CL_WARPS][CM_CHUNK * CM_BLKW];
+    float sums[CL_SEG * 16];                 // block sums of a segment
+    float tot[16];
+    float m3[CL_WARPS][3];
+    int cnt[CL_WARPS];
+    float tb[12], tbest[12];
+    int kv;
+};
+
+// one pass: the sums, the score, the count and the third-smallest distance, on
+// every thread (v[0..14], v[15] count; returns the score)
+__device__ float long_pass(LongSmem& S, const PairGeom& G, int kind, int k0, int k1, const float* tfm,
+                           float d02, int chk, float d82, float thr, int trk, float* v, float& m3out) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const bool frag = kind == PK_FRAG;
+    const bool scr = kind == PK_SCORE || kind == PK_GSCORE;
+    const bool cov = kind == PK_SCORE || kind == PK_EXT;
+    const int lim = frag ? k1 : G.n;
+    const int nblk = (lim + BLK - 1) / BLK;
+    const int f = lane & 15;
+    const int ax = f < 9 ? f / 3 : (f < 12 ? f - 9 : (f < 15 ? f - 9 : 6));
+    const int ay = f < 9 ? 3 + f % 3 : 7;
+    float* buf = S.buf[wp];
+    const float* X = buf + (lane >> 4) * CM_BLKW + ax * CM_BST;
+    const float* Y = buf + (lane >> 4) * CM_BLKW + ay * CM_BST;
+    float s = 0.f, c = 0.f;
+    float m1 = LARGEDST, m2 = LARGEDST, m3 = LARGEDST;
+    int cnt = 0;
+    for (int sb = frag ? k0 / BLK : 0; sb < nblk; sb += CL_SEG) {
+        const int se = sb + CL_SEG < nblk ? sb + CL_SEG : nblk;
+        __syncthreads();                     // the last segment's sums are folded
+        for (int cb = sb + wp * CM_CHUNK; cb < se; cb += CL_WARPS * CM_CHUNK) {
+            float q[CM_CHUNK][6];
+#pragma unroll
+            for (int e = 0; e < CM_CHUNK; e++) {
+                const int p = (cb + e) * BLK + lane;
+#pragma unroll
+                for (int k = 0; k < 6; k++) q[e][k] = 0.f;
+                if (p < lim) G.at(p, q[e][0], q[e][1], q[e][2], q[e][3], q[e][4], q[e][5]);
+            }
+#pragma unroll
+            for (int e = 0; e < CM_CHUNK; e++) {
+                const int p = (cb + e) * BLK + lane;
+                const bool in = p < lim;
+                bool inc = in && k0 <= p;
+                float tm = 0.f;
+                if (!frag) {
+                    const float d = dist2_tf(tfm, q[e][0], q[e][1], q[e][2], q[e][3], q[e][4], q[e][5]);
+                    inc = in && cov && d <= thr;
+                    const float x = tmterm(d02, d);
+                    tm = in && scr && (!chk || d <= d82) ? x : 0.f;
+                    if (trk && in) keep3(d, m1, m2, m3);
+                }
+                float* o = buf + e * CM_BLKW + lane;
+#pragma unroll
+                for (int k = 0; k < 6; k++) o[k * CM_BST] = inc ? q[e][k] : 0.f;
+                o[6 * CM_BST] = tm;
+                cnt += __popc(__ballot_sync(FULL, inc));
+            }
+            __syncwarp();
+            float b[CM_CHUNK / 2];
+#pragma unroll
+            for (int e = 0; e < CM_CHUNK / 2; e++) b[e] = 0.f;
+#pragma unroll
+            for (int p = 0; p < BLK; p += 4)
+#pragma unroll
+                for (int e = 0; e < CM_CHUNK / 2; e++) {
+                    const float4 x = *(const float4*)(X + 2 * e * CM_BLKW + p), y = *(const float4*)(Y + 2 * e * CM_BLKW + p);
+                    b[e] = __fmaf_rn(x.x, y.x, b[e]); b[e] = __fmaf_rn(x.y, y.y, b[e]);
+                    b[e] = __fmaf_rn(x.z, y.z, b[e]); b[e] = __fmaf_rn(x.w, y.w, b[e]);
+                }
+            __syncwarp();
+#pragma unroll
+            for (int e = 0; e < CM_CHUNK / 2; e++) {
+                const int blk = cb + 2 * e + (lane >> 4);
+                if (blk < se) S.sums[(blk - sb) * 16 + f] = b[e];
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x < 16)
+            for (int k = 0; k < se - sb; k++) tfold(s, c, S.sums[k * 16 + threadIdx.x]);
+    }
+    if (threadIdx.x < 16) S.tot[threadIdx.x] = __fadd_rn(s, c);
+    if (trk) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float x1 = __shfl_xor_sync(FULL, m1, o), x2 = __shfl_xor_sync(FULL, m2, o),
+                        x3 = __shfl_xor_sync(FULL, m3, o);
+            keep3(x1, m1, m2, m3); keep3(x2, m1, m2, m3); keep3(x3, m1, m2, m3);
+        }
+        if (lane == 0) { S.m3[wp][0] = m1; S.m3[wp][1] = m2; S.m3[wp][2] = m3; }
+    }
+    if (lane == 0) S.cnt[wp] = cnt;
+    __syncthreads();
+    m1 = m2 = m3 = LARGEDST;
+    cnt = 0;
+#pragma unroll
+    for (int k = 0; k < CL_WARPS; k++) {
+        cnt += S.cnt[k];
+        if (trk) { keep3(S.m3[k][0], m1, m2, m3); keep3(S.m3[k][1], m1, m2, m3); keep3(S.m3[k][2], m1, m2, m3); }
+    }
+    m3out = m3;
+#pragma unroll
+    for (int k = 0; k < 15; k++) v[k] = S.tot[k];
+    v[15] = (float)cnt;
+    const float sc = S.tot[15];
+    __syncthreads();                         // tot, cnt and m3 are read
+    return sc;
+}
+
+// The whole alignment's FP32 RMSD (production phase 1): warp 0 as coop_rmsd, from
+// the pair's positions.
+__device__ float long_rmsd(LongSmem& S, const PairGeom& G) {
+    float r = 0.f;
+    if (threadIdx.x < 32)
+        r = rmsd_warp(S.buf[0], G.n, [&](int p, float* q) { G.at(p, q[0], q[1], q[2], q[3], q[4], q[5]); },
+                      (int)threadIdx.x);
+    return r;
+}
+
+// The CTAs of a long pair (4 * T.rlw_ctas, a candidate each) draw its variants
+// from a counter; k_refine_long_fin picks the winner among the candidates.
+template <int MODE>
+__global__ void __launch_bounds__(CL_WARPS * 32, 4) k_refine_long(Blk B, Bat T) {
+    extern __shared__ __align__(16) unsigned char cl_smem[];
+    LongSmem& S = *(LongSmem*)cl_smem;
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const int nc = T.rlw_ctas * RF_WARPS_LONG, nlong = *T.rl_count;
+    for (int e = 0; e < CM_CHUNK; e++) S.buf[wp][e * CM_BLKW + 7 * CM_BST + lane] = 1.f;
+    for (int slot = (int)blockIdx.x / nc; slot < nlong; slot += (int)gridDim.x / nc) {
+        const int cand = (int)blockIdx.x % nc;
+        const int i = T.rl_long[slot];
+        const int qi = pair_qi(B, T, i), ri = pair_ri(B, T, i);
+        const int lq = B.qlen[qi], lr = B.rlen[ri];
+        const int ml = lq < lr ? lq : lr;
+        const int swap = B.symmetric && (lq < lr);
+        PairGeom G;
+        G.q4 = B.q4 + B.q4off[qi]; G.r4 = B.r4 + B.r4off[ri];
+        G.alc = nullptr;
+        G.q0 = G.r0 = 0;
+        if (MODE == RM_INIT) {
+            G.q0 = T.seedq[i]; G.r0 = T.seedr[i];
+            G.n = (lq - G.q0) < (lr - G.r0) ? (lq - G.q0) : (lr - G.r0);
+        } else {
+            G.alc = (const float2*)(T.alc + 6 * T.off_aln[i]);
+            G.n = T.naln[i];
+        }
+        const int n = G.n;
+        const bool prod = (MODE == RM_PROD1 || MODE == RM_PROD2 || MODE == RM_PLOG);
+        const bool phase2 = (MODE == RM_FIN2 || MODE == RM_PROD2 || MODE == RM_PLOG);
+        const int vk = refine_variants(MODE, B);
+        const float d0 = prod ? B.t_d0fin[ml] : B.t_d0[ml];
+        const float d02 = __fmul_rn(d0, d0);
+        const float d82 = B.t_d82[ml];
+        const int chk = prod ? 0 : 1;
+        const float best_init = (MODE == RM_INIT || MODE == RM_DP) ? 0.f
+                              : MODE == RM_PLOG ? T.grand[i] : -1.f;
+        const int maxalnmax = B.qmax < B.rmax ? B.qmax : B.rmax;
+        const float d0s = d0s_of(d0);
+        const float d0sm = __fsub_rn(d0s, 1.0f);
+        const float d02s = __fmul_rn(d0sm, d0sm);             // iteration 1's usual threshold
+        const float d0sp = __fadd_rn(d0s, 1.0f);
+        const float thr2 = __fmul_rn(d0sp, d0sp);             // threshold of iterations >= 2
+        const bool gscore = prod && lq != lr;                 // also scored by the longer length
+        float g02 = 0.f;
+        if (gscore) { const float g0 = B.t_d0fin[lq > lr ? lq : lr]; g02 = __fmul_rn(g0, g0); }
+        VariantList V;
+        variants_init(V, vk, n, maxalnmax, phase2 ? T.sfndx[i] : 0, phase2 ? T.sfpos[i] : 0, T.plog_round);
+        if (MODE == RM_PROD1 && cand == 0 && V.total > 0) {
+            const float r = long_rmsd(S, G);
+            if (threadIdx.x == 0) T.rmsd32[i] = r;
+        }
+        float lbest = 0.f, lgbest = 0.f;                      // this CTA's best variant so far
+        int lsi = 0x7fffffff, lndx = 0, lpos = 0;
+        unsigned long long vis = 0;
+        for (;;) {
+            __syncthreads();
+            if (threadIdx.x == 0) S.kv = atomicAdd(T.rl_next + slot, 1);
+            __syncthreads();
+            const int kv = S.kv;
+            if (kv >= V.total) break;
+            int si, vndx, vpos, fl, kf;
+            variants_get(V, vk, n, kv, si, vndx, vpos, fl, kf);
+            if (MODE == RM_DP && T.vskip && si < 32 * F3_NSEC &&
+                ((T.vskip[(long long)i * F3_NSEC + (si >> 5)] >> (si & 31)) & 1u))
+                continue;                      // a variant the detailed search's slots rule out
+            float v[16], last[16], tfm[12], m3, best = best_init, thr = d02s;
+            long_pass(S, G, PK_FRAG, kf, kf + fl, nullptr, d02, chk, d82, thr, 0, v, m3);
+            vis += (unsigned)fl;
+            if (v[15] < 1.0f) continue;
+            bool more = true, ext = false;
+            for (int cit = 0; more;) {
+                if (!ext) {
+#pragma unroll
+                    for (int f = 0; f < 16; f++) last[f] = v[f];
+                    solve_sums(v, swap, tfm);
+                    const float sc = long_pass(S, G, PK_SCORE, 0, 0, tfm, d02, chk, d82, thr, cit == 0, v, m3);
+                    vis += (unsigned)n;
+                    if (best < sc) {
+                        best = sc;
+                        if (threadIdx.x == 0) {
+#pragma unroll
+                            for (int f = 0; f < 12; f++) S.tb[f] = tfm[f];
+                        }
+                    }
+                    if (cit++ == 0) {
+                        // iteration 1's threshold from iteration 0's three smallest distances
+                        float dst32;
+                        if (LARGEDST_CMP < m3 || m3 < d02s || n <= 3) dst32 = d02s;
+                        else {
+                            const float t = __fadd_rn(d0sm, __fmul_rn(ceilf(__fmul_rn(__fsub_rn(__fsqrt_rn(m3), d0sm), 2.0f)), 0.5f));
+                            dst32 = __fmul_rn(t, t);
+                        }
+                        if (dst32 != d02s) { ext = true; thr = dst32; continue; }
+                    }
+                } else {
+                    long_pass(S, G, PK_EXT, 0, 0, tfm, d02, chk, d82, thr, 0, v, m3);
+                    vis += (unsigned)n;
+                    ext = false;
+                }
+                more = !(cit >= NMAXCONVIT + 2 || converged16(v, last, 1) || v[15] < 1.0f);
+                thr = thr2;
+            }
+            float gbest = best;
+            __syncthreads();                                  // tb
+            if (gscore && best >= 0.f && (MODE != RM_PLOG || best > best_init)) {
+                // one more pass: the variant's best transform scored with the
+                // d0 of the longer structure
+#pragma unroll
+                for (int f = 0; f < 12; f++) tfm[f] = S.tb[f];
+                gbest = long_pass(S, G, PK_GSCORE, 0, 0, tfm, g02, 0, d82, thr, 0, v, m3);
+                vis += (unsigned)n;
+            }
+            if (best > 0.f && (lbest < best || (lbest == best && si < lsi))) {
+                lbest = best; lgbest = gbest; lsi = si; lndx = vndx; lpos = vpos;
+                if (threadIdx.x < 12) S.tbest[threadIdx.x] = S.tb[threadIdx.x];
+            }
+        }
+        if (threadIdx.x == 0) {
+            work_add(T, WK_REFINE, vis);
+            float* c = T.rl_cand + ((long long)slot * nc + cand) * RLW_CAND;
+            c[0] = lbest;
+            c[1] = __int_as_float(lsi);
+            c[2] = lgbest;
+            c[3] = __int_as_float(lndx);
+            c[4] = __int_as_float(lpos);
+#pragma unroll
+            for (int f = 0; f < 12; f++) c[5 + f] = S.tbest[f];
+        }
+    }
+}
+
 // npair: pairs the launch may have at most (a lane form's grid)
-template <int LPP, bool LONG, bool WIDE = false>
+template <int LPP, bool LONG>
 static void launch_refine_k(int mode, const Blk& B, const Bat& T, cudaStream_t st, int npair = 0,
                             int lo = 0, int hi = 0) {
     constexpr int W = LONG ? RF_WARPS_LONG : RF_WARPS_SHORT;
@@ -2189,13 +2334,13 @@ static void launch_refine_k(int mode, const Blk& B, const Bat& T, cudaStream_t s
                         : (npair + (32 / LPP) * W - 1) / ((32 / LPP) * W);
     const int nt = W * 32;
     switch (mode) {
-        case RM_INIT:  k_refine<RM_INIT, LPP, LONG, WIDE><<<ng, nt, 0, st>>>(B, T, lo, hi); break;
-        case RM_DP:    k_refine<RM_DP, LPP, LONG, WIDE><<<ng, nt, 0, st>>>(B, T, lo, hi); break;
-        case RM_FIN1:  k_refine<RM_FIN1, LPP, LONG, WIDE><<<ng, nt, 0, st>>>(B, T, lo, hi); break;
-        case RM_FIN2:  k_refine<RM_FIN2, LPP, LONG, WIDE><<<ng, nt, 0, st>>>(B, T, lo, hi); break;
-        case RM_PROD1: k_refine<RM_PROD1, LPP, LONG, WIDE><<<ng, nt, 0, st>>>(B, T, lo, hi); break;
-        case RM_PROD2: k_refine<RM_PROD2, LPP, LONG, WIDE><<<ng, nt, 0, st>>>(B, T, lo, hi); break;
-        case RM_PLOG:  k_refine<RM_PLOG, LPP, LONG, WIDE><<<ng, nt, 0, st>>>(B, T, lo, hi); break;
+        case RM_INIT:  k_refine<RM_INIT, LPP, LONG><<<ng, nt, 0, st>>>(B, T, lo, hi); break;
+        case RM_DP:    k_refine<RM_DP, LPP, LONG><<<ng, nt, 0, st>>>(B, T, lo, hi); break;
+        case RM_FIN1:  k_refine<RM_FIN1, LPP, LONG><<<ng, nt, 0, st>>>(B, T, lo, hi); break;
+        case RM_FIN2:  k_refine<RM_FIN2, LPP, LONG><<<ng, nt, 0, st>>>(B, T, lo, hi); break;
+        case RM_PROD1: k_refine<RM_PROD1, LPP, LONG><<<ng, nt, 0, st>>>(B, T, lo, hi); break;
+        case RM_PROD2: k_refine<RM_PROD2, LPP, LONG><<<ng, nt, 0, st>>>(B, T, lo, hi); break;
+        case RM_PLOG:  k_refine<RM_PLOG, LPP, LONG><<<ng, nt, 0, st>>>(B, T, lo, hi); break;
     }
 }
 
@@ -2234,13 +2379,13 @@ static void launch_refine_coop(int mode, const Blk& B, const Bat& T, cudaStream_
 // for the smallest shared-memory carve-out that holds as many CTAs as their
 // registers allow (static arrays + the 1 kB each CTA reserves), leaving the
 // rest of the SM's 256 kB to L1.
-template <int LPP, bool LONG, bool WIDE = false>
+template <int LPP, bool LONG>
 static void carve_refine() {
     constexpr int W = LONG ? RF_WARPS_LONG : RF_WARPS_SHORT;
-    const void* ks[7] = {(const void*)k_refine<RM_INIT, LPP, LONG, WIDE>, (const void*)k_refine<RM_DP, LPP, LONG, WIDE>,
-                         (const void*)k_refine<RM_FIN1, LPP, LONG, WIDE>, (const void*)k_refine<RM_FIN2, LPP, LONG, WIDE>,
-                         (const void*)k_refine<RM_PROD1, LPP, LONG, WIDE>, (const void*)k_refine<RM_PROD2, LPP, LONG, WIDE>,
-                         (const void*)k_refine<RM_PLOG, LPP, LONG, WIDE>};
+    const void* ks[7] = {(const void*)k_refine<RM_INIT, LPP, LONG>, (const void*)k_refine<RM_DP, LPP, LONG>,
+                         (const void*)k_refine<RM_FIN1, LPP, LONG>, (const void*)k_refine<RM_FIN2, LPP, LONG>,
+                         (const void*)k_refine<RM_PROD1, LPP, LONG>, (const void*)k_refine<RM_PROD2, LPP, LONG>,
+                         (const void*)k_refine<RM_PLOG, LPP, LONG>};
     int dev = 0, smem_sm = 0, regs_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
@@ -2264,7 +2409,6 @@ static void carve_refine() {
 void configure_kernels() {
     carve_refine<16, false>();
     carve_refine<32, true>();
-    carve_refine<32, true, true>();
     const void* kc[7] = {(const void*)k_refine_coop<RM_INIT>, (const void*)k_refine_coop<RM_DP>,
                          (const void*)k_refine_coop<RM_FIN1>, (const void*)k_refine_coop<RM_FIN2>,
                          (const void*)k_refine_coop<RM_PROD1>, (const void*)k_refine_coop<RM_PROD2>,
@@ -2274,6 +2418,20 @@ void configure_kernels() {
     float gs[GTB_GONNET_NA * GTB_GONNET_NA];
     gtb_gonnet_scores(gs);
     cudaMemcpyToSymbol(g_gonnet, gs, sizeof(gs));
+}
+
+static void launch_refine_long(int mode, const Blk& B, const Bat& T, cudaStream_t st) {
+    const int ng = T.rl_nlmax * T.rlw_ctas * RF_WARPS_LONG, nt = CL_WARPS * 32;
+    const size_t sm = sizeof(LongSmem);
+    switch (mode) {
+        case RM_INIT:  k_refine_long<RM_INIT><<<ng, nt, sm, st>>>(B, T); break;
+        case RM_DP:    k_refine_long<RM_DP><<<ng, nt, sm, st>>>(B, T); break;
+        case RM_FIN1:  k_refine_long<RM_FIN1><<<ng, nt, sm, st>>>(B, T); break;
+        case RM_FIN2:  k_refine_long<RM_FIN2><<<ng, nt, sm, st>>>(B, T); break;
+        case RM_PROD1: k_refine_long<RM_PROD1><<<ng, nt, sm, st>>>(B, T); break;
+        case RM_PROD2: k_refine_long<RM_PROD2><<<ng, nt, sm, st>>>(B, T); break;
+        case RM_PLOG:  k_refine_long<RM_PLOG><<<ng, nt, sm, st>>>(B, T); break;
+    }
 }
 
 static void launch_refine_long_fin(int mode, const Blk& B, const Bat& T, cudaStream_t st) {
@@ -2318,9 +2476,17 @@ void launch_refine(int mode, const Blk& B, const Bat& T0, cudaStream_t st, bool 
         cudaStreamWaitEvent(T.st2, T.evfork, 0);
     }
     if (T.rl_long) {
-        if (T.rl_nlmax <= RLW_WIDE_MAX) launch_refine_k<32, true, true>(mode, B, T, sl);
-        else launch_refine_k<32, true>(mode, B, T, sl);
-        launch_refine_long_fin(mode, B, T, sl);
+        if (T.rl_nlmax <= RLW_CTA_MAX) {
+            // a CTA to a pass, up to RLW_CTA_GRID CTAs in all; they leave a
+            // candidate each, in the room of 4 CTAs' warps
+            Bat TL = T;
+            TL.rlw_ctas = std::max(4, std::min(T.rlw_ctas, RLW_CTA_GRID / 4 / T.rl_nlmax));
+            launch_refine_long(mode, B, TL, sl);
+            launch_refine_long_fin(mode, B, TL, sl);
+        } else {
+            launch_refine_k<32, true>(mode, B, T, sl);
+            launch_refine_long_fin(mode, B, T, sl);
+        }
         if (T.launches) (*T.launches) += 2;
     } else if (T.nml[3] > 0) {
         launch_refine_k<16, false>(mode, B, T, sl, T.nml[3], RL_LONG, 0);

@@ -36,10 +36,11 @@ constexpr int RLW_CTAS = 16;
 constexpr int RLW_GRID = 1024;
 constexpr int RLW_CTAS_MAX = 256;
 constexpr int RLW_CTA_WARPS = 4;     // warps of a long-pair CTA (one candidate each)
-// a sub-batch with at most this many pairs in the first long-pair tier runs
-// them with a variant per warp (its lanes share each pass) instead of a
-// variant per lane: too few variants to fill the lanes otherwise
-constexpr int RLW_WIDE_MAX = 64;
+// A sub-batch with at most RLW_CTA_MAX long pairs runs their passes a CTA each
+// (k_refine_long) over RLW_CTA_GRID CTAs in all: too few variants to fill the
+// lanes of the other form
+constexpr int RLW_CTA_MAX = 64;
+constexpr int RLW_CTA_GRID = 592;
 constexpr int RLW_CAND = 17;         // floats per warp candidate
 // CTAs per pair of a long-pair tier with `nlong` possible pairs: `base`, or
 // as many as fill RLW_GRID CTAs, at most RLW_CTAS_MAX
