@@ -2853,15 +2853,11 @@ __device__ __forceinline__ bool dp_pair_fast(const float* t, float d02, float gc
 // (the first of its CTA's) makes the walk right after it, beside other pairs' DPs.
 // The 32 words of a (strip,
 // step group), one 128-byte line, come in for BT_WIN groups at a time into
-// shared memory, and the lines the path enters next (the groups below, and the
-// previous strip's around the path's column) are on their way to L1.  32
-// aligned pairs at a time are written out, a pair per lane.
+// shared memory while the ones the path is likely to enter next (the groups below,
+// or the previous strip's where a diagonal path enters it) are on their way to
+// registers.  32 aligned pairs at a time are written out, a pair per lane.
 constexpr int BT_WIN = 16;        // groups of a window
 constexpr int BT_WARPS = 4;
-__device__ __forceinline__ void bt_prefetch(const unsigned* p) {
-    asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
-}
-
 template <int R>
 __device__ __forceinline__ int btck_walk(const unsigned* bt, int lq, int lr, const float4* q4,
                                          const float4* r4, bool constrained, const float* t,
@@ -2870,59 +2866,80 @@ __device__ __forceinline__ int btck_walk(const unsigned* bt, int lq, int lr, con
     const unsigned FULL = 0xffffffffu;
     constexpr int ROWS = 32 * R, SPW = 16 / R;
     const long long sw = bt_strip_words(lr, R);
+    const int ngrp = (int)(sw / 32);
     int y = lq - 1, x = lr - 1, n = 0, pend = 0;
     unsigned mine = 0;                        // this lane's aligned pair among the last 32
     auto flush = [&](int cnt) {
-        float4 cq = make_float4(0.f, 0.f, 0.f, 0.f), cr = cq;
         bool keep = lane < cnt;
-        if (keep) {
-            cq = __ldg(q4 + (mine >> 16));
-            cr = __ldg(r4 + (mine & 0xffffu));
-            if (constrained) keep = dist2_tf(t, cq.x, cq.y, cq.z, cr.x, cr.y, cr.z) <= d82;
+        if (constrained && keep) {
+            const float4 cq = __ldg(q4 + (mine >> 16)), cr = __ldg(r4 + (mine & 0xffffu));
+            keep = dist2_tf(t, cq.x, cq.y, cq.z, cr.x, cr.y, cr.z) <= d82;
         }
         const unsigned m = __ballot_sync(FULL, keep);
-        if (keep) {
-            const int k = n + __popc(m & ((1u << lane) - 1u));
-            aln[k] = mine;
-            float2* c2 = (float2*)(alc + 6 * (long long)k);
-            c2[0] = make_float2(cq.x, cq.y); c2[1] = make_float2(cq.z, cr.x); c2[2] = make_float2(cr.y, cr.z);
-        }
+        if (keep) aln[n + __popc(m & ((1u << lane) - 1u))] = mine;
         n += __popc(m);
+    };
+    // the words of BT_WIN groups, loaded into registers while the walk is in the
+    // window before: strip ps, groups pg, pg - 1, ...
+    unsigned pw[BT_WIN];
+    int ps = -1, pg = 0;
+    auto load = [&](int s, int g) {
+        const unsigned* line = bt + s * sw + lane;
+        ps = s; pg = g;
+#pragma unroll
+        for (int k = 0; k < BT_WIN; k++) pw[k] = g - k >= 0 ? line[(g - k) * 32] : 0u;
     };
     int cs = -1, wlo = 0;                     // the window's strip and lowest group
     while ((x | y) >= 0) {
         const int s = y / ROWS, l = y % ROWS / R, tt = x + l, g = tt / SPW;
         if (s != cs || g < wlo) {
+            if (ps != s || g > pg || g <= pg - BT_WIN / 2) load(s, g);
             cs = s;
-            wlo = g - BT_WIN + 1 > 0 ? g - BT_WIN + 1 : 0;
-            const unsigned* line = bt + s * sw;
+            wlo = pg - BT_WIN + 1 > 0 ? pg - BT_WIN + 1 : 0;
             __syncwarp();
 #pragma unroll
-            for (int k = 0; k < BT_WIN; k++)
-                if (g - k >= 0) win[((g - k) & (BT_WIN - 1)) * 32 + lane] = line[(g - k) * 32 + lane];
-            if (lane < BT_WIN) {
-                if (wlo - 1 - lane >= 0) bt_prefetch(line + (wlo - 1 - lane) * 32);
-            } else if (s > 0) {
-                const int gp = (x + 31) / SPW - (lane - BT_WIN);
-                if (gp >= 0) bt_prefetch(line - sw + gp * 32);
-            }
+            for (int k = 0; k < BT_WIN; k++) win[((pg - k) & (BT_WIN - 1)) * 32 + lane] = pw[k];
             __syncwarp();
-        }
-        // the path through one word: R rows x SPW steps
-        const unsigned w = win[(g & (BT_WIN - 1)) * 32 + l];
-        int rr = y % R, uu = tt % SPW;
-        do {
-            const unsigned b = (w >> (2 * R * uu + 2 * rr)) & 3u;
-            if (b == BTW_DIAG) {
-                if (lane == pend) mine = ((unsigned)y << 16) | (unsigned)x;
-                if (++pend == 32) { flush(32); pend = 0; }
+            // what comes next if the path goes on diagonally: the groups below, or
+            // the previous strip's from where the path leaves this one
+            const int left = y % ROWS + 1;
+            if (left * (R + 1) / R < (g - wlo) * SPW) {
+                const int xn = x - left;
+                if (s > 0 && xn >= 0) load(s - 1, (xn + 31) / SPW + 1 < ngrp ? (xn + 31) / SPW + 1 : ngrp - 1);
+            } else if (wlo > 0) {
+                load(s, wlo - 1);
             }
-            const int dy = b != BTW_LEFT, dx = b < BTW_UP;    // up is 2 or 3, left 1, diagonal 0
-            y -= dy; rr -= dy;
-            x -= dx; uu -= dx;
-        } while ((rr | uu | x) >= 0);
+        }
+        // the path through one word (R rows x SPW steps): bits 0-4 of pos are the
+        // cell's place in the word, row and step above them with a guard bit
+        // each that turns when they fall below 0; the column's sign is looked at
+        // too (a word can hold steps before the first column)
+        const unsigned w = win[(g & (BT_WIN - 1)) * 32 + l];
+        const int rr = y % R, uu = tt % SPW;
+        unsigned pos = (unsigned)(2 * R * uu + 2 * rr) | (unsigned)rr << 8 | (unsigned)uu << 16;
+        do {
+            const unsigned b = (w >> (pos & 31)) & 3u;
+            const unsigned yx = ((unsigned)y << 16) | (unsigned)x;
+            if (b == BTW_DIAG && lane == pend) mine = yx;
+            pend += b == BTW_DIAG;
+            y -= b != BTW_LEFT;
+            x -= b < BTW_UP;
+            // diagonal (0), left (1), up (2 or 3): down a row, back a step
+            pos -= b >= BTW_UP ? 2u + (1u << 8)
+                               : (b == BTW_LEFT ? 2u * R + (1u << 16) : 2u * R + 2u + (1u << 8) + (1u << 16));
+        } while (!(pos & 0x80008000u) && x >= 0);
+        if (pend > 32 - R) { flush(pend); pend = 0; }     // a word adds at most R
     }
     if (pend > 0) flush(pend);
+    // the aligned residues' coordinates, for the passes that read them in a row
+    __syncwarp();
+#pragma unroll 4
+    for (int k = lane; k < n; k += 32) {
+        const unsigned m = aln[k];
+        const float4 cq = __ldg(q4 + (m >> 16)), cr = __ldg(r4 + (m & 0xffffu));
+        float2* c2 = (float2*)(alc + 6 * (long long)k);
+        c2[0] = make_float2(cq.x, cq.y); c2[1] = make_float2(cq.z, cr.x); c2[2] = make_float2(cr.y, cr.z);
+    }
     return n;
 }
 
