@@ -23,7 +23,7 @@
 //    shuffles, each lane packs the 2-bit directions of its cells into
 //    traceback words.  A long pair's strips run as a wavefront over several
 //    single-warp CTAs (cooperative launch, bounded waits on progress counters).
-//  * traceback: a warp per pair; alignment rows, bookkeeping: a thread per pair.
+//  * traceback, alignment rows, final scores: a warp per pair.
 // All floating-point reductions are sequential per thread in forward position
 // order (blocks of BLK positions, Neumaier-compensated), so results do not
 // depend on the launch geometry.
@@ -3324,88 +3324,128 @@ void launch_lowscore(const Blk& B, const Bat& T, float thr, cudaStream_t st) {
 // count is known; that count follows from the first and last aligned pairs:
 // every aligned pair is one column, every skipped query residue between them
 // one, and every skipped reference residue one unless --no-deletions.
-__global__ void k_alnstr(Blk B, Bat T) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+//
+// A warp per pair, a lane per aligned pair: its columns (itself and the skipped
+// residues up to the next aligned pair) start at the running sum of the columns
+// before.  (A thread per pair wrote its rows byte by byte: 0.39 ms for a pair of
+// 1,200 residues, 1.5 ms for 5,000.)
+__global__ void __launch_bounds__(128) k_alnstr(Blk B, Bat T) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int i = blockIdx.x * 4 + (threadIdx.x >> 5);
     if (i >= T.np) return;
     if (T.flags[i] & CONV_LOWTMSC) {
-        if (T.str) T.str_off[i] = -1;      // no alignment
+        if (T.str && lane == 0) T.str_off[i] = -1;      // no alignment
         return;
     }
     int qi = pair_qi(B, T, i), ri = pair_ri(B, T, i);
     const unsigned* aln = T.aln + T.off_aln[i];
-    int n = T.naln[i];
+    const int n = T.naln[i];
     float t[12];
 #pragma unroll
     for (int f = 0; f < 12; f++) t[f] = T.tfm_gr[i * 12 + f];
-    const float *qx = B.qx + B.qoff[qi], *qy = B.qy + B.qoff[qi], *qz = B.qz + B.qoff[qi];
-    const float *rx = B.rx + B.roff[ri], *ry = B.ry + B.roff[ri], *rz = B.rz + B.roff[ri];
+    const float4* q4 = B.q4 + B.q4off[qi];
+    const float4* r4 = B.r4 + B.r4off[ri];
     const unsigned char* qa = B.qa + B.qoff[qi];
     const unsigned char* ra = B.ra + B.roff[ri];
     const char* qs = B.qs + B.qoff[qi];
     const char* rs = B.rs + B.roff[ri];
     char* dst = nullptr;
     int W = 1;
+    unsigned wf = 0, wl = 0;                             // first and last aligned pairs
+    if (n > 0) { wf = aln[n - 1]; wl = aln[0]; }
     if (T.str) {
         int ncol = 0;
         if (n > 0) {
-            const unsigned wf = aln[n - 1], wl = aln[0];   // first and last aligned pairs
             const int qf = (int)(wf >> 16), rf = (int)(wf & 0xffffu);
             const int ql = (int)(wl >> 16), rl = (int)(wl & 0xffffu);
             ncol = n + (ql - qf + 1 - n) + (B.nodeletions ? 0 : (rl - rf + 1 - n));
         }
         W = ncol + 1;
-        const unsigned long long o = atomicAdd(T.str_cnt, 5ull * (unsigned long long)W);
-        T.str_off[i] = (long long)o;
-        dst = T.str + o;
+        unsigned long long o = 0;
+        if (lane == 0) {
+            o = atomicAdd(T.str_cnt, 5ull * (unsigned long long)W);
+            T.str_off[i] = (long long)o;
+        }
+        dst = T.str + __shfl_sync(FULL, o, 0);
     }
-    int col = 0, psts = 0, idts = 0, gaps = 0;
-    unsigned bc = 0, ec = 0;
-    for (int k = 0; k < n; k++) {
-        unsigned wv = aln[n - 1 - k];
-        int q = (int)(wv >> 16), r = (int)(wv & 0xffffu);
-        float d = dist2_tf(t, qx[q], qy[q], qz[q], rx[r], ry[r], rz[r]);
-        unsigned cc = ((unsigned)(r + 1) << 16) | (unsigned)(q + 1);
-        if (k == 0) bc = cc;
-        ec = cc;
-        int eq = d < 25.0f;
-        if (eq) psts++;
-        char a = (char)qa[q], b = (char)ra[r];
-        char mc = eq ? '+' : ' ';
-        if (a != '-' && a == b) { idts++; mc = eq ? a : (char)(a | 32); }
-        if (dst) { dst[col] = a; dst[2 * W + col] = b; dst[3 * W + col] = qs[q]; dst[4 * W + col] = rs[r]; dst[W + col] = mc; }
-        col++;
-        if (k + 1 < n) {
-            unsigned w1 = aln[n - 2 - k];
-            int q1 = (int)(w1 >> 16), r1 = (int)(w1 & 0xffffu);
-            for (int qq = q + 1; qq < q1; qq++) {
-                if (dst) { dst[col] = (char)qa[qq]; dst[3 * W + col] = qs[qq]; dst[2 * W + col] = '-'; dst[4 * W + col] = ' '; dst[W + col] = ' '; }
-                col++; gaps++;
+    int col = 0, psts = 0, idts = 0;                     // col: columns so far (every lane)
+    for (int k0 = 0; k0 < n; k0 += 32) {
+        const int k = k0 + lane;
+        int q = 0, r = 0, gq = 0, gr = 0, wid = 0;
+        if (k < n) {
+            const unsigned wv = aln[n - 1 - k];
+            q = (int)(wv >> 16); r = (int)(wv & 0xffffu);
+            wid = 1;
+            if (k + 1 < n) {
+                const unsigned w1 = aln[n - 2 - k];
+                gq = (int)(w1 >> 16) - q - 1;
+                gr = B.nodeletions ? 0 : (int)(w1 & 0xffffu) - r - 1;
+                wid += gq + gr;
             }
-            if (!B.nodeletions)
-                for (int rr = r + 1; rr < r1; rr++) {
-                    if (dst) { dst[2 * W + col] = (char)ra[rr]; dst[4 * W + col] = rs[rr]; dst[col] = '-'; dst[3 * W + col] = ' '; dst[W + col] = ' '; }
-                    col++; gaps++;
+        }
+        int end = wid;                                   // inclusive sum
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(FULL, end, o);
+            if (lane >= o) end += v;
+        }
+        int c = col + end - wid;
+        col += __shfl_sync(FULL, end, 31);
+        if (k < n) {
+            const float4 u = __ldg(q4 + q), v = __ldg(r4 + r);
+            const int eq = dist2_tf(t, u.x, u.y, u.z, v.x, v.y, v.z) < 25.0f;
+            psts += eq;
+            const char a = (char)qa[q], b = (char)ra[r];
+            char mc = eq ? '+' : ' ';
+            if (a != '-' && a == b) { idts++; mc = eq ? a : (char)(a | 32); }
+            if (dst) {
+                dst[c] = a; dst[2 * W + c] = b; dst[3 * W + c] = qs[q]; dst[4 * W + c] = rs[r]; dst[W + c] = mc;
+                c++;
+                for (int e = q + 1; e <= q + gq; e++, c++) {
+                    dst[c] = (char)qa[e]; dst[3 * W + c] = qs[e]; dst[2 * W + c] = '-'; dst[4 * W + c] = ' '; dst[W + c] = ' ';
                 }
+                for (int e = r + 1; e <= r + gr; e++, c++) {
+                    dst[2 * W + c] = (char)ra[e]; dst[4 * W + c] = rs[e]; dst[c] = '-'; dst[3 * W + c] = ' '; dst[W + c] = ' ';
+                }
+            }
         }
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        psts += __shfl_xor_sync(FULL, psts, o);
+        idts += __shfl_xor_sync(FULL, idts, o);
+    }
+    if (lane != 0) return;
     if (dst) { dst[col] = 0; dst[W + col] = 0; dst[2 * W + col] = 0; dst[3 * W + col] = 0; dst[4 * W + col] = 0; }
-    T.out[i * 16 + 2] = __uint_as_float(bc);
-    T.out[i * 16 + 3] = __uint_as_float(ec);
+    T.out[i * 16 + 2] = __uint_as_float(n > 0 ? ((wf & 0xffffu) + 1) << 16 | ((wf >> 16) + 1) : 0u);
+    T.out[i * 16 + 3] = __uint_as_float(n > 0 ? ((wl & 0xffffu) + 1) << 16 | ((wl >> 16) + 1) : 0u);
     T.out[i * 16 + 4] = (float)col;
     T.out[i * 16 + 5] = (float)psts;
     T.out[i * 16 + 6] = (float)idts;
-    T.out[i * 16 + 7] = (float)gaps;
+    T.out[i * 16 + 7] = (float)(col - n);
 }
 
 void launch_alnstr(const Blk& B, const Bat& T, cudaStream_t st) {
-    k_alnstr<<<(T.np + 127) / 128, 128, 0, st>>>(B, T);
+    k_alnstr<<<(T.np + 3) / 4, 128, 0, st>>>(B, T);
     GTB_LAUNCHED(T);
 }
 
 // ---------------------------------------------------------------------------
 // FP64 recomputation of the reported TM-scores and RMSD, --referenced
-__global__ void k_final(Blk B, Bat T, int referenced) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+//
+// A warp per pair: 32 aligned pairs at a time, a lane each, their score terms and
+// coordinates go to shared memory; then lane f adds the 32 terms of sum f in
+// position order (25 sums: scores by both lengths, without helix mismatches, 9
+// products, 6 coordinates, 6 squares).  (A thread per pair: 860 cycles a
+// position, 0.54 ms for a pair of 1,200 residues.)
+constexpr int FN_WARPS = 4;
+__global__ void __launch_bounds__(FN_WARPS * 32) k_final(Blk B, Bat T, int referenced) {
+    __shared__ float s_x[FN_WARPS][7][33];               // q xyz, r xyz, 1
+    __shared__ double s_t[FN_WARPS][4][33];              // score terms
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const int i = blockIdx.x * FN_WARPS + wp;
     if (i >= T.np) return;
     if (T.flags[i] & CONV_LOWTMSC) return;
     int qi = pair_qi(B, T, i), ri = pair_ri(B, T, i);
@@ -3415,69 +3455,87 @@ __global__ void k_final(Blk B, Bat T, int referenced) {
     float* t = T.tfm_gr + i * 12;
     float* out = T.out + i * 16;
     if (n > 0) {
-        const float *qx = B.qx + B.qoff[qi], *qy = B.qy + B.qoff[qi], *qz = B.qz + B.qoff[qi];
-        const float *rx = B.rx + B.roff[ri], *ry = B.ry + B.roff[ri], *rz = B.rz + B.roff[ri];
+        const float4* q4 = B.q4 + B.q4off[qi];
+        const float4* r4 = B.r4 + B.r4off[ri];
         const char *qs = B.qs + B.qoff[qi], *rs = B.rs + B.roff[ri];
         double d0q = (double)B.t_d0fin[lq], d0r = (double)B.t_d0fin[lr];
-        double d0q2 = __dmul_rn(d0q, d0q), d0r2 = __dmul_rn(d0r, d0r), tq = 0.0, tr = 0.0;
-        double t2q = 0.0, t2r = 0.0;   // --2tm-score sums
-        double dv[21];
-#pragma unroll
-        for (int f = 0; f < 21; f++) dv[f] = 0.0;
+        double d0q2 = __dmul_rn(d0q, d0q), d0r2 = __dmul_rn(d0r, d0r);
         double td[12];
 #pragma unroll
         for (int f = 0; f < 12; f++) td[f] = (double)t[f];
-        for (int k = 0; k < n; k++) {
-            unsigned wv = aln[n - 1 - k];
-            int q = (int)(wv >> 16), r = (int)(wv & 0xffffu);
-            double qq[3] = {(double)qx[q], (double)qy[q], (double)qz[q]};
-            double rr[3] = {(double)rx[r], (double)ry[r], (double)rz[r]};
-            double x = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(td[0], qq[0]), __dmul_rn(td[1], qq[1])), __dmul_rn(td[2], qq[2])), td[9]);
-            double y = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(td[3], qq[0]), __dmul_rn(td[4], qq[1])), __dmul_rn(td[5], qq[2])), td[10]);
-            double z = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(td[6], qq[0]), __dmul_rn(td[7], qq[1])), __dmul_rn(td[8], qq[2])), td[11]);
-            double dx = __dsub_rn(x, rr[0]), dy = __dsub_rn(y, rr[1]), dz = __dsub_rn(z, rr[2]);
-            double d = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-            const double sq = __ddiv_rn(d0q2, __dadd_rn(d0q2, d));
-            const double sr = __ddiv_rn(d0r2, __dadd_rn(d0r2, d));
-            tq = __dadd_rn(tq, sq);
-            tr = __dadd_rn(tr, sr);
+        // this lane's sum (0..20: a product of two components, 21..24: a term)
+        const int ca = lane < 9 ? lane / 3 : lane < 15 ? lane - 9 : lane < 21 ? lane - 15 : 0;
+        const int cb = lane < 9 ? 3 + lane % 3 : lane < 15 ? 6 : lane < 21 ? lane - 15 : 0;
+        const float* X = s_x[wp][ca];
+        const float* Y = s_x[wp][cb];
+        const double* Z = s_t[wp][lane >= 21 && lane < 25 ? lane - 21 : 0];
+        s_x[wp][6][lane] = 1.f;
+        double sum = 0.0;
+        for (int k0 = 0; k0 < n; k0 += 32) {
+            const int k = k0 + lane;
+            __syncwarp();
+            if (k < n) {
+                const unsigned wv = aln[n - 1 - k];
+                const int q = (int)(wv >> 16), r = (int)(wv & 0xffffu);
+                const float4 u = __ldg(q4 + q), v = __ldg(r4 + r);
+                s_x[wp][0][lane] = u.x; s_x[wp][1][lane] = u.y; s_x[wp][2][lane] = u.z;
+                s_x[wp][3][lane] = v.x; s_x[wp][4][lane] = v.y; s_x[wp][5][lane] = v.z;
+                double qq[3] = {(double)u.x, (double)u.y, (double)u.z};
+                double rr[3] = {(double)v.x, (double)v.y, (double)v.z};
+                double x = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(td[0], qq[0]), __dmul_rn(td[1], qq[1])), __dmul_rn(td[2], qq[2])), td[9]);
+                double y = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(td[3], qq[0]), __dmul_rn(td[4], qq[1])), __dmul_rn(td[5], qq[2])), td[10]);
+                double z = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(td[6], qq[0]), __dmul_rn(td[7], qq[1])), __dmul_rn(td[8], qq[2])), td[11]);
+                double dx = __dsub_rn(x, rr[0]), dy = __dsub_rn(y, rr[1]), dz = __dsub_rn(z, rr[2]);
+                double d = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+                const double sq = __ddiv_rn(d0q2, __dadd_rn(d0q2, d));
+                const double sr = __ddiv_rn(d0r2, __dadd_rn(d0r2, d));
+                // MpStageBase.h:825-856: a helix aligned to a non-helix residue is
+                // left out of the --2tm-score sums
+                bool in2 = false;
+                if (B.twotm) {
+                    const char a2 = qs[q], b2 = rs[r];
+                    in2 = !((a2 == 'h' || b2 == 'h') && a2 != b2);
+                }
+                s_t[wp][0][lane] = sq; s_t[wp][1][lane] = sr;
+                s_t[wp][2][lane] = in2 ? sq : 0.0; s_t[wp][3][lane] = in2 ? sr : 0.0;
+            }
+            __syncwarp();
+            const int cnt = n - k0 < 32 ? n - k0 : 32;
+            if (lane < 21) {
+#pragma unroll 8
+                for (int e = 0; e < cnt; e++) sum = __dadd_rn(sum, __dmul_rn((double)X[e], (double)Y[e]));
+            } else {
+#pragma unroll 8
+                for (int e = 0; e < cnt; e++) sum = __dadd_rn(sum, Z[e]);
+            }
+        }
+        double dv[21];
+#pragma unroll
+        for (int f = 0; f < 21; f++) dv[f] = __shfl_sync(FULL, sum, f);
+        const double tq = __shfl_sync(FULL, sum, 21), tr = __shfl_sync(FULL, sum, 22);
+        const double t2q = __shfl_sync(FULL, sum, 23), t2r = __shfl_sync(FULL, sum, 24);
+        if (lane == 0) {
+            double r64 = rmsd_from_sums(dv, (double)n);
+            float r32 = T.rmsd32[i];
+            if (r32 >= 0.f) {
+                T.err[i * 4 + 2] = (float)fabs(__dsub_rn((double)r32, r64));
+                out[8] = (float)r64;
+            }
+            if (out[9] > 0.f || out[10] > 0.f) {
+                double tmq = __ddiv_rn(tq, (double)lq), tmr = __ddiv_rn(tr, (double)lr);
+                T.err[i * 4 + 0] = (float)fabs(__dsub_rn((double)out[9], tmq));
+                T.err[i * 4 + 1] = (float)fabs(__dsub_rn((double)out[10], tmr));
+                out[9] = (float)tmq;
+                out[10] = (float)tmr;
+            }
             if (B.twotm) {
-                // MpStageBase.h:825-856: a helix aligned to a non-helix residue is left out
-                const char a2 = qs[q], b2 = rs[r];
-                if (!((a2 == 'h' || b2 == 'h') && a2 != b2)) { t2q = __dadd_rn(t2q, sq); t2r = __dadd_rn(t2r, sr); }
+                // secondary TM-scores (MpStageFin.cpp:1723-1818), FP64 like the primary ones
+                out[13] = (float)__ddiv_rn(t2q, (double)lq);
+                out[14] = (float)__ddiv_rn(t2r, (double)lr);
             }
-#pragma unroll
-            for (int a = 0; a < 3; a++)
-#pragma unroll
-                for (int b = 0; b < 3; b++) dv[3 * a + b] = __dadd_rn(dv[3 * a + b], __dmul_rn(qq[a], rr[b]));
-#pragma unroll
-            for (int a = 0; a < 3; a++) {
-                dv[9 + a] = __dadd_rn(dv[9 + a], qq[a]);
-                dv[12 + a] = __dadd_rn(dv[12 + a], rr[a]);
-                dv[15 + a] = __dadd_rn(dv[15 + a], __dmul_rn(qq[a], qq[a]));
-                dv[18 + a] = __dadd_rn(dv[18 + a], __dmul_rn(rr[a], rr[a]));
-            }
-        }
-        double r64 = rmsd_from_sums(dv, (double)n);
-        float r32 = T.rmsd32[i];
-        if (r32 >= 0.f) {
-            T.err[i * 4 + 2] = (float)fabs(__dsub_rn((double)r32, r64));
-            out[8] = (float)r64;
-        }
-        if (out[9] > 0.f || out[10] > 0.f) {
-            double tmq = __ddiv_rn(tq, (double)lq), tmr = __ddiv_rn(tr, (double)lr);
-            T.err[i * 4 + 0] = (float)fabs(__dsub_rn((double)out[9], tmq));
-            T.err[i * 4 + 1] = (float)fabs(__dsub_rn((double)out[10], tmr));
-            out[9] = (float)tmq;
-            out[10] = (float)tmr;
-        }
-        if (B.twotm) {
-            // secondary TM-scores (MpStageFin.cpp:1723-1818), FP64 like the primary ones
-            out[13] = (float)__ddiv_rn(t2q, (double)lq);
-            out[14] = (float)__ddiv_rn(t2r, (double)lr);
         }
     }
-    if (referenced) {
+    if (referenced && lane == 0) {
         float R[9];
 #pragma unroll
         for (int f = 0; f < 9; f++) R[f] = t[f];
@@ -3493,7 +3551,7 @@ __global__ void k_final(Blk B, Bat T, int referenced) {
 }
 
 void launch_final(const Blk& B, const Bat& T, int referenced, cudaStream_t st) {
-    k_final<<<(T.np + 127) / 128, 128, 0, st>>>(B, T, referenced);
+    k_final<<<(T.np + FN_WARPS - 1) / FN_WARPS, FN_WARPS * 32, 0, st>>>(B, T, referenced);
     GTB_LAUNCHED(T);
 }
 
