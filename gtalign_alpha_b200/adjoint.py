@@ -83,11 +83,11 @@ class TMScore(torch.autograd.Function):
         N = q.shape[0]
         # one kernel, unless the backward pass itself is to be differentiated
         if P and not torch.is_grad_enabled():
-            grad_q = torch.zeros_like(gq)
+            oc, nc, qc, gqc, tc, gc, go = (t.contiguous() for t in (off, n, q, gq, tfm, g, gout))
+            grad_q = torch.zeros_like(gqc)
             grad_tfm = torch.empty(P, 12, dtype=torch.float32, device=q.device)
-            qc, tc, go = q.contiguous(), tfm.contiguous(), gout.contiguous()
             st = load_library().gtb_tm_backward(
-                None, P, _ptr(off), _ptr(n), _ptr(qc), _ptr(gq), _ptr(tc), _ptr(g), _ptr(go),
+                None, P, _ptr(oc), _ptr(nc), _ptr(qc), _ptr(gqc), _ptr(tc), _ptr(gc), _ptr(go),
                 _ptr(grad_q), _ptr(grad_tfm),
                 ctypes.c_void_p(torch.cuda.current_stream(q.device).cuda_stream))
             if st != 0:

@@ -700,6 +700,8 @@ __device__ __noinline__ float seed_third_distinct(const float4* q, const float4*
     return m3;
 }
 
+// vis counts what findfrag_variant's fused passes visit (the covariance sweep is
+// the same visit's second half)
 __device__ __forceinline__ float findfrag_variant_fast(const float4* q, const float4* r, int n, float d02,
                                                        float d0s, int swap, unsigned long long& vis) {
     float v[16], tfm[12], best = 0.f;
@@ -735,7 +737,6 @@ __device__ __forceinline__ float findfrag_variant_fast(const float4* q, const fl
         if (LARGEDST_CMP < m3 || m3 < d02s || n <= 3) dst32 = d02s;
         else dst32 = __fadd_rn(d02s, __fmul_rn(ceilf(__fmul_rn(__fsub_rn(m3, d02s), 2.0f)), 0.5f));
         seed_cov(q, r, n, tfm, dst32, v);
-        vis += n;
         if (v[15] < 1.0f) break;
         if ((int)v[15] == n) break;
     }

@@ -320,7 +320,7 @@ gtb_status gtb_last_work(const gtb_handle* h, unsigned long long* w4);
  * launch of the seed scan, the refinement passes, the DP and the detailed
  * search's own kernels is bracketed by CUDA events on its stream, and
  * gtb_last_kernel_ms gives the summed times (ms) of the last call:
- * ms4[0] seed, [1] refinement, [2] DP, [3] detailed search.  Launches of
+ * ms4[0] seed, [1] refinement, [2] DP and traceback, [3] detailed search.  Launches of
  * concurrent sub-batches overlap, so a sum can exceed the call's span.
  * Off by default. */
 gtb_status gtb_set_kernel_timing(gtb_handle* h, int on);
@@ -341,9 +341,9 @@ typedef struct {
                               over several CTAs (128..65536; default 512) */
     int refine_long_ctas;  /* CTAs per pair of the refinement's long-pair tier
                               (pairs from 1,536 positions; 1..16; default 16);
-                              raised, up to 256, where a sub-batch has so few
-                              such pairs that their launch would have fewer
-                              than 1,024 CTAs */
+                              raised where a sub-batch has so few such pairs
+                              that their launch would have fewer than 1,024
+                              CTAs; at most 64 such pairs share 592 CTAs */
     int dp_cta_pairs;      /* pairs of each DP launch (its largest matrices)
                               run as a wavefront over a CTA's warps
                               (0..65536; default 592, 4 per SM) */
