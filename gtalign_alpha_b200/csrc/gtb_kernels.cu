@@ -1810,6 +1810,9 @@ __global__ void __launch_bounds__(CM_WARPS * 32, 4) k_refine_coop(Blk B, Bat T, 
     // the first pair by position, the next ones as clusters come free
     int* ctr = T.rhist + RL_NB + 1 + cls;
     const int ncl = (int)gridDim.x / C;
+    // every CTA of the cluster has started before its shared memory is written
+    // from another one (S.win); the later pairs have the barriers at a pair's end
+    if (C > 1) cl.sync();
     for (int slot = first + (int)blockIdx.x / C; slot < last;) {
         const int i = T.rlist[slot];
         const int qi = pair_qi(B, T, i), ri = pair_ri(B, T, i);

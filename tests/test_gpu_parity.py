@@ -388,3 +388,33 @@ def test_detailed_search_batches(oracle, fill, depth):
     d = dict(OPTSETS["frg3s12"], depth=depth, prescore=0.2)
     res, ora = run_both(oracle, q, r, d)
     assert_same(res, ora, q.n, r.n)
+
+
+@pytest.mark.parametrize("nr", [1, 64, 65, 256, 257, 600])
+def test_refinement_clusters_on_a_busy_gpu(oracle, nr):
+    """Batches at the edges of the refinement's cluster sizes (8 CTAs a pair up
+    to 64 pairs, 4 up to 256, then 2) from three handles at once, so that the
+    CTAs of a cluster start beside other calls' work: a cluster's first pair
+    reaches another CTA's shared memory like the later ones.  Every call equals
+    the oracle bit for bit."""
+    import threading
+    from gtalign_alpha_b200 import synth
+    from gtalign_alpha_b200.api import GTalignB200
+    wl = synth.config0(seed=nr, n_refs=nr, qlen=70, lmin=30, lmax=90 if nr > 64 else 300)
+    q, r = synth.pack(wl.queries), synth.pack(wl.refs)
+    d = OPTSETS["speed13"]
+    got = [None] * 3
+
+    def calls(k):
+        with GTalignB200(0, 0, _lib_opts(d)) as g:
+            got[k] = [g.process_block(q, r, scorethld=0.0) for _ in range(3)]
+
+    th = [threading.Thread(target=calls, args=(k,)) for k in range(3)]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    ora = oracle.process_block(q, r, _ora_opts(oracle, d))
+    for res in got:
+        for x in res:
+            assert_same(x, ora, q.n, r.n)
