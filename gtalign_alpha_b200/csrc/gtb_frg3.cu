@@ -125,6 +125,9 @@ __global__ void __launch_bounds__(F3_WARPS * 32) k_f3_localdp(Blk B, Bat T) {
                     }
                 }
                 if (!__shfl_sync(FULL, ok, 0)) return;
+                // lane 0's look at the counter before every lane's reads of the
+                // row (a shuffle alone orders no memory)
+                __syncwarp();
                 __threadfence_block();
             }
             const int jj = t0 + lane;

@@ -2749,14 +2749,17 @@ __device__ __forceinline__ bool dp_pair_fast(const float* t, float d02, float gc
                             __nanosleep(32);
                         }
                     }
-                    ok = __shfl_sync(FULL, ok, 0);
+                    if (!__shfl_sync(FULL, ok, 0)) return false;
+                    // lane 0's look at the counter before every lane's reads of
+                    // the row (a shuffle alone orders no memory)
+                    __syncwarp();
                     if (cta_wave) __threadfence_block();
                     else __threadfence();
-                    if (!ok) return false;
                 }
                 const int jj = t0 + lane;
                 if (s > 0) rb = jj < lr ? (WAVE ? __ldcg(row + jj) : row[jj]) : 0.f;
                 // these 32 columns into the ring, the next 32 on their way
+                __syncwarp();                // the columns in their place are read
                 const int a = jj & (DPR_W - 1), b = (jj + 1) & (DPR_W - 1);
                 ring.c[0][0][a] = cn.x; ring.c[0][1][a] = cn.y; ring.c[0][2][a] = cn.z;
                 ring.c[1][0][b] = cn.x; ring.c[1][1][b] = cn.y; ring.c[1][2][b] = cn.z;
