@@ -207,6 +207,7 @@ struct DevBlock {
     const int *qlen, *rlen, *qoff, *roff, *qmol, *rmol;
     const float *qx, *qy, *qz, *rx, *ry, *rz;
     const float4 *q4, *r4;
+    const unsigned char *qodd, *rodd;
     const unsigned char *qa, *ra;
     char *qs, *rs;
     // index trees (null: none)
@@ -286,6 +287,7 @@ static gtb_status run_block(gtb_handle* h, const DevBlock& D, float scorethld,
     B.qlen = D.qlen; B.rlen = D.rlen; B.qoff = D.qoff; B.roff = D.roff;
     B.qx = D.qx; B.qy = D.qy; B.qz = D.qz; B.rx = D.rx; B.ry = D.ry; B.rz = D.rz;
     B.q4 = D.q4; B.r4 = D.r4; B.q4off = D.qoff; B.r4off = D.roff;
+    B.qodd = D.qodd; B.rodd = D.rodd;
     B.qa = D.qa; B.ra = D.ra; B.qs = D.qs; B.rs = D.rs; B.qmol = D.qmol; B.rmol = D.rmol;
     B.qmax = *std::max_element(D.hqlen.begin(), D.hqlen.end());
     B.qmin = *std::min_element(D.hqlen.begin(), D.hqlen.end());
@@ -508,7 +510,7 @@ static gtb_status run_block(gtb_handle* h, const DevBlock& D, float scorethld,
         T.tfm_ib = (float*)(base + o_tib); T.tfm_gr = (float*)(base + o_tgr);
         T.out = (float*)(base + o_out); T.err = (float*)(base + o_err);
         long long* offs = (long long*)(base + o_offs);
-        T.off_bt = offs; T.off_row = offs + (np + 1); T.off_aln = offs + 2 * (np + 1); T.off_str = offs + 3 * (np + 1);
+        T.off_bt = offs; T.off_row = offs + (np + 1); T.off_aln = offs + 2 * (np + 1);
         T.bt = (unsigned*)(base + o_bt); T.row = (float*)(base + o_row);
         T.aln = (unsigned*)(base + o_aln); T.str = strings ? (base + o_str) : nullptr;
         T.str_off = strings ? (long long*)(base + o_sto) : nullptr;
@@ -790,6 +792,7 @@ struct gtb_block {
     float4* c4 = nullptr;
     cudaStream_t st = nullptr;       // stream of the allocation and of the free
     unsigned char* rsd = nullptr;
+    unsigned char* odd = nullptr;    // per structure (Blk::qodd)
     char* ss = nullptr;
     // index trees (null: none): node x, y, z; left, right, residue
     float *nx = nullptr, *ny = nullptr, *nz = nullptr;
@@ -857,7 +860,7 @@ static gtb_status upload_block(gtb_handle* h, const HostSoA& S, gtb_block* b,
     size_t ot = cls ? carve(S.n * 4) : 0;
     size_t ox = carve(S.npos * 4), oy = carve(S.npos * 4), oz = carve(S.npos * 4);
     size_t oa = carve(S.npos), os = carve(S.npos);
-    size_t o4 = carve(S.npos * 16);
+    size_t o4 = carve(S.npos * 16), od = carve(S.n);
     size_t on = ndx ? carve((size_t)S.npos * 4 * GTB_NNDXFIELDS) : 0;
     size_t ond = ndx ? carve((size_t)S.npos * 16) : 0;
     size_t onc = ndx ? carve((size_t)S.npos * 8) : 0;
@@ -872,7 +875,7 @@ static gtb_status upload_block(gtb_handle* h, const HostSoA& S, gtb_block* b,
     }
     b->x = (float*)(d + ox); b->y = (float*)(d + oy); b->z = (float*)(d + oz);
     b->rsd = (unsigned char*)(d + oa); b->ss = d + os;
-    b->c4 = (float4*)(d + o4);
+    b->c4 = (float4*)(d + o4); b->odd = (unsigned char*)(d + od);
     if (ndx) {
         float* nf = (float*)(d + on);
         int* ni = (int*)(nf + 3 * S.npos);
@@ -891,7 +894,7 @@ static gtb_status upload_block(gtb_handle* h, const HostSoA& S, gtb_block* b,
     CK(cudaMemcpyAsync(b->z, S.z, S.npos * 4, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(b->rsd, S.rsd, S.npos, cudaMemcpyHostToDevice, st));
     long long nl = 0;
-    launch_pack4_structs(b->c4, b->x, b->y, b->z, b->doff, b->dlen, b->doff, b->n, st);
+    launch_pack4_structs(b->c4, b->odd, b->x, b->y, b->z, b->doff, b->dlen, b->doff, b->n, st);
     launch_secstr(b->ss, b->x, b->y, b->z, b->dlen, b->doff, b->dmol, b->n, st, &nl);
     if (ndx)
         launch_pack_nodes(b->nd, b->nc, b->nx, b->ny, b->nz, b->nl, b->nr, b->no, b->doff, b->dlen,
@@ -939,7 +942,7 @@ static DevBlock make_devblock(const gtb_block* Q, const gtb_block* R) {
     D.qlen = Q->dlen; D.qoff = Q->doff; D.qmol = Q->dmol;
     D.rlen = R->dlen; D.roff = R->doff; D.rmol = R->dmol;
     D.qx = Q->x; D.qy = Q->y; D.qz = Q->z; D.rx = R->x; D.ry = R->y; D.rz = R->z;
-    D.q4 = Q->c4; D.r4 = R->c4;
+    D.q4 = Q->c4; D.r4 = R->c4; D.qodd = Q->odd; D.rodd = R->odd;
     D.qa = Q->rsd; D.ra = R->rsd; D.qs = Q->ss; D.rs = R->ss;
     D.qnd = Q->nd; D.qnc = Q->nc; D.rnd = R->nd; D.rnc = R->nc;
     D.rtype = R->dtype; D.qtypeend = Q->typemin + Q->n;

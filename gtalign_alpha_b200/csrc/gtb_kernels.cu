@@ -167,37 +167,35 @@ void launch_secstr(char* ss, const float* x, const float* y, const float* z,
 }
 
 // ---------------------------------------------------------------------------
-// A structure's residues as (x, y, z, 0); its first residue's w is 1 when some
-// coordinate is not ordinary: not a number, or above 10^9, from where on squared
-// distances could leave the range that the DP's fast form takes.
-__global__ void k_pack4s(float4* out, const float* x, const float* y, const float* z,
-                         const int* off, const int* len, const int* coff, int n) {
+// A structure's residues as (x, y, z, 0), and its mark: some coordinate is not
+// ordinary (not a number, or above 10^9, from where on squared distances could
+// leave the range that the DP's fast form takes).  The marks have an array of
+// their own: the residue ranges of two structures may overlap, and then share
+// the copies.
+__global__ void k_pack4s(float4* out, unsigned char* mark, const float* x, const float* y,
+                         const float* z, const int* off, const int* len, const int* coff, int n) {
     int si = blockIdx.x;
     if (si >= n) return;
     int o = off[si], L = len[si], c = coff[si];
-    float4 v0 = make_float4(0.f, 0.f, 0.f, 0.f);
     bool odd = false;
     for (int p = threadIdx.x; p < L; p += blockDim.x) {
         const float4 v = make_float4(x[o + p], y[o + p], z[o + p], 0.f);
         odd = odd || !(fabsf(v.x) <= 1.e9f && fabsf(v.y) <= 1.e9f && fabsf(v.z) <= 1.e9f);
-        if (p == 0) v0 = v;
-        else out[c + p] = v;
+        out[c + p] = v;
     }
     odd = __syncthreads_or(odd);
-    if (threadIdx.x == 0) {
-        v0.w = odd ? 1.f : 0.f;
-        out[c] = v0;
-    }
+    if (threadIdx.x == 0) mark[si] = odd ? 1 : 0;
 }
 
-// c4: a structure's first residue
-__device__ __forceinline__ bool coords_ordinary(const float4* c4) { return __ldg(&c4->w) == 0.f; }
+__device__ __forceinline__ bool coords_ordinary(const Blk& B, int qi, int ri) {
+    return (__ldg(B.qodd + qi) | __ldg(B.rodd + ri)) == 0;
+}
 
-void launch_pack4_structs(float4* out, const float* x, const float* y, const float* z,
-                          const int* off, const int* len, const int* coff, int n,
+void launch_pack4_structs(float4* out, unsigned char* mark, const float* x, const float* y,
+                          const float* z, const int* off, const int* len, const int* coff, int n,
                           cudaStream_t st) {
     if (n <= 0) return;
-    k_pack4s<<<n, 128, 0, st>>>(out, x, y, z, off, len, coff, n);
+    k_pack4s<<<n, 128, 0, st>>>(out, mark, x, y, z, off, len, coff, n);
 }
 
 // ---------------------------------------------------------------------------
@@ -775,7 +773,7 @@ __global__ void __launch_bounds__(128) k_findfrag(Blk B, Bat T) {
     PairGeom G;
     G.q4 = B.q4 + B.q4off[qi]; G.r4 = B.r4 + B.r4off[ri];
     G.alc = nullptr;
-    const bool fast = coords_ordinary(G.q4) && coords_ordinary(G.r4);
+    const bool fast = coords_ordinary(B, qi, ri);
     float lbest = 0.f;
     int lsi = 0x7fffffff;
     unsigned long long vis = 0;
@@ -3006,7 +3004,7 @@ __global__ void __launch_bounds__(128) k_dp(Blk B, Bat T, int tfmsrc, float gcos
     const float* qz = B.qz + B.qoff[qi];
     const float4* q4 = B.q4 + B.q4off[qi];
     const float4* r4 = B.r4 + B.r4off[ri];
-    const bool fast = SC != DP_SC_SSRR && coords_ordinary(q4) && coords_ordinary(r4);
+    const bool fast = SC != DP_SC_SSRR && coords_ordinary(B, qi, ri);
     const char* qs = B.qs + B.qoff[qi];
     const char* rs = B.rs + B.roff[ri];
     float* row = T.row + T.off_row[i];
@@ -3089,7 +3087,7 @@ __global__ void __launch_bounds__(32) k_dp_wave(Blk B, Bat T, int tfmsrc, float 
     const float* qz = B.qz + B.qoff[qi];
     const float4* q4 = B.q4 + B.q4off[qi];
     const float4* r4 = B.r4 + B.r4off[ri];
-    const bool fast = SC != DP_SC_SSRR && coords_ordinary(q4) && coords_ordinary(r4);
+    const bool fast = SC != DP_SC_SSRR && coords_ordinary(B, qi, ri);
     const char* qs = B.qs + B.qoff[qi];
     const char* rs = B.rs + B.roff[ri];
     float* row = T.row + T.off_row[i];
@@ -3249,7 +3247,7 @@ __global__ void __launch_bounds__(128) k_f3_dpscore(Blk B, Bat T) {
 #pragma unroll
         for (int f = 0; f < 12; f++) t[f] = sl[1 + f];
         if (lane == 0) work_add(T, WK_F3CELL, (unsigned long long)lq * (unsigned long long)lr);
-        if (coords_ordinary(q4) && coords_ordinary(r4)) {
+        if (coords_ordinary(B, qi, ri)) {
             if (dp_r(lq) == 4)
                 dp_pair_fast<4, true, DP_SC_TFM, false, true>(t, d02, 0.f, lq, lr, q4, r4, nullptr, nullptr, row,
                                                               nullptr, ring, lane, 0, 1, nullptr, nullptr,

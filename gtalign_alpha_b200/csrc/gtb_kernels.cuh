@@ -80,6 +80,7 @@ struct Blk {
     const float *qx, *qy, *qz, *rx, *ry, *rz;
     const float4 *q4, *r4;           // the same coordinates as (x, y, z, 0),
     const int *q4off, *r4off;        // first residue of each structure in q4/r4
+    const unsigned char *qodd, *rodd;   // a structure's coordinates are not ordinary
     const unsigned char *qa, *ra;    // residue letters
     const char *qs, *rs;             // secondary structure
     const int *qmol, *rmol;          // molecule type per structure
@@ -123,7 +124,7 @@ struct Bat {
     const long long *off_row; float* row;     // DP row buffer per pair
     const long long *off_aln; unsigned* aln;  // aligned pairs, reverse order
     float* alc;                      // their coordinates, 6 floats each (offset 6*off_aln)
-    const long long *off_str; char* str;      // alignment rows (null: not produced)
+    char* str;                                // alignment rows (null: not produced)
     // rows of the pairs with an alignment, packed back to back in str: pair i
     // at str + str_off[i] (-1: none), 5 rows of (columns + 1) bytes each, the
     // last byte of a row its NUL; str_cnt: bytes used
@@ -234,10 +235,10 @@ void launch_secstr(char* ss, const float* x, const float* y, const float* z,
                    const int* len, const int* off, const int* mol, int nstr,
                    cudaStream_t st, long long* launches);
 // (x, y, z, 0) copies of the coordinates, for single 16-byte loads in the
-// passes: structure i's residues [off[i], off[i]+len[i]) go to out[coff[i] ...]
-// (its first residue's w marks coordinates that are not ordinary)
-void launch_pack4_structs(float4* out, const float* x, const float* y, const float* z,
-                          const int* off, const int* len, const int* coff, int n,
+// passes: structure i's residues [off[i], off[i]+len[i]) go to out[coff[i] ...];
+// mark[i]: some coordinate of it is not ordinary
+void launch_pack4_structs(float4* out, unsigned char* mark, const float* x, const float* y,
+                          const float* z, const int* off, const int* len, const int* coff, int n,
                           cudaStream_t st);
 // index tree nodes packed for the walks: nd[k] = (x, y, z, residue | SS << 16),
 // nc[k] = (left, right); n positions of a block (ss: the block's secondary

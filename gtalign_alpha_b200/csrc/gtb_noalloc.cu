@@ -63,11 +63,11 @@ struct DevState {
 static DevState g_dev[MAXDEV];
 static std::mutex g_setup_mutex;
 static float h_tbl[3][TBLN];
-// Host copies of the per-pair offsets (4 arrays of up to MAX_PAIRS+1 entries)
+// Host copies of the per-pair offsets (3 arrays of up to MAX_PAIRS+1 entries)
 // and of the back-to-back residue offsets of the (x, y, z, 0) copies.  One set
 // per host thread, so that threads calling on different devices at once do
 // not overwrite each other's plan before it is copied to the device.
-static thread_local long long h_offs[4 * (GTB_NOALLOC_MAX_PAIRS + 1)];
+static thread_local long long h_offs[3 * (GTB_NOALLOC_MAX_PAIRS + 1)];
 static thread_local int h_coff[2 * (GTB_NOALLOC_MAX_PAIRS + 1)];
 // Flag read back after the molecule-type check (per host thread, as above).
 static thread_local int h_naflag[2];
@@ -171,8 +171,7 @@ extern "C" gtb_status gtb_process_block_noalloc(int device, const gtb_options* o
     long long* obt = h_offs;
     long long* orow = h_offs + (np + 1);
     long long* oaln = h_offs + 2 * (np + 1);
-    long long* ostr = h_offs + 3 * (np + 1);
-    obt[0] = orow[0] = oaln[0] = ostr[0] = 0;
+    obt[0] = orow[0] = oaln[0] = 0;
     int nml[4] = {np, 0, 0, 0};      // pairs of the refinement's length classes
     for (int i = 0; i < np; i++) {
         int lq = q->lens[i / r->n], lr = r->lens[i % r->n];
@@ -181,7 +180,6 @@ extern "C" gtb_status gtb_process_block_noalloc(int device, const gtb_options* o
         obt[i + 1] = obt[i] + gtb::bt_words(lq, lr);
         orow[i + 1] = orow[i] + lr;
         oaln[i + 1] = oaln[i] + (lq < lr ? lq : lr);
-        ostr[i + 1] = 0;
     }
     size_t sz = 0;
     auto carve = [&](size_t bytes) { size_t o = sz; sz += al256(bytes); return o; };
@@ -191,7 +189,9 @@ extern "C" gtb_status gtb_process_block_noalloc(int device, const gtb_options* o
     size_t o_tgr = carve((size_t)np * 12 * sizeof(float));
     size_t o_out = carve((size_t)np * 16 * sizeof(float));
     size_t o_err = carve((size_t)np * 4 * sizeof(float));
-    size_t o_offs = carve((size_t)(np + 1) * 4 * sizeof(long long));
+    // the offsets, and a mark per structure (nq + nr bytes, never above the
+    // 8 (nq nr + 1) that a fourth array would take)
+    size_t o_offs = carve((size_t)(np + 1) * 3 * sizeof(long long) + (size_t)q->n + r->n);
     size_t o_bt = carve((size_t)obt[np] * sizeof(unsigned));
     size_t o_row = carve((size_t)orow[np] * sizeof(float));
     size_t o_aln = carve((size_t)oaln[np] * sizeof(unsigned));
@@ -253,6 +253,8 @@ extern "C" gtb_status gtb_process_block_noalloc(int device, const gtb_options* o
     int* coff = (int*)(base + o_co);
     B.q4 = (const float4*)(base + o_q4); B.r4 = (const float4*)(base + o_r4);
     B.q4off = coff; B.r4off = coff + q->n;
+    unsigned char* odd = base + o_offs + (size_t)(np + 1) * 3 * sizeof(long long);
+    B.qodd = odd; B.rodd = odd + q->n;
     B.qa = q->d_rsd; B.ra = r->d_rsd; B.qs = q->d_ss; B.rs = r->d_ss;
     B.qmol = q->d_mol; B.rmol = r->d_mol;
     B.qmax = qmax; B.qmin = qmin; B.rmax = rmax; B.rmin = rmin;
@@ -273,7 +275,7 @@ extern "C" gtb_status gtb_process_block_noalloc(int device, const gtb_options* o
     T.tfm_ib = (float*)(base + o_tib); T.tfm_gr = (float*)(base + o_tgr);
     T.out = (float*)(base + o_out); T.err = (float*)(base + o_err);
     long long* offs = (long long*)(base + o_offs);
-    T.off_bt = offs; T.off_row = offs + (np + 1); T.off_aln = offs + 2 * (np + 1); T.off_str = offs + 3 * (np + 1);
+    T.off_bt = offs; T.off_row = offs + (np + 1); T.off_aln = offs + 2 * (np + 1);
     T.bt = (unsigned*)(base + o_bt); T.row = (float*)(base + o_row);
     T.aln = (unsigned*)(base + o_aln); T.str = nullptr;
     T.alc = (float*)(base + o_alc);
@@ -284,13 +286,13 @@ extern "C" gtb_status gtb_process_block_noalloc(int device, const gtb_options* o
     for (int k = 0; k < 4; k++) T.nml[k] = nml[k];
 
     // the host offsets are copied from the static host array (no allocation)
-    e = cudaMemcpyAsync(offs, h_offs, (size_t)(np + 1) * 4 * sizeof(long long), cudaMemcpyHostToDevice, st);
+    e = cudaMemcpyAsync(offs, h_offs, (size_t)(np + 1) * 3 * sizeof(long long), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(coff, h_coff, (size_t)(q->n + r->n) * sizeof(int), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) {
         long long nl = 0;
-        launch_pack4_structs((float4*)(base + o_q4), q->d_x, q->d_y, q->d_z, q->d_offs, q->d_lens, coff, q->n, st);
-        launch_pack4_structs((float4*)(base + o_r4), r->d_x, r->d_y, r->d_z, r->d_offs, r->d_lens, coff + q->n, r->n, st);
+        launch_pack4_structs((float4*)(base + o_q4), odd, q->d_x, q->d_y, q->d_z, q->d_offs, q->d_lens, coff, q->n, st);
+        launch_pack4_structs((float4*)(base + o_r4), odd + q->n, r->d_x, r->d_y, r->d_z, r->d_offs, r->d_lens, coff + q->n, r->n, st);
         launch_secstr(q->d_ss, q->d_x, q->d_y, q->d_z, q->d_lens, q->d_offs, q->d_mol, q->n, st, &nl);
         launch_secstr(r->d_ss, r->d_x, r->d_y, r->d_z, r->d_lens, r->d_offs, r->d_mol, r->n, st, &nl);
         launch_stages(B, T, opts->refinement, opts->depth, opts->convergence, opts->prescore,

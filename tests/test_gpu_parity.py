@@ -418,3 +418,31 @@ def test_refinement_clusters_on_a_busy_gpu(oracle, nr):
     for res in got:
         for x in res:
             assert_same(x, ora, q.n, r.n)
+
+
+@pytest.mark.parametrize("first", [0, 1])
+@pytest.mark.parametrize("far", [float("inf"), 1.5e19])
+def test_overlapping_structures_with_far_residues(oracle, first, far):
+    """Two structures that share ten residues, the second with a far residue
+    outside them, in either order: whether a structure's coordinates are
+    ordinary is its own, so each pair equals the oracle's.  (The shared residues
+    and their neighbours are 20 A apart: no secondary structure, whichever
+    structure's ends it is assigned from.)"""
+    from gtalign_alpha_b200 import synth
+    from gtalign_alpha_b200.api import GTalignB200
+    rng = np.random.default_rng(5)
+    c = synth.random_chains(rng, [130], "r")[0]
+    c.xyz[:, 0] += np.cumsum(np.where((np.arange(130) >= 46) & (np.arange(130) < 64), 20.0, 0.0)).astype(np.float32)
+    q = synth.pack([synth.homolog(rng, synth.Chain(c.xyz[a:b], c.seq[a:b], "q"), 1.0, 0.0, "q")
+                    for a, b in ((0, 60), (50, 130))] + synth.random_chains(rng, [90], "u"))
+    c.xyz[100, 0] = far
+    span = [((0, 60), (50, 130))[k] for k in (first, 1 - first)]
+    sep = synth.pack([synth.Chain(c.xyz[a:b], c.seq[a:b], "r") for a, b in span])
+    r = synth.pack([c])
+    r = synth.SoA(sep.lens, np.array([a for a, b in span], np.int32), r.x, r.y, r.z, r.rsd, sep.mol)
+    d = OPTSETS["speed13"]
+    with GTalignB200(0, 0, _lib_opts(d)) as g:
+        res = g.process_block(q, r, scorethld=0.0, alignments=False)
+    ora = oracle.process_block(q, sep, _ora_opts(oracle, d))
+    assert np.array_equal(res.alndata.view(np.uint32), ora.out.view(np.uint32))
+    assert np.array_equal(res.tfm.view(np.uint32), ora.tfm.view(np.uint32))
