@@ -328,8 +328,10 @@ def test_longest_chain_pair_properties():
 @pytest.mark.parametrize("far", [3.0e7, 2.0e18, 1.5e19, float("inf")])
 def test_far_residues(oracle, far):
     """Structures with one residue far away, up to where squared distances
-    reach the end of the FP32 range and beyond: the score terms there are
-    those of an IEEE division, bit for bit."""
+    reach the end of the FP32 range and beyond: the results are the oracle's,
+    whose score terms are IEEE divisions, bit for bit.  (A far residue's own
+    term is lost in the others' sum; test_seeds_chosen_by_far_scores has
+    sums of such terms alone.)"""
     from gtalign_alpha_b200 import synth
     wl = synth.config0(seed=41, n_refs=6, qlen=90, lmin=40, lmax=130)
     q, r = synth.pack(wl.queries), synth.pack(wl.refs)
@@ -446,3 +448,20 @@ def test_overlapping_structures_with_far_residues(oracle, first, far):
     ora = oracle.process_block(q, sep, _ora_opts(oracle, d))
     assert np.array_equal(res.alndata.view(np.uint32), ora.out.view(np.uint32))
     assert np.array_equal(res.tfm.view(np.uint32), ora.tfm.view(np.uint32))
+
+
+@pytest.mark.parametrize("opt", ["speed13", "default", "full"])
+def test_seeds_chosen_by_far_scores(oracle, opt):
+    """References with every second dozen of residues 2.4e19 A away: any diagonal's
+    superposition leaves all squared distances between 2^126 and the end of the
+    FP32 range, so the seed is the diagonal with the largest sum of terms of about
+    1e-37, which an oracle with those terms as zeros answers otherwise (9
+    or 10 of the 12 records)."""
+    from gtalign_alpha_b200 import synth
+    wl = synth.config0(seed=43, n_refs=12, qlen=90, lmin=60, lmax=150)
+    q, r = synth.pack(wl.queries), synth.pack(wl.refs)
+    for o, n in zip(r.offs, r.lens):
+        r.x[o:o + n] = np.where(np.arange(n) // 12 % 2 == 1, np.float32(2.4e19), r.x[o:o + n])
+    res, ora = run_both(oracle, q, r, OPTSETS[opt])
+    assert_same(res, ora, q.n, r.n)
+    assert (ora.out[0, :, 9] > 0.05).all()
