@@ -59,5 +59,16 @@ def build(force: bool = False, verbose: bool = False) -> str:
     return LIB
 
 
+def build_arith_check() -> str:
+    """The tests' check of the device arithmetic (tests/cuda/arith_check.cu)."""
+    src = os.path.join(ROOT, "tests", "cuda", "arith_check.cu")
+    lib = os.path.join(ROOT, "tests", "cuda", "libarith_check.so")
+    deps = [src, os.path.join(CSRC, "gtb_device.cuh")]
+    if os.path.exists(lib) and all(os.path.getmtime(d) <= os.path.getmtime(lib) for d in deps):
+        return lib
+    subprocess.check_call([nvcc(), "-shared"] + NVCC_FLAGS + ["-I", CSRC, src, "-o", lib, "-lcudart"])
+    return lib
+
+
 if __name__ == "__main__":
     print(build(force=True, verbose=True))
