@@ -346,6 +346,8 @@ static gtb_status run_block(gtb_handle* h, const DevBlock& D, float scorethld,
     // A copy to pageable host memory holds the host until it is done, and with
     // it the launches of the next sub-batch: such results are copied once all
     // sub-batches are launched (400 structures all against all 198 -> 113 ms).
+    // Until then they have an allocation of their own (own), so that a
+    // sub-batch's working memory goes to the next one on its stream.
     auto pageable = [](const void* p) {
         cudaPointerAttributes a{};
         if (!p) return false;
@@ -353,6 +355,7 @@ static gtb_status run_block(gtb_handle* h, const DevBlock& D, float scorethld,
         return a.type == cudaMemoryTypeUnregistered;
     };
     const bool late = pageable(h_alndata) || pageable(h_tfm) || pageable(h_err);
+    const bool own = late && !strings;
     struct LateBat { char* base; long long p0; int np; const float *out, *tfm, *err; cudaStream_t st; };
     std::vector<LateBat> latebat;
     auto copy_out = [&](long long q0, int np, const float* out, const float* tfm, const float* err,
@@ -365,7 +368,8 @@ static gtb_status run_block(gtb_handle* h, const DevBlock& D, float scorethld,
             CK(cudaMemcpyAsync(h_err + q0 * 4, err, (size_t)np * 4 * sizeof(float), cudaMemcpyDefault, st));
         return GTB_OK;
     };
-    // frees the memory of sub-batches kept past their launches
+    // frees the memory kept past the launches: whole sub-batches with alignment
+    // rows, else results
     auto drop_kept = [&](bool sync) {
         if (sync) for (int k = 0; k < gtb_handle::NSUB; k++) cudaStreamSynchronize(h->sub[k]);
         if (strings) for (const StrBat& sb : strbat) cudaFreeAsync(sb.base, h->st);
@@ -469,6 +473,8 @@ static gtb_status run_block(gtb_handle* h, const DevBlock& D, float scorethld,
         size_t o_tgr = carve((size_t)np * 12 * sizeof(float));
         size_t o_out = carve((size_t)np * 16 * sizeof(float));
         size_t o_err = carve((size_t)np * 4 * sizeof(float));
+        const size_t nres = sz - o_tgr;         // the results' bytes
+        if (own) sz = o_tgr;
         size_t o_offs = carve((size_t)(np + 1) * (B.f3 ? 5 : 4) * sizeof(long long));
         size_t o_bt = carve((size_t)off_bt[np] * sizeof(unsigned));
         size_t o_row = carve((size_t)off_row[np] * sizeof(float));
@@ -498,8 +504,13 @@ static gtb_status run_block(gtb_handle* h, const DevBlock& D, float scorethld,
         size_t o_f3o = B.f3 ? carve((size_t)np * nbr) : 0;
         size_t o_f32 = B.f3 ? carve((size_t)np * 13 * sizeof(float)) : 0;
         size_t o_f3v = B.f3 ? carve((size_t)np * F3_NSEC * sizeof(unsigned)) : 0;
-        char* base = nullptr;
+        char *base = nullptr, *res = nullptr;
+        if (own) {
+            CK(cudaMallocAsync((void**)&res, nres, st));
+            latebat.push_back({res, q0, np, nullptr, nullptr, nullptr, st});
+        }
         CK(cudaMallocAsync((void**)&base, sz, st));
+        if (!own) res = base + o_tgr;
         Bat T{};
         T.p0 = q0; T.np = np;
         int* ints = (int*)(base + o_ints);
@@ -507,8 +518,8 @@ static gtb_status run_block(gtb_handle* h, const DevBlock& D, float scorethld,
         T.sfndx = ints + 4 * np; T.sfpos = ints + 5 * np; T.sfndx_cur = ints + 6 * np; T.sfpos_cur = ints + 7 * np;
         float* fl = (float*)(base + o_flts);
         T.grand = fl; T.best = fl + np; T.best0 = fl + 2 * np; T.rmsd32 = fl + 3 * np;
-        T.tfm_ib = (float*)(base + o_tib); T.tfm_gr = (float*)(base + o_tgr);
-        T.out = (float*)(base + o_out); T.err = (float*)(base + o_err);
+        T.tfm_ib = (float*)(base + o_tib); T.tfm_gr = (float*)res;
+        T.out = (float*)(res + (o_out - o_tgr)); T.err = (float*)(res + (o_err - o_tgr));
         long long* offs = (long long*)(base + o_offs);
         T.off_bt = offs; T.off_row = offs + (np + 1); T.off_aln = offs + 2 * (np + 1);
         T.bt = (unsigned*)(base + o_bt); T.row = (float*)(base + o_row);
@@ -587,9 +598,10 @@ static gtb_status run_block(gtb_handle* h, const DevBlock& D, float scorethld,
         if (strings) {
             // read after the batch: only the bytes the rows took
             strbat.push_back({base, q0, np, T.str_off, T.str_cnt, T.str});
+            if (late) latebat.push_back({base, q0, np, T.out, T.tfm_gr, T.err, st});
+            return GTB_OK;
         }
-        if (late) latebat.push_back({base, q0, np, T.out, T.tfm_gr, T.err, st});
-        if (strings || late) return GTB_OK;
+        if (own) latebat.back() = {res, q0, np, T.out, T.tfm_gr, T.err, st};
         CK(cudaFreeAsync(base, st));
         return GTB_OK;
     };

@@ -102,3 +102,36 @@ def test_kernel_timing_and_work_counters():
         g.process_block(q, r, scorethld=0.0)
         ms, w = g.last_kernel_ms(), g.last_work()
         assert (ms[:3] > 0).all() and ms[3] == 0 and w[3] == 0
+
+
+def test_pageable_results_take_no_more_device_memory_than_pinned_ones():
+    """Six sub-batches in two waves: a wave's working memory goes to the next one,
+    whichever memory the results are copied to.  The most that the device's pool
+    had in use during a call, with results in pageable and in pinned memory."""
+    import ctypes
+    import torch
+    from gtalign_alpha_b200 import synth
+    from gtalign_alpha_b200.api import NERR, NOUT, GTalignB200, Options, _CResults, pack_fields
+    rng = np.random.default_rng(8)
+    q = pack_fields(synth.pack(synth.random_chains(rng, [200], "q")))
+    r = pack_fields(synth.pack(synth.random_chains(rng, list(rng.integers(150, 250, 7000)), "r")))
+    cu = ctypes.CDLL("libcuda.so.1")
+    pool, used = ctypes.c_void_p(), ctypes.c_uint64()
+    HIGH = 8                                       # CU_MEMPOOL_ATTR_USED_MEM_HIGH
+    high, recs = {}, {}
+    with GTalignB200(0, 0, Options.speed(13)) as g:
+        assert cu.cuDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+        g.set_tuning(sub_pairs=1024)
+        for kind in ("warm", "pinned", "pageable"):
+            a = [torch.zeros(7000, w, pin_memory=kind == "pinned") for w in (NOUT, 12, NERR)]
+            res = _CResults(a[0].data_ptr(), a[1].data_ptr(), None, a[2].data_ptr(), None, None)
+            used.value = 0
+            assert cu.cuMemPoolSetAttribute(pool, HIGH, ctypes.byref(used)) == 0
+            assert g.lib.gtb_process_block(g.handle, 0.5, q.beg, q.end, r.beg, r.end, ctypes.byref(res)) == 0
+            assert cu.cuMemPoolGetAttribute(pool, HIGH, ctypes.byref(used)) == 0
+            high[kind], recs[kind] = used.value, a
+    for x, y in zip(recs["pinned"], recs["pageable"]):
+        assert torch.equal(x.view(torch.int32), y.view(torch.int32))
+    # the pageable results of all sub-batches, and each allocation's rounding
+    assert high["pinned"] > 40e6
+    assert high["pageable"] <= high["pinned"] + 7000 * 4 * (NOUT + 12 + NERR) + 6 * (2 << 20), high
