@@ -37,8 +37,8 @@ constexpr int RLW_GRID = 1024;
 constexpr int RLW_CTAS_MAX = 256;
 constexpr int RLW_CTA_WARPS = 4;     // warps of a long-pair CTA (one candidate each)
 // A sub-batch with at most RLW_CTA_MAX long pairs runs their passes a CTA each
-// (k_refine_long) over RLW_CTA_GRID CTAs in all: too few variants to fill the
-// lanes of the other form
+// (k_refine_long) over RLW_CTA_GRID CTAs in all, at least 16 a pair: too few
+// variants to fill the lanes of the other form
 constexpr int RLW_CTA_MAX = 64;
 constexpr int RLW_CTA_GRID = 592;
 constexpr int RLW_CAND = 17;         // floats per warp candidate

@@ -340,10 +340,11 @@ typedef struct {
     int seed_chunk;        /* seed offsets per CTA; a pair with more is split
                               over several CTAs (128..65536; default 512) */
     int refine_long_ctas;  /* CTAs per pair of the refinement's long-pair tier
-                              (pairs from 1,536 positions; 1..16; default 16);
-                              raised where a sub-batch has so few such pairs
-                              that their launch would have fewer than 1,024
-                              CTAs; at most 64 such pairs share 592 CTAs */
+                              (pairs from 1,536 positions; 1..16; default 16)
+                              where a sub-batch has more than 64 such pairs,
+                              raised where their launch would have fewer than
+                              1,024 CTAs; without effect at 64 or fewer, which
+                              share 592 CTAs, at least 16 a pair */
     int dp_cta_pairs;      /* pairs of each DP launch (its largest matrices)
                               run as a wavefront over a CTA's warps
                               (0..65536; default 592, 4 per SM) */

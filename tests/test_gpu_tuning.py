@@ -5,9 +5,9 @@ pair, CTAs per long refinement pair, DP pairs run as a CTA wavefront, pairs
 per concurrent sub-batch.  Every pair is still aligned by the same arithmetic
 in the same order, so the records, transforms, numeric errors and alignment
 rows must agree bit for bit under every tuning.  The block has long pairs
-(1,600-2,300 residues) so that every path the tuning touches is taken: split
-seeds, the long-pair refinement tier, the CTA-wavefront DP, and two
-sub-batches at the smallest sub_pairs.
+(1,600-2,300 residues) so that split seeds, the CTA-wavefront DP and two
+sub-batches at the smallest sub_pairs are taken.  refine_long_ctas has a part
+only where a sub-batch has more than 64 long pairs: a test of its own.
 """
 import ctypes
 
@@ -57,6 +57,35 @@ def test_results_do_not_depend_on_the_tuning(speed, nshort):
             _same(g.process_block(q, r, scorethld=0.0), ref)
     # the template's three homologs are found by its noisy copy (query 1)
     assert (ref.tm_query[1] > 0.5).sum() >= 3
+
+
+@pytest.mark.parametrize("refinement", [1, -1])
+def test_more_than_64_long_pairs(refinement):
+    """156 pairs of 1,536+ positions in one sub-batch: lanes take the variants,
+    refine_long_ctas CTAs a pair (6 at least, for 1,024 in all: at 1, 7 and 16 the
+    launches differ).  The results equal each other and those of the rows of 13
+    pairs, whose passes take a CTA each."""
+    from gtalign_alpha_b200 import synth
+    from gtalign_alpha_b200.api import GTalignB200, Options
+    rng = np.random.default_rng(64)
+    tmpl = synth.random_chains(rng, [1640], "t")[0]
+    fam = [synth.homolog(rng, tmpl, float(s), 0.02, "h") for s in rng.uniform(0.5, 3.0, 25)]
+    qs, r = fam[:12], synth.pack(fam[12:])
+    q = synth.pack(qs)
+    with GTalignB200(0, 0, Options(refinement=refinement, convergence=2, prescore=0.0)) as g:
+        got = []
+        for c in (1, 7, 16):
+            g.set_tuning(refine_long_ctas=c)
+            got.append(g.process_block(q, r, scorethld=0.0))
+        for x in got[1:]:
+            _same(x, got[0])
+        rows = [g.process_block(synth.pack([c]), r, scorethld=0.0) for c in qs]
+    # alignment length: the passes are over 1,536 positions and more
+    assert (got[0].alndata[..., 4] - got[0].alndata[..., 7] >= 1536).all()
+    for k, x in enumerate(rows):
+        assert np.array_equal(x.alndata[0].view(np.uint32), got[0].alndata[k].view(np.uint32))
+        assert np.array_equal(x.tfm[0].view(np.uint32), got[0].tfm[k].view(np.uint32))
+        assert np.array_equal(x.numerr[0].view(np.uint32), got[0].numerr[k].view(np.uint32))
 
 
 def test_set_tuning_refuses_out_of_range_fields():
