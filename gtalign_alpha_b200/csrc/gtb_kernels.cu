@@ -428,35 +428,6 @@ __device__ float score_pass(const PairGeom& G, const float* tfm, float d02, int 
     return __fadd_rn(ss, sc);
 }
 
-// fused: score under tfm (chk, m3 tracking) and the covariance of the
-// positions with d <= thr (the next pass's threshold when it is known, or
-// its most likely value when it is not)
-__device__ float score_and_ext(const PairGeom& G, const float* tfm, float d02, int chk, float d82,
-                               float thr, float* v, int m3mode, float& m3out) {
-    float ss = 0.f, sc = 0.f, sb = 0.f;
-    float m1 = LARGEDST, m2 = LARGEDST, m3 = LARGEDST;
-    CovAcc a;
-    a.init();
-    for (int b0 = 0; b0 < G.n; b0 += BLK) {
-        int b1 = b0 + BLK < G.n ? b0 + BLK : G.n;
-#pragma unroll 2
-        for (int k = b0; k < b1; k++) {
-            float qx, qy, qz, rx, ry, rz;
-            G.at(k, qx, qy, qz, rx, ry, rz);
-            float d = dist2_tf(tfm, qx, qy, qz, rx, ry, rz);
-            if (!chk || d <= d82) sb = __fadd_rn(sb, tmterm(d02, d));
-            track3(m3mode, d, m1, m2, m3);
-            if (d <= thr) a.add(qx, qy, qz, rx, ry, rz);
-        }
-        nfold(ss, sc, sb);
-        a.fold();
-    }
-    nfold(ss, sc, sb);
-    a.final(v);
-    m3out = m3;
-    return __fadd_rn(ss, sc);
-}
-
 // every one of the 16 sums changed by less than RM_CONVEPS relative (b strided)
 __device__ __forceinline__ int converged16(const float* a, const float* b, int bstr) {
     int cnt = 0;
@@ -2183,8 +2154,8 @@ __device__ float long_pass(LongSmem& S, const PairGeom& G, int kind, int k0, int
     return sc;
 }
 
-// The whole alignment's FP32 RMSD (production phase 1): warp 0 as coop_rmsd, from
-// the pair's positions.
+// The whole alignment's FP32 RMSD (production phase 1): warp 0 from the pair's
+// positions.
 __device__ float long_rmsd(LongSmem& S, const PairGeom& G) {
     float r = 0.f;
     if (threadIdx.x < 32)

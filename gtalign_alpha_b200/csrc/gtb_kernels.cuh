@@ -18,15 +18,25 @@ namespace gtb {
 // (rlw_ctas_for), up to RLW_CTAS_MAX: a lone long pair has variants for many
 // more warps.
 constexpr int RL_LONG = 1536;
-// The warp-a-pass form (k_refine_coop).  It takes every pair where few take
-// part or the batch has at most RC_SMALL pairs: a solve serves 8 variants there
-// against the lane form's 32, so that with the GPU full the lane form is the
-// faster (all launches of 16 x 500 by warps 58 against 54 ms, of 2 x 20,000
-// 123 against 100; of 1 x 1,000 by lanes 12.4 against 11.4).  From RC_N2
-// positions it always does (the lane form's slowest pair sets the launch's
-// time).  CTAs per pair: 8 from RC_N2, at least 4 from RC_N1 (2 and 8: within
-// 4% either way), else by the pairs of the batch (with one CTA instead of two
-// 16 x 500 takes twice as long; 4 for 1,000 pairs 13.9 against 11.4 ms).
+// The warp-a-pass form (k_refine_coop) takes every pair where few take part
+// or the batch has at most RC_SMALL pairs, and from RC_N2 positions always.  A
+// solve serves 8 variants there against the lane form's 32, so that with the GPU
+// full the lane form is the faster: 2 x 20,000 with all launches by warps 97.4
+// against 83.4 ms, 16 x 500 38.3 against 35.7.  In a small batch a launch lasts as
+// long as its slowest pair (1 x 1,000 at the fastest preset by lanes 6.8 against
+// 6.4 ms), and so it does with long pairs by lanes (400 structures all against all
+// 144 against 110 ms; 2 x 20,000 the same).  "Few" is the option, a score filter,
+// which leaves 2 to 5% of the pairs in a search: 2 x 8,000 by lanes 57 against 47
+// ms.  Where all pass, the two come out alike (22,500 pairs of 250 residues 178
+// against 173 ms) up to where lanes fill the GPU (90,000 pairs of 150: 412
+// against 508).
+// CTAs per pair: 8 up to RC_NP8 pairs, 4 up to RC_NP4, 2 up to RC_NP2, else 1; at
+// least 4 from RC_N1 positions and 8 from RC_N2.  Refinement of one query
+// against 32, 64, 128, 256 and 600 with 8 CTAs a pair 2.8, 1.9, 2.9, 3.4, 4.8 ms, with
+// 4 3.3, 2.2, 3.3, 3.4, 4.5, with 2 3.7, 2.8, 4.0, 3.8, 4.7, with 1 5.3, 4.0, 5.7, 5.4, 6.5;
+// against 1,000 at the fastest preset with 4, 2, 1 4.3, 3.4, 4.0; 16 x 500 with 1
+// and 4 within 3%.  From RC_N1 with 2, 4, 8 (16 x 500) 17.3, 15.9, 15.3; from RC_N2
+// with 4 and 8 within 4% (400 all against all, 2 x 20,000).
 constexpr int RC_N1 = 256, RC_N2 = 512;
 constexpr int RC_SMALL = 2048, RC_NP8 = 64, RC_NP4 = 256, RC_NP2 = 4096;
 constexpr int RC_GRID = 592;          // CTAs of a launch at most (4 per SM)
@@ -38,7 +48,10 @@ constexpr int RLW_CTAS_MAX = 256;
 constexpr int RLW_CTA_WARPS = 4;     // warps of a long-pair CTA (one candidate each)
 // A sub-batch with at most RLW_CTA_MAX long pairs runs their passes a CTA each
 // (k_refine_long) over RLW_CTA_GRID CTAs in all, at least 16 a pair: too few
-// variants to fill the lanes of the other form
+// variants to fill the lanes of the other form.  Refinement of a call by CTAs
+// against by lanes: 16 pairs of 1,600 residues 5.3 against 36 ms, 64 18.4 against 48.5
+// (of 2,500 residues 50 against 127), 156 5.9 against 7.4 (unrelated pairs), 400 94.7
+// against 84.5: the two cross above the line.
 constexpr int RLW_CTA_MAX = 64;
 constexpr int RLW_CTA_GRID = 592;
 constexpr int RLW_CAND = 17;         // floats per warp candidate
@@ -270,7 +283,7 @@ __host__ __device__ inline void seed_range(int lq, int lr, int qmax, int qmin, i
     if (sihi > nsteps - 1) sihi = nsteps - 1;
 }
 void launch_findfrag(const Blk& B, const Bat& T, cudaStream_t st);
-// few: most pairs of the batch are already filtered out (32 lanes per pair)
+// few: a score filter has left out most pairs of the batch (RC_SMALL)
 void launch_refine(int mode, const Blk& B, const Bat& T, cudaStream_t st, bool few);
 // DP and traceback.  skipmode 0: skip LOWTMSC|SCOREDP (plain), 1: skip LOWTMSC
 // only; constrained: the traceback keeps the pairs within d8 of the grand best
