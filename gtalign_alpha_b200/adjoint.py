@@ -81,8 +81,15 @@ class TMScore(torch.autograd.Function):
         q, tfm, off, n, g, gq = ctx.saved_tensors
         P = tfm.shape[0]
         N = q.shape[0]
-        # one kernel, unless the backward pass itself is to be differentiated
-        if P and not torch.is_grad_enabled():
+        # one kernel, unless the backward pass itself is to be differentiated or a
+        # saved-tensor hook gave back other types, shapes or devices than were
+        # saved: torch operations then convert or refuse them
+        f32, dev = torch.float32, q.device
+        as_saved = q.is_cuda and all(
+            t.dtype == dt and t.shape == sh and t.device == dev
+            for t, dt, sh in ((q, f32, (N, 3)), (gq, f32, (N, 3)), (tfm, f32, (P, 12)), (g, f32, (P, 6)),
+                              (off, torch.int64, (P,)), (n, torch.int32, (P,)), (gout, f32, (P,))))
+        if P and as_saved and not torch.is_grad_enabled():
             oc, nc, qc, gqc, tc, gc, go = (t.contiguous() for t in (off, n, q, gq, tfm, g, gout))
             grad_q = torch.zeros_like(gqc)
             grad_tfm = torch.empty(P, 12, dtype=torch.float32, device=q.device)

@@ -210,3 +210,35 @@ def test_autograd_rows_weights_and_layouts(lens):
     for o, n in zip(off, lens):
         covered[o:o + n] = True
     assert (out[0][0].cpu()[~covered] == 0).all()
+
+
+def _hooked(unpack, q):
+    """Gradients by q and tfm with a saved-tensor hook that unpacks by `unpack`."""
+    import torch
+    from gtalign_alpha_b200.adjoint import TMScore
+    t = torch.eye(3, device="cuda").reshape(1, 9).repeat(2, 1)
+    t = torch.cat([t, torch.full((2, 3), 0.3, device="cuda")], 1).requires_grad_(True)
+    off = torch.tensor([0, 40], device="cuda")
+    n = torch.tensor([40, 60], dtype=torch.int32, device="cuda")
+    r = q.detach().reshape(-1, 3) + torch.linspace(0.0, 2.0, 300, device="cuda").reshape(100, 3)
+    with torch.autograd.graph.saved_tensors_hooks(lambda x: x, unpack):
+        tm = TMScore.apply(q, t, r, off, n, torch.tensor([2.0, 3.0], device="cuda"))
+    return torch.autograd.grad(tm.sum(), (q, t))
+
+
+def test_backward_of_saved_tensors_that_hooks_changed():
+    """The backward kernel takes raw pointers: what a saved-tensor hook unpacks in
+    another type is converted by torch operations, on another device refused, and
+    so is a q of another shape (as they were before the kernel)."""
+    import torch
+    q = (10.0 * torch.randn(100, 3, generator=torch.Generator().manual_seed(2))).cuda().requires_grad_(True)
+    ref = _hooked(lambda x: x, q)
+    got = _hooked(lambda x: x.double() if x.dtype == torch.float32 else x, q)
+    for a, b in zip(ref, got):
+        assert b.dtype == torch.float32
+        # sums of up to 60 terms in FP32 and in FP64
+        assert (a - b).abs().max() <= 60 * 2.0 ** -24 * b.abs().max()
+    with pytest.raises(RuntimeError):
+        _hooked(lambda x: x.cpu(), q)
+    with pytest.raises((RuntimeError, IndexError)):
+        _hooked(lambda x: x, q.detach().reshape(-1).requires_grad_(True))
