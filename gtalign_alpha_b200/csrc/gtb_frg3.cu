@@ -88,7 +88,7 @@ __device__ __forceinline__ int pair_r(const Blk& B, const Bat& T, int i) { retur
 // kept in shared memory and written a row at a time; the columns' letters and
 // the previous strip's row move from lane to lane.  What bounds it: the chain of
 // steps.  (One warp a pair storing a byte per lane and row at each step, with the
-// row buffer read in the chain: 4.3 ms for 2 x 3,000 references; now 1.0.)
+// row buffer read in the chain: 4.3 ms for 2 x 3,000 references; now 1.1.)
 __global__ void __launch_bounds__(F3_WARPS * 32) k_f3_localdp(Blk B, Bat T) {
     __shared__ volatile int s_prog[F3_WARPS];            // chunks done: strip * nchunks + chunk
     __shared__ unsigned char s_tile[F3_WARPS][32 * 36];
@@ -511,8 +511,8 @@ __device__ __forceinline__ void f3_sync(cooperative_groups::cluster_group& cl, i
 // entries of slot j in order, as one warp going through all configurations
 // would.  What bounds it: the latency of the tree walks.  With one CTA a pair
 // and rounds of 16 configurations a launch lasted as long as its largest pair,
-// SMs busy a fifth of the time: 42 ms for 2 x 3,000 references, now 10; for
-// 2 x 8,000 the stage's own kernels took 61 ms, now 36 (with 3 CTAs a SM 66).
+// SMs busy a fifth of the time: the stage's own kernels took 50 ms for 2 x 3,000
+// references, now 20; for 2 x 8,000 68 ms, now 36 (with 3 CTAs a SM 66).
 __global__ void __launch_bounds__(F3_WARPS * 32, 4) k_f3_search(Blk B, Bat T, int depth) {
     extern __shared__ __align__(16) unsigned char f3_smem[];
     F3Smem& S = *(F3Smem*)f3_smem;
